@@ -60,44 +60,6 @@ __device__ __forceinline__ bool is_representative(uint64_t m, const uint8_t* per
   return true;
 }
 
-// Walks masks in rank order from rank r0: Gosper's successor for one
-// species; for two species the B part advances first and wraps into the A part.
-struct RankWalker {
-  uint64_t m, ca, cbm;
-  int64_t rb;
-  bool two;
-  RsedSpecies sp;
-  __device__ void init(int64_t r0, const rsed_group_t& grp, const int64_t* binom, int kp1) {
-    two = grp.species_b != 0ull;
-    if (!two) {
-      m = rsed_unrank(r0, grp.n_site, grp.n_filled, binom, kp1);
-      return;
-    }
-    sp = rsed_species(grp.species_b, grp.n_site, grp.n_filled, grp.n_filled_b, binom, kp1);
-    const int64_t ra = r0 / sp.cb;
-    rb = r0 % sp.cb;
-    ca = rsed_unrank(ra, sp.na, sp.ka, binom, kp1);
-    cbm = rsed_unrank(rb, sp.nb, sp.kb, binom, kp1);
-    m = rsed_deposit(ca, sp.sa) | rsed_deposit(cbm, sp.sb);
-  }
-  // call only while a next rank exists
-  __device__ void next() {
-    if (!two) {
-      m = rsed_gosper_next(m);
-      return;
-    }
-    if (rb + 1 < sp.cb) {
-      cbm = rsed_gosper_next(cbm);
-      ++rb;
-    } else {
-      cbm = (sp.kb > 0) ? ((1ull << sp.kb) - 1ull) : 0ull;
-      rb = 0;
-      ca = rsed_gosper_next(ca);
-    }
-    m = rsed_deposit(ca, sp.sa) | rsed_deposit(cbm, sp.sb);
-  }
-};
-
 __device__ __forceinline__ int64_t group_cb(const rsed_group_t& grp, const int64_t* binom, int kp1) {
   return grp.species_b ? binom[__popcll(grp.species_b) * kp1 + grp.n_filled_b] : 1;
 }

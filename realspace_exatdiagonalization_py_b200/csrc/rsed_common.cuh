@@ -121,6 +121,44 @@ __device__ __forceinline__ uint64_t rsed_gosper_next(uint64_t x) {
   return (((r ^ x) >> 2) >> (__ffsll((long long)c) - 1)) | r;
 }
 
+// Walks masks in rank order from rank r0: Gosper's successor for one
+// species; for two species the B part advances first and wraps into the A part.
+struct RankWalker {
+  uint64_t m, ca, cbm;
+  int64_t rb;
+  bool two;
+  RsedSpecies sp;
+  __device__ void init(int64_t r0, const rsed_group_t& grp, const int64_t* binom, int kp1) {
+    two = grp.species_b != 0ull;
+    if (!two) {
+      m = rsed_unrank(r0, grp.n_site, grp.n_filled, binom, kp1);
+      return;
+    }
+    sp = rsed_species(grp.species_b, grp.n_site, grp.n_filled, grp.n_filled_b, binom, kp1);
+    const int64_t ra = r0 / sp.cb;
+    rb = r0 % sp.cb;
+    ca = rsed_unrank(ra, sp.na, sp.ka, binom, kp1);
+    cbm = rsed_unrank(rb, sp.nb, sp.kb, binom, kp1);
+    m = rsed_deposit(ca, sp.sa) | rsed_deposit(cbm, sp.sb);
+  }
+  // call only while a next rank exists
+  __device__ void next() {
+    if (!two) {
+      m = rsed_gosper_next(m);
+      return;
+    }
+    if (rb + 1 < sp.cb) {
+      cbm = rsed_gosper_next(cbm);
+      ++rb;
+    } else {
+      cbm = (sp.kb > 0) ? ((1ull << sp.kb) - 1ull) : 0ull;
+      rb = 0;
+      ca = rsed_gosper_next(ca);
+    }
+    m = rsed_deposit(ca, sp.sa) | rsed_deposit(cbm, sp.sb);
+  }
+};
+
 // Image of mask m under the site permutation perm (0-based targets).
 __device__ __forceinline__ uint64_t rsed_permute(uint64_t m, const uint8_t* __restrict__ perm) {
   uint64_t img = 0;
@@ -213,6 +251,30 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
 }
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+
+// Sum over the group elements g with g(s) = m, ascending, of
+// pref * conj(chi(g)) * (product-form phase of U_g on s): the Fock amplitude at
+// m of pref times the orbit sum of the representative s.  `g_last` is the
+// catalog's element with g(s) = m; with a trivial stabilizer it is the only
+// one, so a state costs one phase product instead of |G| images.
+__device__ __forceinline__ double2 rsed_state_amplitude(uint64_t s, uint64_t m, int g_last, uint64_t stab,
+                                                        const rsed_group_t& grp, const uint8_t* __restrict__ perm,
+                                                        const double2* __restrict__ eta,
+                                                        const double2* __restrict__ chi, double2 pref) {
+  const int N = grp.n_site;
+  uint64_t img;
+  double2 sum = make_double2(0.0, 0.0);
+  const bool one = __popcll(stab) == 1;
+  for (int g = one ? g_last : 0; g < grp.n_group; ++g) {
+    if (!one && rsed_permute(s, perm + g * N) != m) continue;
+    const double2 ph = rsed_phase_product(s, perm + g * N, eta + g * N, grp.fermionic, &img);
+    const double2 ch = chi[g];
+    const double2 t = rsed_cmul_exact(rsed_cmul_exact(pref, make_double2(ch.x, -ch.y)), ph);
+    sum = make_double2(sum.x + t.x, sum.y + t.y);
+    if (one) break;
+  }
+  return sum;
 }
 
 // Per-thread error reporting: the first failing check stores its code.

@@ -1,0 +1,72 @@
+"""Kernels whose work split depends on the sizes, at the edges of their tiles:
+each against the oracle's restatement of the same definition."""
+
+from fractions import Fraction
+
+import numpy as np
+import pytest
+
+from oracle import port
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(family, size, nf, theta=None, species=False):
+    """(data, sector set, oracle catalog, perm0, eta) of one lattice."""
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import models
+
+    if family == "heisenberg":
+        m = models.build_heisenberg_second_quantized_model(size[0], 1.0)
+    elif family == "haldane":
+        m = models.build_zero_flux_bosonic_fci_second_quantized_model(sample_size=list(size))
+    elif family == "checkerboard":
+        m = models.build_zero_flux_fermionic_fci_second_quantized_model(sample_size=list(size))
+    else:
+        m = models.build_spinful_hubbard_second_quantized_model(list(size), 1.0, 4.0)
+    if theta is not None and family != "hubbard":
+        ed.update_second_quantized_model_with_twisted_phases(m, twisted_phases_over_2π=list(theta))
+    G = ed.build_translation_group(m.lattice, theta)
+    sp = models.hubbard_spin_species(m, nf // 2) if species else None
+    data = ed.build_ed_data(m, filling_fraction=Fraction(nf, m.lattice.n_site), symmetry_group=G, species=sp)
+    perm0, eta = port.group_arrays(G)
+    osp = None if sp is None else (sum(1 << (i - 1) for i in sp[0]), sp[1])
+    cat = port.catalog(m.lattice.n_site, nf, perm0, eta, m.particle_statistics.name == "FERMIONIC", species=osp)
+    return data, ed.SectorSet(data.orbit_catalog, data.irrep_list), cat, perm0, eta
+
+
+def _vector(n, seed):
+    rng = np.random.default_rng(seed)
+    c = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    return c / np.linalg.norm(c)
+
+
+# no particles, one, all sites taken, one empty; several chunks; more than 32
+# sites (two sites per lane); fermions and twists with stabilizers
+@pytest.mark.parametrize("family,size,nf,theta,sector", [
+    ("haldane", (2, 3), 0, None, 0),
+    ("haldane", (2, 3), 1, None, 1),
+    ("haldane", (2, 3), 11, (0.2, 0.1), 0),
+    ("haldane", (2, 3), 12, None, 0),
+    ("heisenberg", (13, 1), 6, (0.3, 0.0), 5),
+    ("checkerboard", (2, 3), 4, (0.25, 0.4), 2),
+    ("checkerboard", (4, 4), 2, None, 9),
+    ("checkerboard", (3, 6), 2, (0.1, 0.3), 4),
+])
+def test_one_body_density_sizes(family, size, nf, theta, sector):
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import correlators as cr
+
+    data, sset, cat, perm0, eta = _case(family, size, nf, theta)
+    n = data.orbit_catalog.n_site
+    fermion = family == "checkerboard"
+    s = next(k % len(sset.dims) for k in range(sector, sector + len(sset.dims)) if sset.dims[k % len(sset.dims)])
+    basis = ed.Symmetry_Sector_Basis(data.irrep_list[s], data.orbit_catalog, sset, s)
+    c = _vector(basis.dim, 3)
+    chi = np.asarray(data.irrep_list[s].values, dtype=np.complex128)
+    orbits = port.sector_orbits(cat, chi)
+    ref = port.obdm_orbitwise(cat, orbits, c, chi, perm0, eta, fermion, n, nf)
+    rho = cr.one_body_density_matrix(basis, c)
+    # entries are at most nf and sums of at most a few thousand terms
+    np.testing.assert_allclose(rho, ref, atol=1e-12, rtol=0)
+    np.testing.assert_array_equal(rho, cr.one_body_density_matrix(basis, c))
