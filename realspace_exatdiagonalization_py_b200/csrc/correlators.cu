@@ -110,12 +110,16 @@ __global__ void __launch_bounds__(kCT, 2) k_obdm_part(rsed_group_t grp, const in
   uint8_t* perm = smem + lay.perm;
   const int N = grp.n_site, ng = grp.n_group, kp1 = grp.n_filled + 1;
   for (int i = threadIdx.x; i < (N + 1) * kp1; i += kCT) binom[i] = grp.binom[i];
+  bool twisted = false;
   for (int i = threadIdx.x; i < ng * N; i += kCT) {
-    eta[i] = reinterpret_cast<const double2*>(grp.eta)[i];
+    const double2 v = reinterpret_cast<const double2*>(grp.eta)[i];
+    twisted |= v.x != 1.0 || v.y != 0.0;
+    eta[i] = v;
     perm[i] = grp.perm[i];
   }
   for (int i = threadIdx.x; i < ng; i += kCT) chi[i] = chi_g[i];
-  __syncthreads();
+  const bool unit = __syncthreads_or(twisted) == 0;
+  const uint64_t first = (1ull << grp.n_filled) - 1ull;  // stands in for missing states (N <= 63)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const bool fermion = grp.fermionic != 0;
@@ -165,12 +169,15 @@ __global__ void __launch_bounds__(kCT, 2) k_obdm_part(rsed_group_t grp, const in
       int4 e[T::U];
 #pragma unroll
       for (int u = 0; u < T::U; ++u) e[u] = ok[u] ? __ldg(table + idx[u]) : make_int4(-1, 0, 0, 0);
-      double2 c[T::U];
+      double2 c[T::U], ph[T::U];
       uint64_t s[T::U], st[T::U], mem[T::U];
+      int ge[T::U];
 #pragma unroll
       for (int u = 0; u < T::U; ++u) {
         c[u] = make_double2(0.0, 0.0);
-        s[u] = st[u] = mem[u] = 0;
+        s[u] = first;
+        st[u] = mem[u] = 0;
+        ge[u] = e[u].y;
         if (e[u].x >= 0) {
           c[u] = __ldg(x + e[u].x);
           s[u] = __ldg(repr_masks + e[u].x);
@@ -178,6 +185,7 @@ __global__ void __launch_bounds__(kCT, 2) k_obdm_part(rsed_group_t grp, const in
           mem[u] = __ldg(member + e[u].x);
         }
       }
+      rsed_phases<T::U>(s, ge, N, grp.n_filled, perm, eta, fermion, unit, ph);
 #pragma unroll
       for (int u = 0; u < T::U; ++u) {
         const int i = lane + 32 * (u % (NP / 32));
@@ -186,7 +194,7 @@ __global__ void __launch_bounds__(kCT, 2) k_obdm_part(rsed_group_t grp, const in
         if (e[u].x >= 0 && (c[u].x != 0.0 || c[u].y != 0.0)) {
           const double S = (double)__popcll(st[u]);
           const double norm = 1.0 / sqrt((double)ng * S);
-          K = rsed_state_amplitude(s[u], nn | (1ull << i), e[u].y, st[u], grp, perm, eta, chi,
+          K = rsed_state_amplitude(s[u], nn | (1ull << i), e[u].y, ph[u], st[u], grp, perm, eta, chi,
                                    make_double2(c[u].x * norm, c[u].y * norm));
           if ((mem[u] >> sector) & 1ull) {
             const double2 ch = chi[e[u].y];

@@ -2,55 +2,95 @@
 //
 // A sector vector c (one coefficient per representative of the sector) is
 // the state sum_col c_col / sqrt(|G| |Stab(s_col)|) sum_g conj(chi(g)) U_g |s_col>.
-// One thread per basis state m (table rank r): the table gives m's
-// representative s and one g with g(s) = m; the thread sums, in ascending g
-// like the reference's dictionary accumulation, every group element that maps
-// s to m, with the product-form phase U_g|s> = phase * |g s>.  Amplitudes at or
-// below atol are dropped, the norm of the rest is summed per block, and a
-// last pass rescales to unit norm.
+// For a basis state m (table rank r) the table gives m's representative s and
+// one g with g(s) = m.  With a trivial stabilizer that g is the only one; a
+// state of a symmetric orbit sums, in ascending g like the reference's
+// dictionary accumulation, every group element that maps s to m, with the
+// product-form phase U_g|s> = phase * |g s>.  Amplitudes at or below atol are
+// dropped, the norm of the rest is summed per block, and a last pass rescales
+// to unit norm.
+//
+// Bound by the shared-memory and L1 lookups (three loads by representative and
+// k site phases per state, all lane-divergent), then by the 32 B a state of
+// table and amplitude traffic.  Taking every state's |G| images cost 2.12 ms
+// for 10.5 million states on 32 sites; one element per state with the group
+// tables in shared memory: 244 us.  Two or four states per thread measured
+// slower (263, 367 us: fewer warps for the same lookups).
 #include "rsed_internal.cuh"
 
 namespace {
 
 constexpr int kFT = 256;
+constexpr int64_t kFChunk = 8 * kFT;  // ranks per block
 
-__global__ void __launch_bounds__(kFT) k_fock_amps(rsed_group_t grp, const int4* __restrict__ table,
-                                                   const uint64_t* __restrict__ repr_masks,
-                                                   const uint64_t* __restrict__ stab_mask,
-                                                   const double2* __restrict__ xo, const double2* __restrict__ chi,
-                                                   double atol, double2* __restrict__ amp,
-                                                   uint64_t* __restrict__ masks, double* __restrict__ block_norm2) {
+struct FockLayout {
+  size_t eta, chi, perm, total;
+};
+
+FockLayout fock_layout(int n_site, int n_group) {
+  FockLayout l{};
+  l.eta = 0;
+  l.chi = sizeof(double2) * (size_t)n_group * n_site;
+  l.perm = l.chi + sizeof(double2) * (size_t)n_group;
+  l.total = l.perm + align_up((size_t)n_group * n_site, 16);
+  return l;
+}
+
+__global__ void __launch_bounds__(kFT, 6) k_fock_amps(rsed_group_t grp, const int4* __restrict__ table,
+                                                      const uint64_t* __restrict__ repr_masks,
+                                                      const uint64_t* __restrict__ stab_mask,
+                                                      const double2* __restrict__ xo,
+                                                      const double2* __restrict__ chi_g, double atol,
+                                                      double2* __restrict__ amp, uint64_t* __restrict__ masks,
+                                                      double* __restrict__ block_norm2, FockLayout lay) {
+  extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[kFT / 32];
-  const int64_t r = (int64_t)blockIdx.x * kFT + threadIdx.x;
+  __shared__ double inv[RSED_MAX_GROUP + 1];  // 1 / sqrt(|G| |Stab|)
+  double2* eta = reinterpret_cast<double2*>(smem + lay.eta);
+  double2* chi = reinterpret_cast<double2*>(smem + lay.chi);
+  uint8_t* perm = smem + lay.perm;
+  const int N = grp.n_site;
+  bool twisted = false;
+  for (int i = threadIdx.x; i < grp.n_group * N; i += kFT) {
+    const double2 v = reinterpret_cast<const double2*>(grp.eta)[i];
+    twisted |= v.x != 1.0 || v.y != 0.0;
+    eta[i] = v;
+    perm[i] = grp.perm[i];
+  }
+  for (int i = threadIdx.x; i < grp.n_group; i += kFT) {
+    chi[i] = chi_g[i];
+    inv[i + 1] = 1.0 / sqrt((double)grp.n_group * (double)(i + 1));
+  }
+  const bool unit = __syncthreads_or(twisted) == 0;
+  // |z| > atol by its square, the square root only next to the threshold
+  const double sure = 1.0001 * atol * atol;
+  auto above = [&](double2 z) {
+    const double q = z.x * z.x + z.y * z.y;
+    return q > sure || sqrt(q) > atol;
+  };
   double n2 = 0.0;
-  if (r < grp.n_states) {
+  for (int64_t r = (int64_t)blockIdx.x * kFChunk + threadIdx.x;
+       r < min(grp.n_states, ((int64_t)blockIdx.x + 1) * kFChunk); r += kFT) {
     const int4 e = __ldg(table + r);
     double2 sum = make_double2(0.0, 0.0);
     uint64_t m = 0;
     if (e.x >= 0) {
-      const uint64_t s = repr_masks[e.x];
-      const double2 co = xo[e.x];
-      const int N = grp.n_site;
-      const double2* eta = reinterpret_cast<const double2*>(grp.eta);
-      uint64_t img;
-      rsed_phase_product(s, grp.perm + (int64_t)e.y * N, eta + (int64_t)e.y * N, grp.fermionic, &m);
-      if (sqrt(co.x * co.x + co.y * co.y) > atol) {
-        const double inv = 1.0 / sqrt((double)grp.n_group * (double)__popcll(stab_mask[e.x]));
-        const double2 pref = make_double2(co.x * inv, co.y * inv);
-        for (int g = 0; g < grp.n_group; ++g) {
-          const double2 ph = rsed_phase_product(s, grp.perm + (int64_t)g * N, eta + (int64_t)g * N, grp.fermionic,
-                                                &img);
-          if (img != m) continue;
-          const double2 ch = chi[g];
-          const double2 t = rsed_cmul_exact(rsed_cmul_exact(pref, make_double2(ch.x, -ch.y)), ph);
-          sum = make_double2(sum.x + t.x, sum.y + t.y);
-        }
-        if (sqrt(sum.x * sum.x + sum.y * sum.y) <= atol) sum = make_double2(0.0, 0.0);
+      const double2 co = __ldg(xo + e.x);
+      const uint64_t s[1] = {__ldg(repr_masks + e.x)};
+      const uint64_t stab = __ldg(stab_mask + e.x);
+      const int order = __popcll(stab), g[1] = {e.y};
+      if (masks || order > 1) m = rsed_permute(s[0], perm + e.y * N);
+      if (above(co)) {
+        double2 ph[1];
+        rsed_phases<1>(s, g, N, grp.n_filled, perm, eta, grp.fermionic, unit, ph);
+        sum = rsed_state_amplitude(s[0], m, e.y, ph[0], stab, grp, perm, eta, chi,
+                                   make_double2(co.x * inv[order], co.y * inv[order]));
+        if (!above(sum)) sum = make_double2(0.0, 0.0);
       }
     }
     amp[r] = sum;
     if (masks) masks[r] = m;
-    n2 = sum.x * sum.x + sum.y * sum.y;
+    n2 += sum.x * sum.x + sum.y * sum.y;
   }
   for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = n2;
@@ -88,7 +128,7 @@ __global__ void k_fock_scale(double2* __restrict__ amp, int64_t n, const double*
 }  // namespace
 
 extern "C" size_t rsed_fock_scratch_bytes(int64_t n_states) {
-  const int64_t n_blocks = (n_states + kFT - 1) / kFT;
+  const int64_t n_blocks = (n_states + kFChunk - 1) / kFChunk;
   return sizeof(double) * (size_t)(n_blocks + 2);
 }
 
@@ -103,12 +143,15 @@ extern "C" int rsed_fock_expand(const rsed_group_t* grp, const rsed_entry_t* tab
   RSED_REQUIRE(grp->eta != nullptr, RSED_EINVAL, "Fock expansion needs the group's eta phases");
   RSED_REQUIRE(scratch_bytes >= rsed_fock_scratch_bytes(grp->n_states), RSED_ESCRATCH, "Fock scratch too small");
   cudaStream_t stream = as_stream(stream_);
-  const int64_t n_blocks = (grp->n_states + kFT - 1) / kFT;
+  const int64_t n_blocks = (grp->n_states + kFChunk - 1) / kFChunk;
+  const FockLayout lay = fock_layout(grp->n_site, grp->n_group);
+  if (lay.total > 48 * 1024)
+    RSED_TRY_CUDA(cudaFuncSetAttribute(k_fock_amps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.total));
   double* bn = reinterpret_cast<double*>(scratch);
   double* nrm = bn + n_blocks;
-  k_fock_amps<<<(unsigned)n_blocks, kFT, 0, stream>>>(
+  k_fock_amps<<<(unsigned)n_blocks, kFT, lay.total, stream>>>(
       *grp, reinterpret_cast<const int4*>(table), repr_masks, stab_mask, reinterpret_cast<const double2*>(x_orbit),
-      reinterpret_cast<const double2*>(chi), atol, reinterpret_cast<double2*>(amp), masks, bn);
+      reinterpret_cast<const double2*>(chi), atol, reinterpret_cast<double2*>(amp), masks, bn, lay);
   RSED_CHECK_LAUNCH();
   k_fock_norm<<<1, kFT, 0, stream>>>(bn, n_blocks, nrm);
   RSED_CHECK_LAUNCH();
@@ -249,6 +292,7 @@ __global__ void k_fock_overlap_final(const double2* __restrict__ part, int n_m, 
   const int k = (i % tile) * tile + j % tile;
   const double2* src = part + (p * n_tiles * n_tiles + t) * tt + k;
   double x = 0.0, y = 0.0;
+#pragma unroll 8
   for (int64_t c = lane; c < n_chunks; c += 32) {
     const double2 v = src[c * per_chunk * tt];
     x += v.x;

@@ -253,26 +253,64 @@ __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
+// Product-form phases (rsed_phase_product, without the images) of U masks under
+// U group elements at once: the U chains of complex products run side by side.
+// Every mask holds n_filled particles; `unit` = every site phase of the group
+// is exactly 1, so only the fermionic sign is left.
+template <int U>
+__device__ __forceinline__ void rsed_phases(const uint64_t (&s)[U], const int (&g)[U], int n_site, int n_filled,
+                                            const uint8_t* __restrict__ perm, const double2* __restrict__ eta,
+                                            bool fermion, bool unit, double2 (&ph)[U]) {
+  uint64_t m[U], placed[U];
+  int par[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    m[u] = s[u];
+    placed[u] = 0;
+    par[u] = 0;
+    ph[u] = make_double2(1.0, 0.0);
+  }
+  if (!unit || fermion) {
+    for (int j = 0; j < n_filled; ++j) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int at = g[u] * n_site + __ffsll((long long)m[u]) - 1;
+        m[u] &= m[u] - 1;
+        if (fermion) {
+          const int p = perm[at];
+          par[u] ^= __popcll(placed[u] & ~((2ull << p) - 1ull)) & 1;
+          placed[u] |= 1ull << p;
+        }
+        if (!unit) ph[u] = rsed_cmul_exact(ph[u], eta[at]);
+      }
+    }
+  }
+  if (fermion) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) ph[u] = rsed_cmul_exact(ph[u], make_double2(par[u] ? -1.0 : 1.0, 0.0));
+  }
+}
+
 // Sum over the group elements g with g(s) = m, ascending, of
 // pref * conj(chi(g)) * (product-form phase of U_g on s): the Fock amplitude at
 // m of pref times the orbit sum of the representative s.  `g_last` is the
-// catalog's element with g(s) = m; with a trivial stabilizer it is the only
-// one, so a state costs one phase product instead of |G| images.
-__device__ __forceinline__ double2 rsed_state_amplitude(uint64_t s, uint64_t m, int g_last, uint64_t stab,
+// catalog's element with g(s) = m and `ph` its phase: with a trivial
+// stabilizer (`stab` the bitmask of the elements that fix s) it is the only
+// one, so the state costs one phase product instead of |G| images.
+__device__ __forceinline__ double2 rsed_state_amplitude(uint64_t s, uint64_t m, int g_last, double2 ph, uint64_t stab,
                                                         const rsed_group_t& grp, const uint8_t* __restrict__ perm,
                                                         const double2* __restrict__ eta,
                                                         const double2* __restrict__ chi, double2 pref) {
+  if (__popcll(stab) == 1)
+    return rsed_cmul_exact(rsed_cmul_exact(pref, make_double2(chi[g_last].x, -chi[g_last].y)), ph);
   const int N = grp.n_site;
-  uint64_t img;
   double2 sum = make_double2(0.0, 0.0);
-  const bool one = __popcll(stab) == 1;
-  for (int g = one ? g_last : 0; g < grp.n_group; ++g) {
-    if (!one && rsed_permute(s, perm + g * N) != m) continue;
-    const double2 ph = rsed_phase_product(s, perm + g * N, eta + g * N, grp.fermionic, &img);
-    const double2 ch = chi[g];
-    const double2 t = rsed_cmul_exact(rsed_cmul_exact(pref, make_double2(ch.x, -ch.y)), ph);
+  for (int g = 0; g < grp.n_group; ++g) {
+    if (rsed_permute(s, perm + g * N) != m) continue;
+    uint64_t img;
+    const double2 pg = rsed_phase_product(s, perm + g * N, eta + g * N, grp.fermionic, &img);
+    const double2 t = rsed_cmul_exact(rsed_cmul_exact(pref, make_double2(chi[g].x, -chi[g].y)), pg);
     sum = make_double2(sum.x + t.x, sum.y + t.y);
-    if (one) break;
   }
   return sum;
 }

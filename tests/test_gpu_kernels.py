@@ -70,3 +70,33 @@ def test_one_body_density_sizes(family, size, nf, theta, sector):
     # entries are at most nf and sums of at most a few thousand terms
     np.testing.assert_allclose(rho, ref, atol=1e-12, rtol=0)
     np.testing.assert_array_equal(rho, cr.one_body_density_matrix(basis, c))
+
+
+# one state, several blocks' worth of ranks, symmetric orbits (the sum over the
+# group elements that reach a state), fermions, twists, two species
+@pytest.mark.parametrize("family,size,nf,theta,species", [
+    ("haldane", (2, 3), 0, None, False),
+    ("haldane", (2, 3), 12, (0.2, 0.1), False),
+    ("heisenberg", (16, 1), 8, (0.3, 0.0), False),
+    ("checkerboard", (2, 3), 4, (0.25, 0.4), False),
+    ("hubbard", (2, 3), 6, (0.15, 0.0), True),
+])
+def test_fock_amplitudes_sizes(family, size, nf, theta, species):
+    import realspace_exatdiagonalization_py_b200 as ed
+
+    data, sset, cat, perm0, eta = _case(family, size, nf, theta, species)
+    fermion = family in ("checkerboard", "hubbard")
+    for s in [k for k, d in enumerate(sset.dims) if d][:3]:
+        basis = ed.Symmetry_Sector_Basis(data.irrep_list[s], data.orbit_catalog, sset, s)
+        c = _vector(basis.dim, s)
+        chi = np.asarray(data.irrep_list[s].values, dtype=np.complex128)
+        ref = port.fock_expand(cat, port.sector_orbits(cat, chi), c, chi, perm0, eta, fermion)
+        keys = np.array(sorted(ref), dtype=np.uint64)
+        m, a = ed.expand_sector_state_to_fock_amplitudes(c, basis, as_dict=False)
+        m, a = m.cpu().numpy().view(np.uint64), a.cpu().numpy()
+        order = np.argsort(m)
+        np.testing.assert_array_equal(m[order], keys)
+        # unit vectors: a few ulps of the largest amplitude
+        np.testing.assert_allclose(a[order], np.array([ref[int(k)] for k in keys]), atol=1e-14, rtol=0)
+        dense = ed.expand_sector_state_to_fock_dense(c, basis).cpu().numpy()
+        np.testing.assert_array_equal(dense[dense != 0], a)
