@@ -14,8 +14,12 @@
 namespace {
 
 constexpr int kFlagThreads = 256;           // threads per block in the flag pass
-constexpr int kRanksPerThread = 32;         // one uint32 bitmap word per thread
-constexpr int kRanksPerBlock = kFlagThreads * kRanksPerThread;
+constexpr int kRanksPerWord = 32;           // one uint32 bitmap word
+// Ranks of one block of the flag and list passes: large bases amortise the
+// block's tables over 8192 ranks; below 2^20 states 256 ranks a block (one
+// rank per thread) spread the little work over the SMs (12,870 states: two
+// blocks of 8192 took 329 us).
+int ranks_per_block(int64_t n_states) { return n_states >= (1ll << 20) ? 8192 : 256; }
 
 struct GroupView {
   const int64_t* binom;
@@ -51,63 +55,179 @@ __device__ GroupView stage_group(const rsed_group_t& g, unsigned char* smem, siz
   return v;
 }
 
-__device__ __forceinline__ bool is_representative(uint64_t m, const uint8_t* perm, int n_site,
-                                                  int n_group) {
-  for (int g = 0; g < n_group; ++g) {
-    uint64_t img = rsed_permute(m, perm + g * n_site);
-    if (img < m) return false;
+// A site permutation as rotations: the sites that move by the same distance
+// form a class, and the image of a mask is the union of its classes, each
+// rotated by its distance.  A translation of a periodic lattice has two classes
+// per wrapped direction at most (4 in two dimensions), so an image takes 4
+// and-rotate-or steps instead of one table step per occupied site.  Groups with
+// an element of more than kClasses distances take the images bit by bit.
+constexpr int kClasses = 8;
+
+template <typename M>
+struct MoveClass {
+  M mask;
+  M rot;
+};
+template <typename M>
+struct GroupMoves {
+  MoveClass<M> cls[RSED_MAX_GROUP][kClasses];
+  int n[RSED_MAX_GROUP];
+};
+
+__device__ __forceinline__ uint32_t rotl(uint32_t x, uint32_t d) { return __funnelshift_l(x, x, d); }
+__device__ __forceinline__ uint64_t rotl(uint64_t x, uint64_t d) {
+  const int s = (int)d & 63;
+  return (x << s) | (x >> ((64 - s) & 63));
+}
+
+__device__ __forceinline__ int low_bit(uint32_t m) { return __ffs((int)m) - 1; }
+__device__ __forceinline__ int low_bit(uint64_t m) { return __ffsll((long long)m) - 1; }
+__device__ __forceinline__ int count_bits(uint32_t m) { return __popc(m); }
+__device__ __forceinline__ int count_bits(uint64_t m) { return __popcll(m); }
+
+// rsed_rank_any on masks and ranks of the width of M (up to 32 sites every rank
+// is below C(32, 16) < 2^31).
+template <typename M, typename I>
+__device__ __forceinline__ I rank_of(M m, const I* binom, int kp1, M sb, I cb) {
+  I ra = 0, rb = 0;
+  int ja = 1, jb = 1;
+  while (m) {
+    const int b = low_bit(m);
+    m &= m - 1;
+    if (sb == 0) {
+      ra += binom[b * kp1 + ja];
+      ++ja;
+    } else {
+      const int below_b = count_bits((M)(sb & (((M)1 << b) - 1)));
+      if ((sb >> b) & 1) {
+        rb += binom[below_b * kp1 + jb];
+        ++jb;
+      } else {
+        ra += binom[(b - below_b) * kp1 + ja];
+        ++ja;
+      }
+    }
   }
-  return true;
+  return sb ? ra * cb + rb : ra;
+}
+
+// Fills `mv` from the staged permutations; false if some element has more than
+// kClasses classes.  All threads of the block call it.
+template <typename M>
+__device__ bool stage_moves(const rsed_group_t& grp, const uint8_t* perm, GroupMoves<M>& mv) {
+  constexpr int W = 8 * sizeof(M) - 1;
+  for (int g = threadIdx.x; g < grp.n_group; g += blockDim.x) mv.n[g] = 0;
+  __syncthreads();
+  bool fits = true;
+  for (int t = threadIdx.x; t < grp.n_group * grp.n_site; t += blockDim.x) {
+    const int g = t / grp.n_site, i = t % grp.n_site;
+    const uint8_t* pg = perm + g * grp.n_site;
+    const int d = (pg[i] - i) & W;
+    bool first = true;
+    for (int k = 0; k < i && first; ++k) first = ((pg[k] - k) & W) != d;
+    if (!first) continue;
+    M mask = 0;
+    for (int k = i; k < grp.n_site; ++k)
+      if (((pg[k] - k) & W) == d) mask |= (M)1 << k;
+    const int at = atomicAdd(&mv.n[g], 1);  // the order of the classes does not matter
+    if (at < kClasses)
+      mv.cls[g][at] = MoveClass<M>{mask, (M)d};
+    else
+      fits = false;
+  }
+  return __syncthreads_and(fits);
 }
 
 __device__ __forceinline__ int64_t group_cb(const rsed_group_t& grp, const int64_t* binom, int kp1) {
   return grp.species_b ? binom[__popcll(grp.species_b) * kp1 + grp.n_filled_b] : 1;
 }
 
-// Pass 1: representative flags as a bitmap, one 32-rank word per thread
-// (symmetry_resolved_ed.py:519-528).
-__global__ void k_rep_flags(rsed_group_t grp, uint32_t* bitmap, int64_t* block_count,
-                            GroupSmemLayout lay) {
+// Pass 1: representative flags as a bitmap (symmetry_resolved_ed.py:519-528).
+// A thread tests R consecutive ranks (32 / R lanes share a bitmap word) against
+// all |G| images at once, each move class loaded once for the R masks.  Bound by
+// integer issue: some lane of a warp nearly always holds a representative, so
+// leaving the loop at the first smaller image saved nothing, and the images
+// themselves are the cost.  M = uint32_t up to 32 sites.
+// 10.5 million states, 32 sites, |G| = 16: 865 us with one image per occupied
+// site step and 32 ranks per thread, @MS@ in this form.
+template <typename M, int R>
+__global__ void __launch_bounds__(kFlagThreads) k_rep_flags(rsed_group_t grp, uint32_t* bitmap, int64_t* block_count,
+                                                            int per_block, GroupSmemLayout lay) {
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ GroupMoves<M> mv;
+  __shared__ int warp_sums[kFlagThreads / 32];
   GroupView gv = stage_group(grp, smem, lay.binom_off, lay.perm_off, 0, 0, false, false);
-  __shared__ int64_t warp_sums[kFlagThreads / 32];
+  const bool moves = stage_moves<M>(grp, gv.perm, mv);
   const int kp1 = grp.n_filled + 1;
-  const int64_t word = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t r0 = word * kRanksPerThread;
-  uint32_t bits = 0;
-  if (r0 < grp.n_states) {
+  int count = 0;
+  for (int t = 0; t < per_block; t += kFlagThreads * R) {
+    const int64_t r0 = (int64_t)blockIdx.x * per_block + t + (int64_t)threadIdx.x * R;
+    M m[R];
+    uint32_t bits = 0;
     RankWalker w;
-    w.init(r0, grp, gv.binom, kp1);
-    for (int i = 0; i < kRanksPerThread; ++i) {
-      const int64_t r = r0 + i;
-      if (r >= grp.n_states) break;
-      if (is_representative(w.m, gv.perm, grp.n_site, grp.n_group)) bits |= 1u << i;
-      if (r + 1 < grp.n_states) w.next();
+    if (r0 < grp.n_states) w.init(r0, grp, gv.binom, kp1);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      m[i] = 0;
+      if (r0 + i < grp.n_states) {
+        m[i] = (M)w.m;
+        bits |= 1u << i;
+      }
+      if (i + 1 < R && r0 + i + 1 < grp.n_states) w.next();
     }
-    bitmap[word] = bits;
+    for (int g = 0; g < grp.n_group; ++g) {
+      M img[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) img[i] = 0;
+      if (moves) {
+        for (int c = 0; c < mv.n[g]; ++c) {
+          const MoveClass<M> cl = mv.cls[g][c];
+#pragma unroll
+          for (int i = 0; i < R; ++i) img[i] |= rotl(m[i] & cl.mask, cl.rot);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < R; ++i) img[i] = (M)rsed_permute(m[i], gv.perm + g * grp.n_site);
+      }
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (img[i] < m[i]) bits &= ~(1u << i);
+    }
+    count += __popc(bits);
+    // the 32 / R lanes of a word put their bits together
+    if (R < 32) {
+      bits <<= (threadIdx.x & (32 / R - 1)) * R;
+#pragma unroll
+      for (int o = 1; o < 32 / R; o <<= 1) bits |= __shfl_xor_sync(0xffffffffu, bits, o);
+    }
+    if ((threadIdx.x & (32 / R - 1)) == 0 && r0 < grp.n_states) bitmap[r0 / kRanksPerWord] = bits;
   }
-  int c = __popc(bits);
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = c;
+  for (int o = 16; o > 0; o >>= 1) count += __shfl_down_sync(0xffffffffu, count, o);
+  if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = count;
   __syncthreads();
   if (threadIdx.x == 0) {
     int64_t s = 0;
-    for (int w = 0; w < kFlagThreads / 32; ++w) s += warp_sums[w];
+    for (int k = 0; k < kFlagThreads / 32; ++k) s += warp_sums[k];
     block_count[blockIdx.x] = s;
   }
 }
 
 // Pass 2a: representative masks in rank order; rep index = exclusive scan of
-// the flags (symmetry_resolved_ed.py:531-532).
-__global__ void k_rep_list(rsed_group_t grp, const uint32_t* bitmap, const int64_t* block_off,
-                           uint64_t* repr_masks, GroupSmemLayout lay) {
+// the flags (symmetry_resolved_ed.py:531-532).  The block also sets its ranks'
+// entries to (rep -1, g 0, alpha 0), the reference's initial table
+// (symmetry_resolved_ed.py:1359-1361); every state of a group's catalog is
+// overwritten by k_expand.
+__global__ void k_rep_list(rsed_group_t grp, const uint32_t* bitmap, const int64_t* block_off, int per_block,
+                           uint64_t* repr_masks, RsedEntry* table, GroupSmemLayout lay) {
   extern __shared__ __align__(16) unsigned char smem[];
   GroupView gv = stage_group(grp, smem, lay.binom_off, lay.perm_off, 0, 0, false, false);
   __shared__ int warp_tot[kFlagThreads / 32];
   const int kp1 = grp.n_filled + 1;
-  const int64_t word = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t r0 = word * kRanksPerThread;
-  uint32_t bits = (r0 < grp.n_states) ? bitmap[word] : 0u;
+  const int64_t first = (int64_t)blockIdx.x * per_block;
+  for (int64_t r = first + threadIdx.x; r < min(grp.n_states, first + per_block); r += blockDim.x)
+    reinterpret_cast<int4*>(table)[r] = make_int4(-1, 0, 0, 0);
+  const int64_t r0 = first + (int64_t)threadIdx.x * kRanksPerWord;
+  uint32_t bits = ((int)threadIdx.x * kRanksPerWord < per_block && r0 < grp.n_states) ? bitmap[r0 / kRanksPerWord] : 0u;
   // block-exclusive prefix of popcounts
   int c = __popc(bits);
   int incl = c;
@@ -124,9 +244,9 @@ __global__ void k_rep_list(rsed_group_t grp, const uint32_t* bitmap, const int64
   if (bits) {
     RankWalker w;
     w.init(r0, grp, gv.binom, kp1);
-    for (int i = 0; i < kRanksPerThread; ++i) {
+    for (int i = 0; i < kRanksPerWord; ++i) {
       if ((bits >> i) & 1u) repr_masks[off++] = w.m;
-      const uint32_t rest = (i < kRanksPerThread - 1) ? (bits >> (i + 1)) : 0u;
+      const uint32_t rest = (i < kRanksPerWord - 1) ? (bits >> (i + 1)) : 0u;
       if (rest == 0u) break;
       w.next();
     }
@@ -151,51 +271,98 @@ __device__ __forceinline__ double2 catalog_alpha(uint64_t m, int g, const rsed_g
   return a;
 }
 
-// Pass 2b: orbit expansion into the representative table, g ascending so the
-// last writer wins for stabilizer cosets (symmetry_resolved_ed.py:553-560),
-// plus the stabilizer bitmask (:563).
-__global__ void k_expand(rsed_group_t grp, int64_t n_orb, const uint64_t* repr_masks,
-                         RsedEntry* table, uint64_t* stab_mask, GroupSmemLayout lay, int* err) {
+// Pass 2b: orbit expansion into the representative table (g ascending, the last
+// writer wins for stabilizer cosets, symmetry_resolved_ed.py:553-560) and the
+// stabilizer bitmask (:563).  One thread per (orbit, group element), the group
+// tables transposed to [site][g] so that the lanes of an orbit read consecutive
+// words; the image, the byte-ordered angle sum and the parity come out of one
+// walk over the occupied sites.  In an orbit with a stabilizer several elements
+// reach the same state and only the largest of them writes.
+// Bound by integer issue and the shared-memory lookups of the two walks (with
+// sincos or the scattered writes taken out it ran as long); masks and ranks are
+// 32-bit up to 32 sites.  657,756 orbits of 16 elements: 267 us with one thread
+// per orbit walking its images, 309 us with 64-bit masks, 224 us in this form.
+template <typename M, typename I>
+__global__ void __launch_bounds__(256) k_expand(rsed_group_t grp, int64_t n_orb, const uint64_t* repr_masks,
+                                                RsedEntry* table, uint64_t* stab_mask, GroupSmemLayout lay, int* err) {
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ unsigned long long s_stab[256];
   const bool product_form = (grp.n_filled == 0 || grp.n_filled == grp.n_site);
-  GroupView gv = stage_group(grp, smem, lay.binom_off, lay.perm_off, lay.angle_off, lay.eta_off,
-                             true, product_form);
-  const int kp1 = grp.n_filled + 1;
-  const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= n_orb) return;
-  const uint64_t m = repr_masks[o];
-  uint64_t smask = 0;
-  for (int g = 0; g < grp.n_group; ++g) {
-    uint64_t img;
-    double2 a = catalog_alpha(m, g, grp, gv, product_form, &img);
-    int64_t idx = rsed_rank_any(img, gv.binom, kp1, grp.species_b, group_cb(grp, gv.binom, kp1));
+  const int N = grp.n_site, ng = grp.n_group, kp1 = grp.n_filled + 1;
+  I* binom = reinterpret_cast<I*>(smem + lay.binom_off);
+  double* angle = reinterpret_cast<double*>(smem + lay.angle_off);   // [site][g]
+  uint8_t* perm = smem + lay.perm_off;                               // [site][g]
+  for (int i = threadIdx.x; i < (N + 1) * kp1; i += blockDim.x) binom[i] = (I)grp.binom[i];
+  for (int i = threadIdx.x; i < ng * N; i += blockDim.x) {
+    const int g = i / N, b = i % N;
+    perm[b * ng + g] = grp.perm[i];
+    angle[b * ng + g] = grp.angle[i];
+  }
+  const int per_block = 256 / ng;  // orbits of one block and step
+  const int lo = threadIdx.x / ng, g = threadIdx.x % ng;
+  const I cb = grp.species_b ? (I)grp.binom[__popcll(grp.species_b) * kp1 + grp.n_filled_b] : 1;
+  for (int64_t o0 = (int64_t)blockIdx.x * per_block; o0 < n_orb; o0 += (int64_t)gridDim.x * per_block) {
+    __syncthreads();  // the tables are staged, the previous step's stabilizers read
+    if (threadIdx.x < per_block) s_stab[threadIdx.x] = 0ull;
+    __syncthreads();
+    const int64_t o = o0 + lo;
+    const bool act = lo < per_block && o < n_orb;
+    M m = 0, img = 0;
+    double2 a = make_double2(1.0, 0.0);
+    if (act) {
+      m = (M)repr_masks[o];
+      if (product_form) {
+        uint64_t placed;
+        a = rsed_phase_product(m, grp.perm + g * N, reinterpret_cast<const double2*>(grp.eta) + g * N, grp.fermionic,
+                               &placed);
+        img = (M)placed;
+      } else {
+        // rsed_angle_sum's order: partial sums per byte, bytes ascending
+        double total = 0.0, part = 0.0;
+        int byte = 0, par = 0;
+        for (M t = m; t; t &= t - 1) {
+          const int b = low_bit(t);
+          const int p = perm[b * ng + g];
+          // placed images above p (the shift by p + 1 in two steps: p + 1 can be the width)
+          if (grp.fermionic) par ^= count_bits((M)((img >> p) >> 1)) & 1;
+          img |= (M)1 << p;
+          if ((b >> 3) != byte) {
+            total = __dadd_rn(total, part);
+            part = 0.0;
+            byte = b >> 3;
+          }
+          part = __dadd_rn(part, angle[b * ng + g]);
+        }
+        total = __dadd_rn(total, part);
+        if (total != 0.0) sincos(total, &a.y, &a.x);  // sincos(0) = (0, 1)
+        if (par) a = rsed_cmul_exact(a, make_double2(-1.0, 0.0));
+      }
+      if (img == m) atomicOr(&s_stab[lo], 1ull << g);
+    }
+    __syncthreads();
+    if (!act) continue;
+    const uint64_t stab = s_stab[lo];
+    if (g == 0) stab_mask[o] = stab;
+    bool last = true;
+    if (__popcll(stab) > 1) {
+      for (int h = g + 1; h < ng && last; ++h) {
+        M other = 0;
+        for (M t = m; t; t &= t - 1) other |= (M)1 << perm[low_bit(t) * ng + h];
+        last = other != img;
+      }
+    }
+    if (!last) continue;
+    const int64_t idx = rank_of<M, I>(img, binom, kp1, (M)grp.species_b, cb);
     if (idx < 0 || idx >= grp.n_states) {
       rsed_flag_error(err, 1);
       continue;
     }
-    RsedEntry e;
-    e.rep = (int32_t)o;
-    e.g = g;
-    e.re = __double2float_rn(a.x);
-    e.im = __double2float_rn(a.y);
-    table[idx] = e;
-    if (img == m) smask |= 1ull << g;
-  }
-  stab_mask[o] = smask;
-}
-
-// Entries start as (rep -1, g 0, alpha 0), the reference's initial table
-// (symmetry_resolved_ed.py:1359-1361); every state of a group's catalog is
-// overwritten by k_expand.
-__global__ void k_table_init(int64_t n, RsedEntry* table) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    RsedEntry e;
-    e.rep = -1;
-    e.g = 0;
-    e.re = 0.0f;
-    e.im = 0.0f;
-    table[i] = e;
+    int4 e;
+    e.x = (int32_t)o;
+    e.y = g;
+    e.z = __float_as_int(__double2float_rn(a.x));
+    e.w = __float_as_int(__double2float_rn(a.y));
+    reinterpret_cast<int4*>(table)[idx] = e;
   }
 }
 
@@ -474,9 +641,13 @@ static int set_catalog_smem_limits() {
   static bool done = false;
   if (done) return RSED_OK;
   const int big = 160 * 1024;
-  RSED_TRY_CUDA(cudaFuncSetAttribute(k_rep_flags, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  RSED_TRY_CUDA(cudaFuncSetAttribute(k_rep_flags<uint32_t, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  RSED_TRY_CUDA(cudaFuncSetAttribute(k_rep_flags<uint32_t, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  RSED_TRY_CUDA(cudaFuncSetAttribute(k_rep_flags<uint64_t, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  RSED_TRY_CUDA(cudaFuncSetAttribute(k_rep_flags<uint64_t, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   RSED_TRY_CUDA(cudaFuncSetAttribute(k_rep_list, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  RSED_TRY_CUDA(cudaFuncSetAttribute(k_expand, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  RSED_TRY_CUDA(cudaFuncSetAttribute(k_expand<uint32_t, int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  RSED_TRY_CUDA(cudaFuncSetAttribute(k_expand<uint64_t, int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   RSED_TRY_CUDA(cudaFuncSetAttribute(k_stab_phases, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   RSED_TRY_CUDA(cudaFuncSetAttribute(k_phase_update, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   RSED_TRY_CUDA(cudaFuncSetAttribute(k_sector_members, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
@@ -513,17 +684,18 @@ struct CatalogScratch {
   int64_t* block_off;  // n_blocks + 1
   void* scan;
   size_t scan_bytes;
-  int64_t n_blocks, n_words;
+  int64_t n_blocks;
+  int per_block;  // ranks of one block
 };
 
 CatalogScratch carve_catalog_scratch(const rsed_group_t* g, void* base) {
   CatalogScratch s{};
-  s.n_words = (g->n_states + kRanksPerThread - 1) / kRanksPerThread;
-  s.n_blocks = (g->n_states + kRanksPerBlock - 1) / kRanksPerBlock;
+  s.per_block = ranks_per_block(g->n_states);
+  s.n_blocks = (g->n_states + s.per_block - 1) / s.per_block;
   char* p = reinterpret_cast<char*>(base);
   size_t off = 0;
   s.bitmap = reinterpret_cast<uint32_t*>(p + off);
-  off = align_up(off + sizeof(uint32_t) * (size_t)(s.n_blocks * kFlagThreads), 256);
+  off = align_up(off + sizeof(uint32_t) * (size_t)(s.n_blocks * (s.per_block / kRanksPerWord)), 256);
   s.block_count = reinterpret_cast<int64_t*>(p + off);
   off = align_up(off + sizeof(int64_t) * (size_t)s.n_blocks, 256);
   s.block_off = reinterpret_cast<int64_t*>(p + off);
@@ -536,8 +708,9 @@ CatalogScratch carve_catalog_scratch(const rsed_group_t* g, void* base) {
 
 extern "C" size_t rsed_catalog_scratch_bytes(const rsed_group_t* g) {
   if (!g || g->n_states < 1) return 0;
-  int64_t n_blocks = (g->n_states + kRanksPerBlock - 1) / kRanksPerBlock;
-  size_t b = align_up(sizeof(uint32_t) * (size_t)(n_blocks * kFlagThreads), 256);
+  const int per_block = ranks_per_block(g->n_states);
+  int64_t n_blocks = (g->n_states + per_block - 1) / per_block;
+  size_t b = align_up(sizeof(uint32_t) * (size_t)(n_blocks * (per_block / kRanksPerWord)), 256);
   b += align_up(sizeof(int64_t) * (size_t)n_blocks, 256);
   b += align_up(sizeof(int64_t) * (size_t)(n_blocks + 1), 256);
   b += rsed_scan_scratch_bytes(n_blocks);
@@ -556,8 +729,10 @@ extern "C" int rsed_catalog_count(const rsed_group_t* g, void* scratch, size_t s
   if (rc) return rc;
   CatalogScratch s = carve_catalog_scratch(g, scratch);
   GroupSmemLayout lay = group_smem_layout(g->n_site, g->n_filled, g->n_group, false, false);
-  k_rep_flags<<<(unsigned)s.n_blocks, kFlagThreads, lay.total, stream>>>(*g, s.bitmap,
-                                                                          s.block_count, lay);
+  const bool wide = g->n_site > 32;
+  auto flags = s.per_block == 8192 ? (wide ? k_rep_flags<uint64_t, 8> : k_rep_flags<uint32_t, 8>)
+                                   : (wide ? k_rep_flags<uint64_t, 1> : k_rep_flags<uint32_t, 1>);
+  flags<<<(unsigned)s.n_blocks, kFlagThreads, lay.total, stream>>>(*g, s.bitmap, s.block_count, s.per_block, lay);
   RSED_CHECK_LAUNCH();
   rc = rsed_exclusive_scan_i64(s.block_count, s.block_off, s.n_blocks, s.scan, s.scan_bytes, stream);
   if (rc) return rc;
@@ -583,18 +758,23 @@ extern "C" int rsed_catalog_fill(const rsed_group_t* g, const void* scratch, siz
   cudaStream_t stream = as_stream(stream_);
   CatalogScratch s = carve_catalog_scratch(g, const_cast<void*>(scratch));
   GroupSmemLayout lay0 = group_smem_layout(g->n_site, g->n_filled, g->n_group, false, false);
-  k_rep_list<<<(unsigned)s.n_blocks, kFlagThreads, lay0.total, stream>>>(*g, s.bitmap, s.block_off,
-                                                                          repr_masks, lay0);
+  k_rep_list<<<(unsigned)s.n_blocks, kFlagThreads, lay0.total, stream>>>(
+      *g, s.bitmap, s.block_off, s.per_block, repr_masks, reinterpret_cast<RsedEntry*>(table), lay0);
   RSED_CHECK_LAUNCH();
   GroupSmemLayout lay = group_smem_layout(g->n_site, g->n_filled, g->n_group, true, true);
   int* err = reinterpret_cast<int*>(s.block_count);  // block counts are consumed by now
   RSED_TRY_CUDA(cudaMemsetAsync(err, 0, sizeof(int), stream));
-  k_table_init<<<(unsigned)((g->n_states + 255) / 256), 256, 0, stream>>>(
-      g->n_states, reinterpret_cast<RsedEntry*>(table));
-  RSED_CHECK_LAUNCH();
-  const unsigned nb = (unsigned)((n_orbits + 255) / 256);
-  k_expand<<<nb, 256, lay.total, stream>>>(*g, n_orbits, repr_masks,
-                                           reinterpret_cast<RsedEntry*>(table), stab_mask, lay, err);
+  const int per_block = 256 / g->n_group;
+  const int64_t steps = (n_orbits + per_block - 1) / per_block;
+  int dev = 0, n_sm = 0;
+  RSED_TRY_CUDA(cudaGetDevice(&dev));
+  RSED_TRY_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+  // eight blocks per SM walk the orbits: the tables are staged once per block
+  // (one step per block measured 20 us slower on 657,756 orbits)
+  const int64_t wave = (int64_t)n_sm * 8;
+  auto expand = g->n_site > 32 ? k_expand<uint64_t, int64_t> : k_expand<uint32_t, int32_t>;
+  expand<<<(unsigned)(steps < wave ? steps : wave), 256, lay.total, stream>>>(
+      *g, n_orbits, repr_masks, reinterpret_cast<RsedEntry*>(table), stab_mask, lay, err);
   RSED_CHECK_LAUNCH();
   int herr = 0;
   RSED_TRY_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, stream));

@@ -100,3 +100,45 @@ def test_fock_amplitudes_sizes(family, size, nf, theta, species):
         np.testing.assert_allclose(a[order], np.array([ref[int(k)] for k in keys]), atol=1e-14, rtol=0)
         dense = ed.expand_sector_state_to_fock_dense(c, basis).cpu().numpy()
         np.testing.assert_array_equal(dense[dense != 0], a)
+
+
+def _check_catalog(cat, ref):
+    np.testing.assert_array_equal(np.array(cat.representative_mask_list, dtype=np.uint64), ref["reprs"])
+    np.testing.assert_array_equal(cat.rep_rank_table, ref["rep_rank"])
+    np.testing.assert_array_equal(cat.rep_sym_table, ref["rep_sym"])
+    assert [list(x) for x in cat.stabilizer_g_indices_list] == [list(x) for x in ref["stab_g"]]
+    # both sides round a double within one ulp of the phase to float32
+    a, b = cat.rep_amp_table, np.asarray(ref["rep_amp"], dtype=np.complex64)
+    assert np.abs((a - b).view(np.float32)).max() <= 6e-8
+
+
+# 32-bit and 64-bit images, one and eight ranks per thread (2^20 states and
+# more), no particles, all sites taken, |G| that does not divide a block
+@pytest.mark.parametrize("family,size,nf,theta", [
+    ("haldane", (2, 3), 0, (0.2, 0.1)),
+    ("haldane", (2, 3), 12, (0.2, 0.1)),
+    ("heisenberg", (13, 1), 6, (0.3, 0.0)),
+    ("checkerboard", (3, 3), 4, (0.25, 0.4)),
+    ("checkerboard", (4, 4), 3, None),
+    ("checkerboard", (3, 6), 3, (0.1, 0.3)),
+    ("checkerboard", (3, 6), 6, (0.1, 0.3)),
+    ("heisenberg", (23, 1), 11, None),
+])
+def test_catalog_sizes(family, size, nf, theta):
+    data, _, cat, _, _ = _case(family, size, nf, theta)
+    _check_catalog(data.orbit_catalog, cat)
+
+
+def test_catalog_element_without_few_distances():
+    """A reflection moves every site by another distance: images bit by bit."""
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import models
+
+    n, nf = 18, 9
+    m = models.build_heisenberg_second_quantized_model(n, 1.0)
+    ops = [ed.Symmetry_Operation("e", list(range(1, n + 1))), ed.Symmetry_Operation("r", list(range(n, 0, -1)))]
+    G = ed.Finite_Symmetry_Group("reflection", ops, identity_idx=0)
+    cat = ed.build_symmetry_orbit_catalog(second_quantized_model=m, n_filled=nf, symmetry_group=G,
+                                          particle_statistics=m.particle_statistics)
+    perm0, eta = port.group_arrays(G)
+    _check_catalog(cat, port.catalog(n, nf, perm0, eta, False))
