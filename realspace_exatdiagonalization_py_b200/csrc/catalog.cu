@@ -138,10 +138,6 @@ __device__ bool stage_moves(const rsed_group_t& grp, const uint8_t* perm, GroupM
   return __syncthreads_and(fits);
 }
 
-__device__ __forceinline__ int64_t group_cb(const rsed_group_t& grp, const int64_t* binom, int kp1) {
-  return grp.species_b ? binom[__popcll(grp.species_b) * kp1 + grp.n_filled_b] : 1;
-}
-
 // Pass 1: representative flags as a bitmap (symmetry_resolved_ed.py:519-528).
 // A thread tests R consecutive ranks (32 / R lanes share a bitmap word) against
 // all |G| images at once, each move class loaded once for the R masks.  Bound by
@@ -392,18 +388,15 @@ __global__ void k_stab_phases(rsed_group_t grp, int64_t n_orb, const uint64_t* r
   }
 }
 
-// K4: flux phase update in product form (symmetry_resolved_ed.py:1248-1268).
-__global__ void k_phase_update(rsed_group_t grp, int64_t n_orb, const uint64_t* repr_masks,
-                               const uint64_t* stab_mask, const int64_t* stab_off,
-                               double2* stab_phase, RsedEntry* table, GroupSmemLayout lay,
-                               int* err) {
+// K4: flux phase update in product form (symmetry_resolved_ed.py:1248-1268),
+// stabilizer phases of every orbit, ascending g (:1248-1257).
+__global__ void k_phase_stab(rsed_group_t grp, int64_t n_orb, const uint64_t* repr_masks, const uint64_t* stab_mask,
+                             const int64_t* stab_off, double2* stab_phase, GroupSmemLayout lay) {
   extern __shared__ __align__(16) unsigned char smem[];
   GroupView gv = stage_group(grp, smem, lay.binom_off, lay.perm_off, 0, lay.eta_off, false, true);
-  const int kp1 = grp.n_filled + 1;
   const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= n_orb) return;
   const uint64_t m = repr_masks[o];
-  // stabilizer phases first (reference order: :1248-1257)
   uint64_t s = stab_mask[o];
   int64_t off = stab_off[o];
   while (s) {
@@ -413,25 +406,61 @@ __global__ void k_phase_update(rsed_group_t grp, int64_t n_orb, const uint64_t* 
         rsed_phase_product(m, gv.perm + g * grp.n_site, gv.eta + g * grp.n_site, grp.fermionic, &img);
     s &= s - 1;
   }
-  for (int g = 0; g < grp.n_group; ++g) {
-    uint64_t img;
-    double2 a =
-        rsed_phase_product(m, gv.perm + g * grp.n_site, gv.eta + g * grp.n_site, grp.fermionic, &img);
-    int64_t idx = rsed_rank_any(img, gv.binom, kp1, grp.species_b, group_cb(grp, gv.binom, kp1));
-    if (idx < 0 || idx >= grp.n_states) {
-      rsed_flag_error(err, 1);
-      continue;
-    }
-    if (table[idx].rep != (int32_t)o) {
+}
+
+// The amplitudes of the representative table.  The permutations are those the
+// table was built with, so every state keeps its orbit and its (last) group
+// element and only the phase is new: one thread per table entry, read and
+// written in rank order.  The entry is checked against the group: its element
+// has to map the representative to the state of this rank.
+// Bound by the walk over the occupied sites (a 16-B lookup and an unfused
+// complex product per site, a lookup per site of the image's rank).  10.5
+// million states, 32 sites: 247 us with one thread per orbit, its |G| entries
+// read and rewritten at random, 145 us in this form (135 without the products).
+template <typename M, typename I>
+__global__ void __launch_bounds__(256) k_phase_table(rsed_group_t grp, int64_t n_orb, const uint64_t* repr_masks,
+                                                     int4* table, GroupSmemLayout lay, int* err) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int N = grp.n_site, ng = grp.n_group, kp1 = grp.n_filled + 1;
+  I* binom = reinterpret_cast<I*>(smem + lay.binom_off);
+  double2* eta = reinterpret_cast<double2*>(smem + lay.eta_off);
+  uint8_t* perm = smem + lay.perm_off;
+  for (int i = threadIdx.x; i < (N + 1) * kp1; i += blockDim.x) binom[i] = (I)grp.binom[i];
+  bool twisted = false;
+  for (int i = threadIdx.x; i < ng * N; i += blockDim.x) {
+    const double2 v = reinterpret_cast<const double2*>(grp.eta)[i];
+    twisted |= v.x != 1.0 || v.y != 0.0;
+    eta[i] = v;
+    perm[i] = grp.perm[i];
+  }
+  const bool unit = __syncthreads_or(twisted) == 0;  // products of exact ones are left out
+  const I cb = grp.species_b ? binom[__popcll(grp.species_b) * kp1 + grp.n_filled_b] : 1;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < grp.n_states; r += stride) {
+    int4 e = table[r];
+    if (e.x < 0 || e.x >= n_orb || e.y < 0 || e.y >= ng) {
       rsed_flag_error(err, 2);
       continue;
     }
-    RsedEntry e;
-    e.rep = (int32_t)o;
-    e.g = g;
-    e.re = __double2float_rn(a.x);
-    e.im = __double2float_rn(a.y);
-    table[idx] = e;
+    const int base = e.y * N;
+    M img = 0;
+    int par = 0;
+    double2 a = make_double2(1.0, 0.0);
+    for (M t = (M)__ldg(repr_masks + e.x); t; t &= t - 1) {
+      const int b = low_bit(t);
+      const int p = perm[base + b];
+      if (grp.fermionic) par ^= count_bits((M)((img >> p) >> 1)) & 1;
+      img |= (M)1 << p;
+      if (!unit) a = rsed_cmul_exact(a, eta[base + b]);
+    }
+    if (grp.fermionic) a = rsed_cmul_exact(a, make_double2(par ? -1.0 : 1.0, 0.0));
+    if ((int64_t)rank_of<M, I>(img, binom, kp1, (M)grp.species_b, cb) != r) {
+      rsed_flag_error(err, 2);
+      continue;
+    }
+    e.z = __float_as_int(__double2float_rn(a.x));
+    e.w = __float_as_int(__double2float_rn(a.y));
+    table[r] = e;
   }
 }
 
@@ -649,9 +678,21 @@ static int set_catalog_smem_limits() {
   RSED_TRY_CUDA(cudaFuncSetAttribute(k_expand<uint32_t, int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   RSED_TRY_CUDA(cudaFuncSetAttribute(k_expand<uint64_t, int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   RSED_TRY_CUDA(cudaFuncSetAttribute(k_stab_phases, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  RSED_TRY_CUDA(cudaFuncSetAttribute(k_phase_update, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  RSED_TRY_CUDA(cudaFuncSetAttribute(k_phase_stab, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  RSED_TRY_CUDA(cudaFuncSetAttribute(k_phase_table<uint32_t, int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  RSED_TRY_CUDA(cudaFuncSetAttribute(k_phase_table<uint64_t, int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   RSED_TRY_CUDA(cudaFuncSetAttribute(k_sector_members, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   done = true;
+  return RSED_OK;
+}
+
+// Blocks of `threads` that the device holds at once.
+static int blocks_of_one_wave(const void* kern, int threads, size_t smem, int64_t* out) {
+  int dev = 0, n_sm = 0, per_sm = 0;
+  RSED_TRY_CUDA(cudaGetDevice(&dev));
+  RSED_TRY_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+  RSED_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
+  *out = (int64_t)n_sm * (per_sm > 0 ? per_sm : 1);
   return RSED_OK;
 }
 
@@ -766,13 +807,12 @@ extern "C" int rsed_catalog_fill(const rsed_group_t* g, const void* scratch, siz
   RSED_TRY_CUDA(cudaMemsetAsync(err, 0, sizeof(int), stream));
   const int per_block = 256 / g->n_group;
   const int64_t steps = (n_orbits + per_block - 1) / per_block;
-  int dev = 0, n_sm = 0;
-  RSED_TRY_CUDA(cudaGetDevice(&dev));
-  RSED_TRY_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-  // eight blocks per SM walk the orbits: the tables are staged once per block
+  // one wave of blocks walks the orbits: the tables are staged once per block
   // (one step per block measured 20 us slower on 657,756 orbits)
-  const int64_t wave = (int64_t)n_sm * 8;
   auto expand = g->n_site > 32 ? k_expand<uint64_t, int64_t> : k_expand<uint32_t, int32_t>;
+  int64_t wave = 0;
+  rc = blocks_of_one_wave((const void*)expand, 256, lay.total, &wave);
+  if (rc) return rc;
   expand<<<(unsigned)(steps < wave ? steps : wave), 256, lay.total, stream>>>(
       *g, n_orbits, repr_masks, reinterpret_cast<RsedEntry*>(table), stab_mask, lay, err);
   RSED_CHECK_LAUNCH();
@@ -840,9 +880,16 @@ extern "C" int rsed_phase_update(const rsed_group_t* g, int64_t n_orbits, const 
   if (rc) return rc;
   GroupSmemLayout lay = group_smem_layout(g->n_site, g->n_filled, g->n_group, true, false);
   RSED_TRY_CUDA(cudaMemsetAsync(err_dev, 0, sizeof(int), stream));
-  k_phase_update<<<(unsigned)((n_orbits + 255) / 256), 256, lay.total, stream>>>(
-      *g, n_orbits, repr_masks, stab_mask, stab_off, reinterpret_cast<double2*>(stab_phase),
-      reinterpret_cast<RsedEntry*>(table), lay, err_dev);
+  k_phase_stab<<<(unsigned)((n_orbits + 255) / 256), 256, lay.total, stream>>>(
+      *g, n_orbits, repr_masks, stab_mask, stab_off, reinterpret_cast<double2*>(stab_phase), lay);
+  RSED_CHECK_LAUNCH();
+  auto kern = g->n_site > 32 ? k_phase_table<uint64_t, int64_t> : k_phase_table<uint32_t, int32_t>;
+  int64_t wave = 0;
+  rc = blocks_of_one_wave((const void*)kern, 256, lay.total, &wave);
+  if (rc) return rc;
+  const int64_t blocks = (g->n_states + 255) / 256;
+  kern<<<(unsigned)(blocks < wave ? blocks : wave), 256, lay.total, stream>>>(*g, n_orbits, repr_masks,
+                                                                            reinterpret_cast<int4*>(table), lay, err_dev);
   RSED_CHECK_LAUNCH();
   return RSED_OK;
 }
