@@ -249,6 +249,11 @@ int rsed_triplets_fill(const rsed_model_t* model, int64_t n_rows, const int32_t*
  * symmetry_resolved_ed.py:1965-1976, 1979-2069). */
 int rsed_csr_spmv(int64_t n_rows, const int64_t* row_ptr, const int32_t* col_idx,
                   const double* vals, int32_t n_vec, const double* x, double* y, void* stream);
+/* The same with any layout of the vectors: element r of vector v of x and y at
+ * [r*row_stride + v*vec_stride] (complex elements), e.g. row-major blocks. */
+int rsed_csr_spmv_strided(int64_t n_rows, const int64_t* row_ptr, const int32_t* col_idx,
+                          const double* vals, int32_t n_vec, const double* x, double* y,
+                          int64_t row_stride, int64_t vec_stride, void* stream);
 
 /* ---- K9: sector state -> Fock amplitudes ------------------------------------
  * Replaces _expand_sector_state_to_fock_amplitudes

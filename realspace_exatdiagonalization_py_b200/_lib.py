@@ -204,6 +204,10 @@ SIGNATURES = {
         c_int,
         [c_int64, c_void_p, c_void_p, c_void_p, c_int32, c_void_p, c_void_p, c_void_p],
     ),
+    "rsed_csr_spmv_strided": (
+        c_int,
+        [c_int64, c_void_p, c_void_p, c_void_p, c_int32, c_void_p, c_void_p, c_int64, c_int64, c_void_p],
+    ),
     "rsed_lanczos_partial_len": (c_int64, [c_int64, c_int32, c_int32, c_int32]),
     "rsed_lanczos_coef_len": (c_int64, [c_int32, c_int32]),
     "rsed_lanczos_max_block": (c_int, []),

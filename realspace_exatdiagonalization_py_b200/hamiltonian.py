@@ -239,8 +239,7 @@ class MatrixFreeHamiltonian:
         """``H x`` for ``ncols`` compact column vectors ``x [n, ncols]`` on the device."""
         if self.precision == 32:
             return self.adjoint_device(x, ncols, precision=32)
-        xt = x.reshape(self.n, ncols).to(torch.complex128).T.contiguous()
-        return self.csr().matvec(xt).T.reshape(self.n, ncols)
+        return self.csr().matmat(x.reshape(self.n, ncols))
 
     def adjoint_device(self, x: torch.Tensor, ncols: int = 1, precision: int = 64) -> torch.Tensor:
         """``H^dagger x`` through the streaming orbit-layout apply of the
@@ -366,6 +365,18 @@ class DeviceCSR:
         _lib.check(_lib.lib().rsed_csr_spmv(self.n, _lib.ptr(self.row_ptr), _lib.ptr(self.col),
                                             _lib.ptr(self.val), nvec, _lib.ptr(x), _lib.ptr(y),
                                             _lib.stream_ptr()))
+        return y
+
+    def matmat(self, x: torch.Tensor) -> torch.Tensor:
+        """``A x`` for a row-major block ``x [n, k]``."""
+        x = x.to(torch.complex128).contiguous()
+        if x.is_conj() or x.is_neg():  # the kernel reads the memory as it is
+            x = x.resolve_conj().resolve_neg()
+        k = x.shape[1]
+        y = torch.empty_like(x)
+        _lib.check(_lib.lib().rsed_csr_spmv_strided(self.n, _lib.ptr(self.row_ptr), _lib.ptr(self.col),
+                                                    _lib.ptr(self.val), k, _lib.ptr(x), _lib.ptr(y), k, 1,
+                                                    _lib.stream_ptr()))
         return y
 
 

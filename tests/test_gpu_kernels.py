@@ -142,3 +142,33 @@ def test_catalog_element_without_few_distances():
                                           particle_statistics=m.particle_statistics)
     perm0, eta = port.group_arrays(G)
     _check_catalog(cat, port.catalog(n, nf, perm0, eta, False))
+
+
+# rows of no, few and many entries (shorter and longer than the lanes of a row
+# times their entries in flight), row counts off the block, 1 to 9 vectors in
+# both layouts
+@pytest.mark.parametrize("n,most,k", [(1, 1, 1), (31, 3, 2), (257, 40, 3), (1000, 90, 4), (1023, 200, 7), (300, 33, 9)])
+def test_csr_products(n, most, k):
+    import scipy.sparse as sp
+    import torch
+
+    from realspace_exatdiagonalization_py_b200.hamiltonian import DeviceCSR
+
+    rng = np.random.default_rng(n)
+    per = rng.integers(0, most + 1, n)
+    rows = np.repeat(np.arange(n), per)
+    cols = rng.integers(0, n, per.sum())
+    vals = rng.standard_normal(per.sum()) + 1j * rng.standard_normal(per.sum())
+    A = sp.csr_matrix((vals, (rows, cols)), shape=(n, n))
+    x = rng.standard_normal((n, k)) + 1j * rng.standard_normal((n, k))
+    dev = DeviceCSR(*(torch.from_numpy(a).cuda() for a in (rows, cols, vals)), n)
+    tol = 1e-15 * (most + 1) * 20  # ulps of sums of `most` products of size about 10 at most
+    xd = torch.from_numpy(x).cuda()
+    if not per.sum():  # a matrix without entries has no buffers: refused
+        with pytest.raises(ValueError):
+            dev.matmat(xd)
+        return
+    np.testing.assert_allclose(dev.matmat(xd).cpu().numpy(), A @ x, atol=tol, rtol=0)
+    np.testing.assert_allclose(dev.matmat(xd.conj()).cpu().numpy(), A @ x.conj(), atol=tol, rtol=0)
+    np.testing.assert_allclose(dev.matvec(xd.T.contiguous()).T.cpu().numpy(), A @ x, atol=tol, rtol=0)
+    np.testing.assert_allclose(dev.matvec(xd[:, 0].contiguous()).cpu().numpy(), A @ x[:, 0], atol=tol, rtol=0)
