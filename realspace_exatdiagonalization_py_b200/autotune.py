@@ -139,7 +139,8 @@ class Autotuner:
             try:
                 p = LanczosParams(**{**base.__dict__, "precision": precision, "block": max(cfg.block_sizes)})
                 sol = BatchedSectorSolver(dm, sset, sectors, nev, precision=precision, params=p, config=cfg)
-                sol.solve(None, vectors=False, host=False)  # capture graphs, warm caches
+                for _ in range(2):  # warm caches, then capture the graphs
+                    sol.solve(None, vectors=False, host=False)
                 # two sets of start blocks: convergence is decided at restarts,
                 # so a solve's step count is quantised by the restart period and
                 # one start set can favour either basis length; the trials

@@ -27,7 +27,7 @@ from .sector import SectorSet
 # rsed_apply_h variants: 0 = automatic (projection table when present),
 # 999 = automatic on-the-fly mapping
 APPLY_AUTO, APPLY_ON_THE_FLY = 0, 999
-# one thread-block cluster per sector only pays while a sector is a few hundred KB
+# largest basis of the persistent path's automatic use (an explicit cluster size)
 PERSISTENT_MAX_ORBITS = 1 << 16
 
 
@@ -64,7 +64,15 @@ class BatchedSectorSolver:
 
     def __init__(self, model: DeviceModel, sset: SectorSet, sectors: list[int], nev: int, *,
                  precision: int = 64, params: LanczosParams | None = None, poll: int = 16,
-                 graph: bool = True, persistent: int = 4, config: SolverConfig | None = None):
+                 graph: bool = True, persistent: int | None = None, config: SolverConfig | None = None):
+        """``persistent`` asks for the one-launch path with clusters of that
+        size where it applies (bases up to ``PERSISTENT_MAX_ORBITS``, uniform
+        blocks of 1, 2 or 4).  The default is the per-iteration kernels: on
+        every basis measured (810 to 12,586 orbits, 12 to 20 sectors, blocks
+        of 2 and 4, both precisions) they are faster, 10.7 against 3.9 ms on
+        16 sectors of 810 orbits, 398 against 21 ms on 12 sectors of 11,240,
+        since one cluster per sector leaves most SMs idle and re-derives its
+        hops in every product."""
         p = params or LanczosParams()
         if p.precision != precision:
             p = LanczosParams(**{**p.__dict__, "precision": precision})
@@ -73,8 +81,8 @@ class BatchedSectorSolver:
         if config is None:
             bs = (p.block,) * len(self.sectors)
             small = model.catalog.n_orbits <= PERSISTENT_MAX_ORBITS
-            config = SolverConfig(bs, persistent if small and persistent_ok(bs) and persistent in (1, 2, 4, 8)
-                                  else 0, projection=model.proj is not None, n_slots=p.n_slots, poll=poll)
+            cluster = persistent if small and persistent_ok(bs) and persistent in (1, 2, 4, 8) else 0
+            config = SolverConfig(bs, cluster, projection=model.proj is not None, n_slots=p.n_slots, poll=poll)
         if len(config.block_sizes) != len(self.sectors):
             raise ValueError("config.block_sizes needs one entry per sector")
         if config.persistent and not persistent_ok(config.block_sizes):
@@ -149,6 +157,22 @@ def projection_precisions(model: DeviceModel, precision: int, fraction: float = 
         return (64,)
     free, _ = torch.cuda.mem_get_info(model.hdiag.device)
     return (64, 32) if model.projection_bytes((64, 32)) <= fraction * free else (32,)
+
+
+def ensure_projection(model: DeviceModel, sset: SectorSet, precision: int) -> None:
+    """Build the model's projection table unless it has one, it takes more than
+    half the free memory (asked only for tables above 1 GiB: the query can
+    stall for 100 ms), or there is no room for it; without it the products
+    run on the fly."""
+    if model.proj is not None:
+        return
+    nbytes = model.projection_bytes((precision,))
+    if nbytes > 1 << 30 and nbytes > 0.5 * torch.cuda.mem_get_info(model.hdiag.device)[0]:
+        return
+    try:
+        model.build_projection(sset.sqrt_stab, precisions=projection_precisions(model, precision))
+    except torch.cuda.OutOfMemoryError:
+        model.drop_projection()
 
 
 def plan_waves(n_orbits: int, block_sizes: list[int], budget: int, n_slots: int = 16,

@@ -209,14 +209,11 @@ def solve_sectors_batched(ed_data, sector_ids: list[int], *, nev: int = 5, preci
         else:
             big.append(s)
     if big:
-        from .batched import lanczos_footprint_bytes, plan_waves, projection_precisions
+        from .batched import ensure_projection, lanczos_footprint_bytes, plan_waves
 
         p = params or LanczosParams(precision=precision)
-        if dm.proj is None and (config is None or config.projection):
-            # the streaming matvec, when its table fits half the free memory
-            free, _ = torch.cuda.mem_get_info()
-            if dm.projection_bytes((precision,)) <= 0.5 * free:
-                dm.build_projection(sset.sqrt_stab, precisions=projection_precisions(dm, precision))
+        if config is None or config.projection:
+            ensure_projection(dm, sset, precision)  # the streaming matvec, when its table fits
         cache = ed_data.__dict__.setdefault("_solvers", {})
         resident = None
         if not (config is None and autotune):

@@ -101,6 +101,7 @@ class DeviceModel:
                                          _lib.ptr(self._di), _lib.ptr(self._dj), _lib.ptr(self._dv),
                                          _lib.ptr(self.hdiag), _lib.stream_ptr(stream)))
         self.proj = None
+        self._hops = None  # (hop count, row offsets): the same at every flux point
         self.refresh()
 
     def refresh(self) -> None:
@@ -126,7 +127,7 @@ class DeviceModel:
             skip = ("rowptr", "cg") if self.proj.get("shared") else ()
             return sum(int(t.numel() * t.element_size()) for k, t in self.proj.items()
                        if torch.is_tensor(t) and k not in skip)
-        n = self.count_hops()
+        n = self.count_hops() if self._hops is None else self._hops[0]
         return 8 * (self.catalog.n_orbits + 1) + n * (4 + (16 if 64 in precisions else 0)
                                                       + (8 if 32 in precisions else 0))
 
@@ -140,7 +141,7 @@ class DeviceModel:
         n = ctypes.c_int64()
         _lib.check(lib.rsed_proj_count(ctypes.byref(self.c), _lib.ptr(rowptr), ctypes.byref(n),
                                        _lib.ptr(scratch), scratch.numel(), _lib.stream_ptr(stream)))
-        self._rowptr_cache = rowptr
+        self._hops = (int(n.value), rowptr)
         return int(n.value)
 
     def build_projection(self, sqrt_stab: torch.Tensor, precisions=(64, 32), stream=None,
@@ -168,8 +169,9 @@ class DeviceModel:
                          "table_version": self.catalog.version, "shared": True}
             self.refresh()
             return
-        n = self.count_hops(stream)
-        rowptr = self._rowptr_cache
+        if self._hops is None:
+            self.count_hops(stream)
+        n, rowptr = self._hops
         dev = rowptr.device
         cg = torch.empty(max(n, 1), dtype=torch.int32, device=dev)
         w64 = torch.empty(max(n, 1), dtype=torch.complex128, device=dev) if 64 in want else None

@@ -13,6 +13,8 @@ from __future__ import annotations
 
 import ctypes
 import math
+import os
+from concurrent.futures import ThreadPoolExecutor
 from dataclasses import dataclass
 
 import numpy as np
@@ -79,12 +81,31 @@ def start_block(n: int, b: int, seed: int = 12345) -> np.ndarray:
 
     Column 0 with ``seed=12345`` is the reference's ``v0``
     (``symmetry_resolved_ed.py:2291-2293``)."""
-    cols = []
-    for j in range(b):
-        rng = np.random.default_rng(seed + 7919 * j)
+    return start_blocks([(n, b, seed)])[0]
+
+
+def start_blocks(specs) -> list[np.ndarray]:
+    """:func:`start_block` of every ``(n, b, seed)``.  The columns are drawn by
+    a few threads at once when there is enough to draw (numpy's generators run
+    without the interpreter lock): 112,720 rows x 4 columns in 4 ms instead of
+    12 ms."""
+    def column(job):
+        n, seed = job
+        rng = np.random.default_rng(seed)
         v = rng.standard_normal(n) + 1j * rng.standard_normal(n)
-        cols.append(v / np.linalg.norm(v))
-    return np.stack(cols, axis=1)
+        return v / np.linalg.norm(v)
+
+    jobs = [(n, seed + 7919 * j) for n, b, seed in specs for j in range(b)]
+    if len(jobs) > 1 and sum(n for n, _ in jobs) >= 1 << 16:
+        with ThreadPoolExecutor(max_workers=min(len(jobs), 16, os.cpu_count() or 1)) as pool:
+            cols = list(pool.map(column, jobs))
+    else:
+        cols = [column(job) for job in jobs]
+    out, at = [], 0
+    for _, b, _ in specs:
+        out.append(np.stack(cols[at: at + b], axis=1))
+        at += b
+    return out
 
 
 def _auto_keep(nev: int, b: int, n_slots: int) -> int:
@@ -170,6 +191,7 @@ class LanczosBatch:
         self._graph = None
         self._graph_iters = None
         self._spans = None  # restart-aligned graphs: ((head, launches), (cycle, launches))
+        self._aligned_runs = 0
 
     @property
     def n_inst(self) -> int:
@@ -184,19 +206,19 @@ class LanczosBatch:
         self.W.zero_()
         lib = _lib.lib()
         sp = _lib.stream_ptr(stream)
+        # seeded blocks are deterministic: drawn on the host once per
+        # (sector, width, seed) and kept on the device for later solves
+        cache = self.__dict__.setdefault("_start_cache", {})
+        keys = [None if blocks is not None and blocks[i] is not None else
+                (s, self.sset.dims[s], self.block_sizes[i], 12345 if seeds is None else seeds[i])
+                for i, s in enumerate(self.inst_sectors)]
+        new = [k for k in dict.fromkeys(keys) if k is not None and k not in cache]
+        for key, blk in zip(new, start_blocks([k[1:] for k in new])):
+            cache[key] = torch.from_numpy(blk).to(self.dev)
         for i, s in enumerate(self.inst_sectors):
             d = self.sset.dims[s]
             b = self.block_sizes[i]
-            blk = blocks[i] if blocks is not None else None
-            if blk is None:
-                # seeded blocks are deterministic: drawn on the host once per
-                # (sector, width, seed) and kept on the device for later solves
-                seed = 12345 if seeds is None else seeds[i]
-                key = (s, d, b, seed)
-                cache = self.__dict__.setdefault("_start_cache", {})
-                if key not in cache:
-                    cache[key] = torch.from_numpy(start_block(d, b, seed)).to(self.dev)
-                blk = cache[key]
+            blk = blocks[i] if keys[i] is None else cache[keys[i]]
             if isinstance(blk, np.ndarray):
                 blk = torch.from_numpy(np.ascontiguousarray(blk, dtype=np.complex128))
             blk = blk.to(self.dev, torch.complex128, non_blocking=True).reshape(d, -1).contiguous()
@@ -281,37 +303,44 @@ class LanczosBatch:
                 break
         return self._final_status()
 
-    def run_aligned(self, max_iter: int = 12000, poll: int = 8) -> np.ndarray:
-        """``run(graph=True)`` from a fresh ``start()``, with the graphs cut at
-        the restarts: a head graph of ``keep`` steps that launches no Ritz
-        check, then a cycle graph of ``restart_period`` steps that checks (and
-        restarts) after its last step only, replayed until every instance
-        converged.  Convergence is only decided at restarts (unless
-        ``check_every`` falls due first), so the host polls once per cycle and
-        no step runs past the restart that finished the batch.  The kernels
-        and their order are those of ``run`` minus the launches that find no
-        check due, so the results are the same.  A periodic check that would
-        fall inside a graph hands the rest of the solve to ``run``'s per-step
-        path."""
+    def run_aligned(self, max_iter: int = 12000, poll: int = 8, graph: bool = True) -> np.ndarray:
+        """``run(graph=True)`` from a fresh ``start()``, cut at the restarts: a
+        head of ``keep`` steps that launches no Ritz check, then cycles of
+        ``restart_period`` steps that check (and restart) after their last
+        step only, until every instance converged.  Convergence is only
+        decided at restarts (unless ``check_every`` falls due first), so the
+        host polls once per cycle and no step runs past the restart that
+        finished the batch.  The kernels and their order are those of ``run``
+        minus the launches that find no check due, so the results are the
+        same.  The first solve of a batch launches its spans directly; head
+        and cycle are captured as graphs by the second one (a capture costs
+        10 to 60 ms and saves a tenth of a later solve, so a batch that solves
+        once never pays for it).  ``graph=False`` never captures.  A periodic
+        check that would fall inside a span hands the rest of the solve to
+        ``run``'s per-step path."""
         h, period = self.keep, self.restart_period
         check_inside = self.periodic_check_in
         if h < 1 or period < 1 or check_inside(1, h):
-            return self.run(max_iter, poll, graph=True)
-        if self._spans is None:
-            self.iterate(h)  # first solve: every kernel runs once before the captures
+            return self.run(max_iter, poll, graph=graph)
+        if graph and self._spans is None and self._aligned_runs > 0:
+            # every kernel has run before the captures
             self._spans = (self.capture_span(h, False), self.capture_span(period, True))
-        else:
-            g, n = self._spans[0]
+        self._aligned_runs += 1
+
+        def span(k):
+            if self._spans is None:
+                self.iterate_span((h, period)[k], bool(k))
+                return
+            g, n = self._spans[k]
             g.replay()
             self.replays += 1
             self.replayed_launches += n
+
+        span(0)
         it = h
-        g, n = self._spans[1]
         converged = False
         while it < max_iter and not check_inside(it + 1, it + period - 1):
-            g.replay()
-            self.replays += 1
-            self.replayed_launches += n
+            span(1)
             it += period
             if self.done():
                 converged = True
@@ -483,10 +512,19 @@ def diagonalize_block_dense(H, *, nev: int = 5):
 
 
 def _solve_sector(model: DeviceModel, sset: SectorSet, s: int, nev: int, params: LanczosParams):
+    from .batched import APPLY_AUTO, ensure_projection
+
+    if params.apply_variant == APPLY_AUTO:
+        # the table costs one or two products and serves every step and the
+        # model's other sectors
+        try:
+            ensure_projection(model, sset, params.precision)
+        except ValueError:
+            model.drop_projection()  # beyond the table's limits (2^26 orbits, 48 KB of terms): on the fly
     b = LanczosBatch(model, sset, [s], nev, params)
     b.load_start(None)
     b.start()
-    b.run()
+    b.run_aligned(graph=False)
     if params.precision == 32:
         refine(b)
     vals = b.eigenvalues()[0]
