@@ -450,10 +450,12 @@ int rsed_proj_apply(const rsed_model_t& md, const rsed_sectors_t& sc, const void
     // columns (3.7 ms vs 4.5 ms with 16-B segments; at 32 columns 1.48 ms in
     // one chunk vs 1.95 ms in chunks of 16 that keep x in L2); FP64 with
     // 16-B segments and 16-column chunks, one after another (7.5 ms; wider
-    // segments spill into lower occupancy), except at 17-32 columns.  Small (latency-bound) bases prefer 16 columns
-    // per chunk with all chunks in one launch, for more warps in flight.
+    // segments spill into lower occupancy), except at 17-32 columns.  Small (latency-bound) bases prefer up to 16
+    // columns per chunk with all chunks in one launch, for more warps in flight.
     if (md.n_orbits < 65536) {
-      variant = 416;
+      int nc = 4;
+      while (nc < sc.n_cols && nc < 16) nc *= 2;  // a narrow block keeps every lane of its slots
+      variant = 400 + nc;
     } else if (precision == 32) {
       int nc = 8;
       while (nc < sc.n_cols && nc < 64) nc *= 2;

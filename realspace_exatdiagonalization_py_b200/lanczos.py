@@ -13,7 +13,6 @@ from __future__ import annotations
 
 import ctypes
 import math
-import os
 from concurrent.futures import ThreadPoolExecutor
 from dataclasses import dataclass
 
@@ -81,30 +80,26 @@ def start_block(n: int, b: int, seed: int = 12345) -> np.ndarray:
 
     Column 0 with ``seed=12345`` is the reference's ``v0``
     (``symmetry_resolved_ed.py:2291-2293``)."""
-    return start_blocks([(n, b, seed)])[0]
+    x = _normal_streams(2 * n, [seed + 7919 * j for j in range(b)])
+    v = x[:, :n] + 1j * x[:, n:]
+    return np.stack([c / np.linalg.norm(c) for c in v], axis=1)
 
 
-def start_blocks(specs) -> list[np.ndarray]:
-    """:func:`start_block` of every ``(n, b, seed)``.  The columns are drawn by
-    a few threads at once when there is enough to draw (numpy's generators run
-    without the interpreter lock): 112,720 rows x 4 columns in 4 ms instead of
-    12 ms."""
-    def column(job):
-        n, seed = job
-        rng = np.random.default_rng(seed)
-        v = rng.standard_normal(n) + 1j * rng.standard_normal(n)
-        return v / np.linalg.norm(v)
+def _normal_streams(n: int, seeds: list[int]) -> np.ndarray:
+    """``[len(seeds), n]``: the first ``n`` standard normals of every seed's
+    generator, drawn by a thread per seed when there are enough of them
+    (numpy's generators run without the interpreter lock)."""
+    out = np.empty((len(seeds), n))
 
-    jobs = [(n, seed + 7919 * j) for n, b, seed in specs for j in range(b)]
-    if len(jobs) > 1 and sum(n for n, _ in jobs) >= 1 << 16:
-        with ThreadPoolExecutor(max_workers=min(len(jobs), 16, os.cpu_count() or 1)) as pool:
-            cols = list(pool.map(column, jobs))
+    def draw(j):
+        np.random.default_rng(seeds[j]).standard_normal(out=out[j])
+
+    if len(seeds) > 1 and n >= 1 << 15:
+        with ThreadPoolExecutor(max_workers=min(len(seeds), 8)) as pool:
+            list(pool.map(draw, range(len(seeds))))
     else:
-        cols = [column(job) for job in jobs]
-    out, at = [], 0
-    for _, b, _ in specs:
-        out.append(np.stack(cols[at: at + b], axis=1))
-        at += b
+        for j in range(len(seeds)):
+            draw(j)
     return out
 
 
@@ -206,15 +201,24 @@ class LanczosBatch:
         self.W.zero_()
         lib = _lib.lib()
         sp = _lib.stream_ptr(stream)
-        # seeded blocks are deterministic: drawn on the host once per
-        # (sector, width, seed) and kept on the device for later solves
+        # seeded blocks are deterministic: made once per (rows, width, seed) and
+        # kept on the device for later solves.  Column j of every block of a
+        # seed starts from the same stream of normals (real parts, then
+        # imaginary parts), so the host draws each stream once for all sectors
         cache = self.__dict__.setdefault("_start_cache", {})
         keys = [None if blocks is not None and blocks[i] is not None else
-                (s, self.sset.dims[s], self.block_sizes[i], 12345 if seeds is None else seeds[i])
+                (self.sset.dims[s], self.block_sizes[i], 12345 if seeds is None else seeds[i])
                 for i, s in enumerate(self.inst_sectors)]
         new = [k for k in dict.fromkeys(keys) if k is not None and k not in cache]
-        for key, blk in zip(new, start_blocks([k[1:] for k in new])):
-            cache[key] = torch.from_numpy(blk).to(self.dev)
+        for seed in dict.fromkeys(k[2] for k in new):
+            same = [k for k in new if k[2] == seed]
+            x = torch.from_numpy(_normal_streams(2 * max(d for d, _, _ in same),
+                                                 [seed + 7919 * j for j in range(max(b for _, b, _ in same))]))
+            x = x.to(self.dev)
+            for d, b, _ in same:
+                v = torch.complex(x[:b, :d], x[:b, d: 2 * d])
+                v /= torch.linalg.vector_norm(v, dim=1, keepdim=True)
+                cache[(d, b, seed)] = v.T.contiguous()
         for i, s in enumerate(self.inst_sectors):
             d = self.sset.dims[s]
             b = self.block_sizes[i]
