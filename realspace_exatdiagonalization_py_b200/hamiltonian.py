@@ -40,8 +40,11 @@ __all__ = [
 
 def _merge_terms(bilinear_terms, n_site, merge: bool = True):
     """Group directed terms by source site.  ``merge``: duplicate (i, j)
-    amplitudes add (one hop per site pair, what the solvers stream);
-    otherwise every term stays its own entry, in input order within a site
+    amplitudes add (one hop per site pair, what the solvers stream) and
+    terms of amplitude zero are left out (a coupling that is switched off
+    costs no hops: a quarter of them on the Haldane lattice with t'' = 0).
+    Only terms that are zero themselves go, not sums that cancel, so a model
+    keeps the same hops at every boundary twist.  Otherwise every term stays its own entry, in input order within a site
     pair (one triplet per term, as the reference's per-term builder emits)."""
     acc: dict[tuple[int, ...], complex] = {}
     order: list[tuple[int, ...]] = []
@@ -53,6 +56,8 @@ def _merge_terms(bilinear_terms, n_site, merge: bool = True):
             raise ValueError(
                 f"bilinear term ({i}, {i}) is on-site; put on-site energies in the density terms"
             )
+        if merge and complex(t) == 0:
+            continue
         key = (i - 1, j - 1) if merge else (i - 1, j - 1, n_in)
         if key not in acc:
             acc[key] = 0j
@@ -85,6 +90,7 @@ class DeviceModel:
         self.density_terms = [(int(i), int(j), complex(v)) for (i, j, v) in density_terms]
         begin, to, amp, jw = _merge_terms(self.bilinear_terms, n_site, merge_terms)
         self.n_terms = int(len(to))
+        self._term_key = (begin.tobytes(), to.tobytes())  # the hops of every state
         self.term_begin = torch.from_numpy(begin).to(dev)
         self.term_to = torch.from_numpy(to if len(to) else np.zeros(1, np.uint8)).to(dev)
         self.term_amp = torch.from_numpy(amp if len(amp) else np.zeros(1, np.complex128)).to(dev)
@@ -158,6 +164,8 @@ class DeviceModel:
         if self.proj is not None and self.proj["table_version"] == self.catalog.version and \
                 set(want) <= set(self.proj["precisions"]):
             return
+        if share is not None and share["terms"] != self._term_key:
+            share = None  # other hops: a table of its own
         if share is not None:
             rowptr, cg, n = share["rowptr"], share["cg"], share["n_hops"]
             dev = rowptr.device
@@ -166,7 +174,7 @@ class DeviceModel:
             _lib.check(lib.rsed_proj_fill(ctypes.byref(self.c), _lib.ptr(sqrt_stab), _lib.ptr(rowptr), None,
                                           _lib.ptr(w64), _lib.ptr(w32), _lib.stream_ptr(stream)))
             self.proj = {"rowptr": rowptr, "cg": cg, "w64": w64, "w32": w32, "n_hops": n, "precisions": want,
-                         "table_version": self.catalog.version, "shared": True}
+                         "terms": self._term_key, "table_version": self.catalog.version, "shared": True}
             self.refresh()
             return
         if self._hops is None:
@@ -179,7 +187,7 @@ class DeviceModel:
         _lib.check(lib.rsed_proj_fill(ctypes.byref(self.c), _lib.ptr(sqrt_stab), _lib.ptr(rowptr),
                                       _lib.ptr(cg), _lib.ptr(w64), _lib.ptr(w32), _lib.stream_ptr(stream)))
         self.proj = {"rowptr": rowptr, "cg": cg, "w64": w64, "w32": w32, "n_hops": n,
-                     "precisions": want, "table_version": self.catalog.version}
+                     "precisions": want, "terms": self._term_key, "table_version": self.catalog.version}
         self.refresh()
 
     def drop_projection(self) -> None:
