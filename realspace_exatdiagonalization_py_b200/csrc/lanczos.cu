@@ -70,6 +70,7 @@ struct LzDims {
   int chunk_rows;
   int n_chunks;
   int pslots;  // n_slots + 2 reduction slots per instance
+  bool uniform;  // every instance has bmax columns, 32-B segments of the rows
 };
 
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
@@ -617,6 +618,138 @@ __global__ void __launch_bounds__(256, 3) k_lz_update_rows(rsed_lanczos_t st, Lz
       }
     }
     __syncthreads();
+  }
+}
+
+// Two complex values of a row in one 32-B access.
+struct Pair {
+  double2 a, b;
+};
+__device__ __forceinline__ Pair load_pair(const double2* p) {
+  Pair v;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(v.a.x), "=d"(v.a.y), "=d"(v.b.x), "=d"(v.b.y)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void store_pair(double2* p, double2 a, double2 b) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a.x), "d"(a.y), "d"(b.x), "d"(b.y) : "memory");
+}
+
+// The block update for batches of one even block size BB: thread = one
+// instance's BB columns of RG rows, so a row segment is read once, in 32-B
+// words, US slots at a time (US * RG * BB / 2 words in flight per thread), the
+// coefficients of a slot serve RG rows, and x R = w is solved in registers:
+// nothing is exchanged between threads and no barrier stands in the row loop.
+// HBM bound.  657,756 rows of 32 columns, blocks of 2: k_lz_update_rows, which
+// reads every segment BB times and passes w through shared memory between
+// barriers, took 866 us a pass (0.64 of the measured copy rate), this form 557
+// us (four slots of two rows in flight: 608, six of one row: 595).
+template <int BB, int RG, int US>
+__global__ void __launch_bounds__(256, 2) k_lz_update_own(rsed_lanczos_t st, LzDims d, int pass) {
+  extern __shared__ __align__(16) unsigned char smem_u[];
+  constexpr int BP = BB / 2;
+  const int ni = d.n_inst;
+  double2* cs = reinterpret_cast<double2*>(smem_u);                  // [(s*BB + p)*BB + q][inst]
+  double2* Rs = cs + (size_t)st.n_slots * BB * BB * ni;              // [k*BB + p][inst]
+  bool any_work = false;
+  for (int i = 0; i < ni; ++i) {
+    const int* stt = st.state + i * kStateInts;
+    const bool one_i = stt[S_ONEPASS] != 0;
+    const int nb_i = (pass == 2 || one_i) ? stt[S_NEWSLOT] : stt[S_NB];
+    if (!stt[S_ACTIVE] || nb_i > st.n_slots || (pass == 2 && one_i)) continue;
+    any_work = true;
+    const double2* coef = reinterpret_cast<const double2*>(st.coef) +
+                          (int64_t)i * 2 * d.pslots * kBMax * kBMax + (pass - 1) * d.pslots * kBMax * kBMax;
+    for (int e = threadIdx.x; e < nb_i * BB * BB; e += blockDim.x) {
+      const int r = e / BB, q = e % BB;  // r = s * BB + p
+      cs[(size_t)e * ni + i] = coef[(r / BB) * kBMax * kBMax + (r % BB) * kBMax + q];
+    }
+    for (int e = threadIdx.x; e < BB * BB; e += blockDim.x)
+      Rs[e * ni + i] = coef[(d.pslots - 1) * kBMax * kBMax + (e / BB) * kBMax + e % BB];
+  }
+  __syncthreads();
+  if (!any_work) return;  // every thread read the same state words
+  const int rows_pg = blockDim.x / ni;
+  const int rloc = threadIdx.x / ni, inst = threadIdx.x % ni;
+  const int* stt = st.state + inst * kStateInts;
+  const bool one = stt[S_ONEPASS] != 0;
+  const int nb = (pass == 2 || one) ? stt[S_NEWSLOT] : stt[S_NB];
+  if (rloc >= rows_pg || !stt[S_ACTIVE] || nb > st.n_slots || (pass == 2 && one)) return;
+  const int c0 = st.inst_col0[inst];
+  const double2* ci = cs + inst;
+  const double2* Ri = Rs + inst;
+  double2* V = reinterpret_cast<double2*>(st.V) + c0;
+  double2* W = reinterpret_cast<double2*>(st.W) + c0;
+  const int64_t slot_stride = d.n_orb * d.ld;
+  const int64_t step = (int64_t)gridDim.x * rows_pg * RG;
+  for (int64_t row0 = (int64_t)blockIdx.x * rows_pg * RG + rloc; row0 < d.n_orb; row0 += step) {
+    double2 w[RG][BB];
+    int64_t at[RG];
+    bool live[RG];
+#pragma unroll
+    for (int h = 0; h < RG; ++h) {
+      const int64_t row = row0 + h * rows_pg;
+      live[h] = row < d.n_orb;
+      at[h] = (live[h] ? row : row0) * d.ld;  // past the end: the first row again, not stored
+#pragma unroll
+      for (int p = 0; p < BP; ++p) {
+        const Pair v = load_pair(W + at[h] + 2 * p);
+        w[h][2 * p] = v.a;
+        w[h][2 * p + 1] = v.b;
+      }
+    }
+    for (int s0 = 0; s0 < nb; s0 += US) {
+      Pair v[US][RG][BP];
+#pragma unroll
+      for (int u = 0; u < US; ++u)
+        if (s0 + u < nb) {
+#pragma unroll
+          for (int h = 0; h < RG; ++h)
+#pragma unroll
+            for (int p = 0; p < BP; ++p) v[u][h][p] = load_pair(V + (s0 + u) * slot_stride + at[h] + 2 * p);
+        }
+#pragma unroll
+      for (int u = 0; u < US; ++u)
+        if (s0 + u < nb) {
+          const double2* cu = ci + (size_t)(s0 + u) * BB * BB * ni;
+#pragma unroll
+          for (int p = 0; p < BB; ++p)
+#pragma unroll
+            for (int q = 0; q < BB; ++q) {
+              const double2 k = cu[(p * BB + q) * ni];
+#pragma unroll
+              for (int h = 0; h < RG; ++h)
+                w[h][q] = csub(w[h][q], cmul(p & 1 ? v[u][h][p / 2].b : v[u][h][p / 2].a, k));
+            }
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < RG; ++h) {
+      // forward substitution over the block's columns, in place
+#pragma unroll
+      for (int q = 0; q < BB; ++q) {
+#pragma unroll
+        for (int k = 0; k < q; ++k) w[h][q] = csub(w[h][q], cmul(w[h][k], Ri[(k * BB + q) * ni]));
+        const double rr = Ri[(q * BB + q) * ni].x;
+        w[h][q] = make_double2(w[h][q].x / rr, w[h][q].y / rr);
+      }
+      if (!live[h]) continue;
+#pragma unroll
+      for (int p = 0; p < BP; ++p) {
+        const double2 xa = w[h][2 * p], xb = w[h][2 * p + 1];
+        if (pass == 1 && !one) {
+          store_pair(W + at[h] + 2 * p, xa, xb);
+          continue;
+        }
+        store_pair(V + nb * slot_stride + at[h] + 2 * p, xa, xb);
+        if (st.Xf)
+          *reinterpret_cast<float4*>(reinterpret_cast<float2*>(st.Xf) + c0 + at[h] + 2 * p) =
+              make_float4((float)xa.x, (float)xa.y, (float)xb.x, (float)xb.y);
+        else  // the FP64 matvec reads the current-block slot
+          store_pair(V + (int64_t)(d.n_slots + 1) * slot_stride + at[h] + 2 * p, xa, xb);
+      }
+    }
   }
 }
 
@@ -1920,6 +2053,77 @@ __global__ void __launch_bounds__(256, 2) k_lz_restart_rows(rsed_lanczos_t st, L
   }
 }
 
+// The restart for batches of one even block size BB: thread = one instance's BB
+// columns of a row, K = keep * BB <= KM sums in registers.  A thread reads and
+// rewrites its own elements only, so no barrier separates the reads of a row
+// from its rewrite, and each 32-B segment is read once.  A block serves a group
+// of `ig` instances (blockIdx.y) whose coefficients fit its shared memory.
+// Bound by FP64 FMA and the coefficient reads from shared memory, then by HBM.
+// 657,756 rows of 32 columns, 13 blocks of 2 to 5: 2.55 ms in the whole-row form
+// above, 1.77 ms in this one (2 or 3 slots in flight: 1.90, 1.82 ms).
+template <int BB, int KM, int US>
+__global__ void __launch_bounds__(256, 2) k_lz_restart_own(rsed_lanczos_t st, LzDims d, int ig) {
+  extern __shared__ __align__(16) unsigned char smem_r[];
+  constexpr int BP = BB / 2;
+  const int keep = st.keep_blocks, K = keep * BB;
+  const int i0 = blockIdx.y * ig, ni = min(ig, d.n_inst - i0);
+  double2* St = reinterpret_cast<double2*>(smem_r);  // [l*K + j][inst of the group]
+  bool any_work = false;
+  for (int i = 0; i < ni; ++i) {
+    const int nb_old = st.state[(i0 + i) * kStateInts + S_RESTART_NB];
+    if (nb_old < 1 || nb_old > d.n_slots + 1) continue;
+    any_work = true;
+    const double2* S = reinterpret_cast<const double2*>(st.ritz_vec) + (int64_t)(i0 + i) * d.pm * d.pm;
+    for (int e = threadIdx.x; e < (nb_old - 1) * BB * K; e += blockDim.x)
+      St[(size_t)e * ni + i] = S[(int64_t)(e / K) * d.pm + e % K];
+  }
+  __syncthreads();
+  if (!any_work) return;  // every thread read the same state words
+  const int rows_pg = blockDim.x / ni;
+  const int rloc = threadIdx.x / ni, inst = i0 + threadIdx.x % ni;
+  const int nb_old = st.state[inst * kStateInts + S_RESTART_NB];
+  if (rloc >= rows_pg || nb_old < 1 || nb_old > d.n_slots + 1) return;
+  const int nslot = nb_old - 1;
+  const double2* Si = St + (inst - i0);
+  double2* V = reinterpret_cast<double2*>(st.V) + st.inst_col0[inst];
+  const int64_t slot_stride = d.n_orb * d.ld;
+  for (int64_t row = (int64_t)blockIdx.x * rows_pg + rloc; row < d.n_orb; row += (int64_t)gridDim.x * rows_pg) {
+    double2* at = V + row * d.ld;
+    double2 a[KM];
+#pragma unroll
+    for (int j = 0; j < KM; ++j) a[j] = make_double2(0.0, 0.0);
+    for (int l0 = 0; l0 < nslot; l0 += US) {
+      Pair v[US][BP];
+#pragma unroll
+      for (int u = 0; u < US; ++u)
+        if (l0 + u < nslot) {
+#pragma unroll
+          for (int p = 0; p < BP; ++p) v[u][p] = load_pair(at + (l0 + u) * slot_stride + 2 * p);
+        }
+#pragma unroll
+      for (int u = 0; u < US; ++u)
+        if (l0 + u < nslot) {
+#pragma unroll
+          for (int p = 0; p < BB; ++p) {
+            const double2* sp = Si + (size_t)((l0 + u) * BB + p) * K * ni;
+            const double2 vp = p & 1 ? v[u][p / 2].b : v[u][p / 2].a;
+#pragma unroll
+            for (int j = 0; j < KM; ++j)
+              if (j < K) a[j] = cadd(a[j], cmul(vp, sp[(size_t)j * ni]));
+          }
+        }
+    }
+    Pair r[BP];
+#pragma unroll
+    for (int p = 0; p < BP; ++p) r[p] = load_pair(at + nslot * slot_stride + 2 * p);
+#pragma unroll
+    for (int j = 0; j < KM; j += 2)
+      if (j < K) store_pair(at + (j / BB) * slot_stride + j % BB, a[j], a[j + 1]);
+#pragma unroll
+    for (int p = 0; p < BP; ++p) store_pair(at + keep * slot_stride + 2 * p, r[p].a, r[p].b);
+  }
+}
+
 // U[inst][j][row] = sum_l V_l[row] S[l][j], j < nev (Ritz vectors of the last check).
 __global__ void __launch_bounds__(256) k_lz_extract(rsed_lanczos_t st, LzDims d, double2* U, int64_t u_stride) {
   const int inst = blockIdx.x % d.n_inst;
@@ -2645,6 +2849,12 @@ LzDims make_dims(const rsed_model_t* md, const rsed_sectors_t* sc, const rsed_la
   d.chunk_rows = st->chunk_rows;
   d.n_chunks = (int)((d.n_orb + d.chunk_rows - 1) / d.chunk_rows);
   d.pslots = st->n_slots + 3;
+  // blocks of bmax columns that fill the columns in use lie at multiples of
+  // bmax; with an even ld and aligned buffers a segment of an even block is
+  // whole 32-B (V, W) and 16-B (Xf) words
+  auto aligned = [](const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; };
+  d.uniform = sc->n_cols == st->n_inst * st->bmax && (d.ld & 1) == 0 && aligned(st->V, 32) && aligned(st->W, 32) &&
+              (st->Xf == nullptr || aligned(st->Xf, 16));
   return d;
 }
 
@@ -2670,6 +2880,35 @@ int check_lz(const rsed_model_t* md, const rsed_sectors_t* sc, const rsed_lanczo
   return RSED_OK;
 }
 
+// (row, instance) pairs from which the register forms of update and restart are used
+constexpr int64_t kOwnPairs = 65536;
+
+// One wave of blocks of 256 threads over `units` block-sized pieces of work.
+int wave_grid(const void* kern, size_t smem, int64_t units, int64_t* grid) {
+  int dev = 0, n_sm = 148, per_sm = 1;
+  RSED_TRY_CUDA(cudaGetDevice(&dev));
+  RSED_TRY_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+  RSED_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem));
+  const int64_t wave = (int64_t)n_sm * (per_sm > 0 ? per_sm : 1);
+  *grid = units < wave ? units : wave;
+  return RSED_OK;
+}
+
+template <int BB, int KM, int US>
+int launch_restart_own(const rsed_lanczos_t& st, const LzDims& d, int ig, cudaStream_t stream) {
+  auto kern = k_lz_restart_own<BB, KM, US>;
+  const size_t smem = sizeof(double2) * (size_t)st.n_slots * BB * st.keep_blocks * BB * ig;
+  if (smem > 48 * 1024)
+    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int rows_pg = 256 / ig, groups = (d.n_inst + ig - 1) / ig;
+  int64_t grid = 0;
+  const int rc = wave_grid((const void*)kern, smem, (d.n_orb + rows_pg - 1) / rows_pg * groups, &grid);
+  if (rc) return rc;
+  kern<<<dim3((unsigned)((grid + groups - 1) / groups), (unsigned)groups), 256, smem, stream>>>(st, d, ig);
+  RSED_CHECK_LAUNCH();
+  return RSED_OK;
+}
+
 constexpr int kRestartRG = 2;  // row groups per thread iteration of k_lz_restart_rows (keep <= 8)
 
 template <int KM, int RG, int BB>
@@ -2689,6 +2928,23 @@ int launch_restart_rows(const rsed_lanczos_t& st, const LzDims& d, int64_t grid,
 // whole-row form when its coefficients fit shared memory (two blocks per SM
 // up to 115 KB, one up to 220 KB), else the per-instance form.
 int launch_restart(const rsed_lanczos_t& st, const LzDims& d, cudaStream_t stream) {
+  // one even block size for all instances: registers only, no barriers; groups
+  // of instances whose coefficients fit 100 KB (two blocks per SM).  Below 64k
+  // (row, instance) pairs the staging outweighs it (12 instances of 892 rows:
+  // 44 us in the forms below, 57 us in this one)
+  if (!(st.reserved & kFlagNoRowRestart) && d.uniform && (st.bmax == 2 || st.bmax == 4) &&
+      d.n_orb * d.n_inst >= kOwnPairs) {
+    const int K = st.keep_blocks * st.bmax;
+    const size_t per = sizeof(double2) * (size_t)st.n_slots * st.bmax * K;  // <= 16 KB
+    int ig = (int)(100 * 1024 / per);
+    if (ig > 64) ig = 64;
+    if (ig > d.n_inst) ig = d.n_inst;
+    const int groups = (d.n_inst + ig - 1) / ig;
+    ig = (d.n_inst + groups - 1) / groups;
+    if (st.bmax == 2)
+      return K <= 10 ? launch_restart_own<2, 10, 4>(st, d, ig, stream) : launch_restart_own<2, 16, 4>(st, d, ig, stream);
+    return K <= 12 ? launch_restart_own<4, 12, 2>(st, d, ig, stream) : launch_restart_own<4, 16, 2>(st, d, ig, stream);
+  }
   const size_t smem = sizeof(double2) * (size_t)st.n_slots * st.bmax * st.keep_blocks * d.ld +
                       sizeof(int) * (size_t)d.ld;
   if (!(st.reserved & kFlagNoRowRestart) && d.ld <= 256 && smem <= 220 * 1024 && st.keep_blocks <= 16) {
@@ -2740,7 +2996,30 @@ int launch_update_rows(const rsed_lanczos_t& st, const LzDims& d, int pass, size
   return RSED_OK;
 }
 
+template <int BB, int RG, int US>
+int launch_update_own(const rsed_lanczos_t& st, const LzDims& d, int pass, size_t smem, cudaStream_t stream) {
+  auto kern = k_lz_update_own<BB, RG, US>;
+  if (smem > 48 * 1024)
+    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int rows = 256 / d.n_inst * RG;
+  int64_t grid = 0;
+  const int rc = wave_grid((const void*)kern, smem, (d.n_orb + rows - 1) / rows, &grid);
+  if (rc) return rc;
+  kern<<<(unsigned)grid, 256, smem, stream>>>(st, d, pass);
+  RSED_CHECK_LAUNCH();
+  return RSED_OK;
+}
+
 int launch_update(const rsed_lanczos_t& st, const LzDims& d, int pass, cudaStream_t stream) {
+  // one even block size for all instances: registers only, no barriers
+  const size_t own = sizeof(double2) * (size_t)(st.n_slots + 1) * st.bmax * st.bmax * d.n_inst;
+  // (below 64k (row, instance) pairs the per-instance form has more blocks than
+  // this one has coefficient copies to stage: 5.6 against 10.5 us for 12
+  // instances of 892 rows)
+  if (d.uniform && (st.bmax == 2 || st.bmax == 4) && d.n_inst <= 256 && own <= 100 * 1024 &&
+      d.n_orb * d.n_inst >= kOwnPairs)
+    return st.bmax == 2 ? launch_update_own<2, 2, 3>(st, d, pass, own, stream)
+                        : launch_update_own<4, 2, 2>(st, d, pass, own, stream);
   // all instances per block when their coefficients fit in shared memory
   const int crows = st.n_slots * st.bmax;
   const size_t smem = sizeof(double2) * ((size_t)crows * d.ld + (size_t)d.n_inst * st.bmax * st.bmax +

@@ -172,3 +172,85 @@ def test_csr_products(n, most, k):
     np.testing.assert_allclose(dev.matmat(xd.conj()).cpu().numpy(), A @ x.conj(), atol=tol, rtol=0)
     np.testing.assert_allclose(dev.matvec(xd.T.contiguous()).T.cpu().numpy(), A @ x, atol=tol, rtol=0)
     np.testing.assert_allclose(dev.matvec(xd[:, 0].contiguous()).cpu().numpy(), A @ x[:, 0], atol=tol, rtol=0)
+
+
+# the recurrence's kernels (Gram reduction, update) by what they have to leave:
+# orthonormal blocks and the projected matrix V^H H V.  Uniform blocks of 2 and
+# 4 on one and many sectors (full and part-filled rows of columns), a mixed
+# batch, and a basis below the register forms' size
+@pytest.mark.parametrize("n_site,blocks,prec", [
+    (20, [2] * 8, 64), (20, [2] * 20, 32), (22, [4] * 3, 64), (22, [4] * 11, 32), (24, [4], 64), (24, [2], 64),
+    (22, [4, 2, 4], 64), (16, [4] * 5, 64), (24, [2] * 3, 32), (22, [1] * 4, 64),
+])
+def test_block_recurrence(n_site, blocks, prec):
+    import torch
+
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import models
+    from realspace_exatdiagonalization_py_b200.lanczos import LanczosBatch
+
+    m = models.build_heisenberg_second_quantized_model(n_site, 1.0)
+    data = ed.build_ed_data(m, filling_fraction=Fraction(n_site // 2, n_site),
+                            symmetry_group=ed.build_translation_group(m.lattice))
+    dm, sset = data._device()
+    dm.build_projection(sset.sqrt_stab, precisions=(64, 32))
+    secs = list(range(len(blocks)))
+    b = LanczosBatch(dm, sset, secs, 1, ed.LanczosParams(block=max(blocks), precision=prec), block_sizes=blocks)
+    b.load_start(None)
+    b.start()
+    n = 6
+    b.iterate_span(n, False)
+    V = b.V[: n + 1]
+    P = b.P.cpu()
+    HV = torch.empty_like(V)
+    for s in range(n + 1):
+        dm.apply_block(sset, b.col_sector, V[s], HV[s], 64)
+    for i, (c0, k) in enumerate(zip(b.col0, blocks)):
+        Q = torch.cat([V[s][:, c0: c0 + k] for s in range(n + 1)], 1)
+        Z = torch.cat([HV[s][:, c0: c0 + k] for s in range(n + 1)], 1)
+        G = (Q.conj().T @ Q).cpu()
+        # a few ulps per Gram-Schmidt step, sums of up to 112,720 products
+        assert (G - torch.eye(G.shape[0], dtype=G.dtype)).abs().max() < 2e-13
+        T = (Q.conj().T @ Z).cpu()[:, : n * k]
+        # the norm of H is below n_site; an FP32 product rounds at 6e-8 of it
+        tol = 1e-12 * n_site if prec == 64 else 1e-6 * n_site
+        assert (T - P[i, : (n + 1) * k, : n * k]).abs().max() < tol
+
+
+# the restart at sizes of the register form: groups of instances, part-filled
+# groups, instances that do not restart
+@pytest.mark.parametrize("n_site,n_inst,block", [(20, 8, 2), (20, 20, 4), (22, 3, 4), (20, 17, 2)])
+def test_restart_sizes(n_site, n_inst, block):
+    import torch
+
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import models
+    from realspace_exatdiagonalization_py_b200.lanczos import S_RESTART_NB, LanczosBatch
+
+    m = models.build_heisenberg_second_quantized_model(n_site, 1.0)
+    data = ed.build_ed_data(m, filling_fraction=Fraction(n_site // 2, n_site),
+                            symmetry_group=ed.build_translation_group(m.lattice))
+    dm, sset = data._device()
+    p = ed.LanczosParams(block=block, n_slots=12)
+    b = LanczosBatch(dm, sset, list(range(n_inst)), 2, p)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    b.V.copy_(torch.randn(b.V.shape, dtype=b.V.dtype, device="cuda", generator=g))
+    b.ritz_vec.copy_(torch.randn(b.ritz_vec.shape, dtype=b.V.dtype, device="cuda", generator=g))
+    nb_old = [13 - i % 3 for i in range(n_inst)]
+    nb_old[1] = 0
+    st = b.state.cpu()
+    st[:, S_RESTART_NB] = torch.tensor(nb_old, dtype=torch.int32)
+    b.state.copy_(st)
+    want = b.V.clone()
+    K = b.keep * block
+    for i in range(n_inst):
+        if nb_old[i]:
+            c = slice(i * block, (i + 1) * block)
+            old = torch.cat([b.V[s][:, c] for s in range(nb_old[i] - 1)], 1)
+            new = old @ b.ritz_vec[i, : old.shape[1], :K]
+            for s in range(b.keep):
+                want[s][:, c] = new[:, s * block: (s + 1) * block]
+            want[b.keep][:, c] = b.V[nb_old[i] - 1][:, c]
+    b.restart()
+    # sums of 48 products of size about 10 in another order
+    assert (b.V - want).abs().max() < 1e-11
