@@ -145,7 +145,7 @@ extern "C" int rsed_fock_expand(const rsed_group_t* grp, const rsed_entry_t* tab
   cudaStream_t stream = as_stream(stream_);
   const int64_t n_blocks = (grp->n_states + kFChunk - 1) / kFChunk;
   const FockLayout lay = fock_layout(grp->n_site, grp->n_group);
-  if (lay.total > 48 * 1024)
+  if (lay.total > 40 * 1024)  // beside the static tables
     RSED_TRY_CUDA(cudaFuncSetAttribute(k_fock_amps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.total));
   double* bn = reinterpret_cast<double*>(scratch);
   double* nrm = bn + n_blocks;

@@ -191,11 +191,11 @@ __device__ void lz_finalize(const rsed_lanczos_t& st, const LzDims& d, int inst,
   // G threads per entry sum interleaved chunk subsets, then the G partial
   // sums are added in order (deterministic for a given chunk count)
   const int nent = (nb + 1) * b * b;
-  const int G = max(1, kRT / nent);
+  const int G = max(1, (int)blockDim.x / nent);
   {
-    // fin: kRT * kBMax >= nent * G entries
+    // fin: kRT * kBMax >= max(nent, blockDim.x) entries
     const int64_t cstride = (int64_t)d.n_inst * d.pslots * kBMax * kBMax;
-    for (int t = threadIdx.x; t < nent * G; t += kRT) {
+    for (int t = threadIdx.x; t < nent * G; t += blockDim.x) {
       const int e = t % nent, g = t / nent;
       const int sl = e / (b * b), pq = e % (b * b), p = pq / b, q = pq % b;
       const double2* src = part + (int64_t)inst * d.pslots * kBMax * kBMax + sl * kBMax * kBMax + p * kBMax + q;
@@ -205,7 +205,7 @@ __device__ void lz_finalize(const rsed_lanczos_t& st, const LzDims& d, int inst,
       fin[g * nent + e] = a;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < nent; e += kRT) {
+    for (int e = threadIdx.x; e < nent; e += blockDim.x) {
       const int sl = e / (b * b), pq = e % (b * b), p = pq / b, q = pq % b;
       double2 a = make_double2(0.0, 0.0);
       for (int g = 0; g < G; ++g) a = cadd(a, fin[g * nent + e]);
@@ -779,7 +779,7 @@ constexpr int kSW = 8;                        // consumer warps
 constexpr int kSThreads = (kSW + 1) * 32;     // + the producer warp
 constexpr int kPanelElems = 512;              // entries of one panel at most (8 KB)
 constexpr int kStreamGridMax = 320;           // streaming blocks at most (Gram partials per instance)
-constexpr int kStreamInstMax = 64;            // instances of a streamed batch at most (ld <= 64)
+constexpr int kStreamInstMax = 64;            // instances of a streamed batch at most
 constexpr int kListMax = 2 * kJacobiMax + 8;  // panels of one chunk at most
 constexpr unsigned long long kWaitNs = 2000000000ull;
 constexpr int kFlagNoStream = 2;              // st.reserved bit 1: use the per-instance kernels
@@ -930,9 +930,8 @@ __device__ void stream_produce(const rsed_lanczos_t& st, const LzDims& d, int ns
 // shared memory (thread = entry of the panel); then every basis slot s < max
 // nb is streamed, and warp s % kSW adds it into its registers (lane = column
 // c0 + p, all q of the instance), reading W_loc from shared memory.  BB is
-// the largest block of the batch rounded up to a power of two, CPL the
-// columns per lane (ld <= 32 * CPL).
-template <int BB, int CPL>
+// the largest block of the batch rounded up to a power of two (ld <= 32).
+template <int BB>
 __global__ void __launch_bounds__(kSThreads, 2)
     k_lz_gram_stream(rsed_lanczos_t st, LzDims d, int pass, int ns, int pr, int crows) {
   constexpr int SW = kJacobiMax / BB / kSW + 1;  // slots one warp owns at most
@@ -945,8 +944,8 @@ __global__ void __launch_bounds__(kSThreads, 2)
   double2* lc = reinterpret_cast<double2*>(smem_s + L.coef);
   __shared__ int s_b[kStreamInstMax], s_c0[kStreamInstMax], s_nb[kStreamInstMax], s_jloc[kStreamInstMax];
   __shared__ unsigned long long s_lnz[kStreamInstMax];
-  __shared__ double s_sig[32 * CPL];  // sigma of each column
-  __shared__ int s_col_inst[32 * CPL];
+  __shared__ double s_sig[32];  // sigma of each column
+  __shared__ int s_col_inst[32];
   __shared__ int s_list[kListMax];
   __shared__ int s_npc, s_nloc, s_nbmax;
   __shared__ int s_abort_store;
@@ -954,7 +953,7 @@ __global__ void __launch_bounds__(kSThreads, 2)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ld = d.ld;
   if (tid == 0) s_abort_store = 0;
-  for (int c = tid; c < 32 * CPL; c += kSThreads) s_col_inst[c] = -1;
+  if (tid < 32) s_col_inst[tid] = -1;
   __syncthreads();
   for (int i = tid; i < d.n_inst; i += kSThreads) {
     const int* stt = st.state + i * kStateInts;
@@ -1029,24 +1028,16 @@ __global__ void __launch_bounds__(kSThreads, 2)
   if (warp == kSW) {
     if (lane == 0) stream_produce(st, d, ns, pr, s_list, npc, my_chunks, full, empty, ring, s_abort);
   } else {
-    double2 acc[SW][CPL][BB];
+    double2 acc[SW][BB];
 #pragma unroll
     for (int j = 0; j < SW; ++j)
 #pragma unroll
-      for (int c = 0; c < CPL; ++c)
-#pragma unroll
-        for (int q = 0; q < BB; ++q) acc[j][c][q] = make_double2(0.0, 0.0);
-    // this lane's columns (Gram) and this thread's two entries (W_loc)
-    int cinst[CPL], cnb[CPL], cb[CPL], cc0[CPL];
-#pragma unroll
-    for (int c = 0; c < CPL; ++c) {
-      const int col = lane + 32 * c;
-      const int i = col < ld ? s_col_inst[col] : -1;
-      cinst[c] = i;
-      cnb[c] = i >= 0 ? s_nb[i] : -1;
-      cb[c] = i >= 0 ? s_b[i] : 0;
-      cc0[c] = i >= 0 ? s_c0[i] : 0;
-    }
+      for (int q = 0; q < BB; ++q) acc[j][q] = make_double2(0.0, 0.0);
+    // this lane's column (Gram) and this thread's two entries (W_loc)
+    const int cinst = lane < ld ? s_col_inst[lane] : -1;
+    const int cnb = cinst >= 0 ? s_nb[cinst] : -1;
+    const int cb = cinst >= 0 ? s_b[cinst] : 0;
+    const int cc0 = cinst >= 0 ? s_c0[cinst] : 0;
     int einst[2], erow[2], ecol[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
@@ -1101,19 +1092,16 @@ __global__ void __launch_bounds__(kSThreads, 2)
         if (erow[u] < pr) wl[erow[u] * ld + ecol[u]] = w[u];
       consumer_sync();
       // Gram of W_loc itself: slot nb of the lane's instance
-#pragma unroll
-      for (int c = 0; c < CPL; ++c) {
-        if (cinst[c] < 0) continue;
-        const int col = lane + 32 * c;
+      if (cinst >= 0) {
 #pragma unroll
         for (int jj = 0; jj < SW; ++jj) {
-          if (cnb[c] != jj * kSW + warp) continue;
+          if (cnb != jj * kSW + warp) continue;
           for (int r = 0; r < rows; ++r) {
-            const double2 y = wl[r * ld + col];
-            const double2* wr = wl + r * ld + cc0[c];
+            const double2 y = wl[r * ld + lane];
+            const double2* wr = wl + r * ld + cc0;
 #pragma unroll
             for (int q = 0; q < BB; ++q)
-              if (q < cb[c]) acc[jj][c][q] = cadd(acc[jj][c][q], cdotc(y, wr[q]));
+              if (q < cb) acc[jj][q] = cadd(acc[jj][q], cdotc(y, wr[q]));
           }
         }
       }
@@ -1124,20 +1112,15 @@ __global__ void __launch_bounds__(kSThreads, 2)
           const int s = jj * kSW + ww;
           if (s >= nbmax) break;
           mbar_wait(&full[stg], ph, s_abort);
-          if (ww == warp) {
+          if (ww == warp && s < cnb) {
             const double2* pnl = ring + (size_t)stg * kPanelElems;
-#pragma unroll
-            for (int c = 0; c < CPL; ++c) {
-              if (s >= cnb[c]) continue;
-              const int col = lane + 32 * c;
 #pragma unroll 4
-              for (int r = 0; r < rows; ++r) {
-                const double2 y = pnl[r * ld + col];
-                const double2* wr = wl + r * ld + cc0[c];
+            for (int r = 0; r < rows; ++r) {
+              const double2 y = pnl[r * ld + lane];
+              const double2* wr = wl + r * ld + cc0;
 #pragma unroll
-                for (int q = 0; q < BB; ++q)
-                  if (q < cb[c]) acc[jj][c][q] = cadd(acc[jj][c][q], cdotc(y, wr[q]));
-              }
+              for (int q = 0; q < BB; ++q)
+                if (q < cb) acc[jj][q] = cadd(acc[jj][q], cdotc(y, wr[q]));
             }
           }
           __syncwarp();
@@ -1146,22 +1129,17 @@ __global__ void __launch_bounds__(kSThreads, 2)
         }
       }
     }
-    if (!*s_abort) {
+    if (!*s_abort && cinst >= 0) {
       double2* part = reinterpret_cast<double2*>(st.partial);
+      const int p = lane - cc0;
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) {
-        const int i = cinst[c];
-        if (i < 0) continue;
-        const int p = lane + 32 * c - cc0[c];
+      for (int jj = 0; jj < SW; ++jj) {
+        const int s = jj * kSW + warp;
+        if (s > cnb) continue;
+        double2* out = part + (((int64_t)blockIdx.x * d.n_inst + cinst) * d.pslots + s) * kBMax * kBMax + p * kBMax;
 #pragma unroll
-        for (int jj = 0; jj < SW; ++jj) {
-          const int s = jj * kSW + warp;
-          if (s > cnb[c]) continue;
-          double2* out = part + (((int64_t)blockIdx.x * d.n_inst + i) * d.pslots + s) * kBMax * kBMax + p * kBMax;
-#pragma unroll
-          for (int q = 0; q < BB; ++q)
-            if (q < cb[c]) out[q] = acc[jj][c][q];
-        }
+        for (int q = 0; q < BB; ++q)
+          if (q < cb) out[q] = acc[jj][q];
       }
     }
   }
@@ -1176,9 +1154,198 @@ __global__ void __launch_bounds__(kSThreads, 2)
   }
 }
 
+// ---------------------------------------------------------------------------
+// Gram reduction of batches of one even block size BB straight from global
+// memory.  blockIdx.y = group of `ig` instances with at most 32 columns; a block
+// takes tiles of kTileElems entries (all columns of the group) of W: it forms
+// W_loc of the tile in shared memory (thread = column, FE rows in flight), then
+// its 8 warps walk the work of the tile as one list of units (slot, row step),
+// slot-major, each warp a fixed contiguous share of it -- so the warps are
+// equally loaded for any number of slots, touch at most NS slots each, and keep
+// those slots' sums in registers over all tiles of the block (lane = row of the
+// step and column, UN steps in flight).  Row segments are read once, contiguous,
+// with no staging, ring or barrier per slot.
+// HBM bound.  657,756 rows: 32 columns in blocks of 2, 850 us a pass of the
+// 12-slot solve with the bulk-copy ring (every warp waits on every panel), 692
+// in this form; over the first 11 steps, 32 columns in blocks of 4, 1048 us with
+// the ring and 894 here; 64 columns, 2656 us with one instance per block and
+// 1747 here, in two groups.
+constexpr int kTileElems = 2048;
+constexpr int kTileCols = 32;    // columns of a group at most
+constexpr int kTileGridMax = kStreamGridMax;  // blocks per group at most (Gram partials per instance)
+
+template <int BB, int NS>
+__global__ void __launch_bounds__(256, 2) k_lz_gram_tiles(rsed_lanczos_t st, LzDims d, int pass, int ig) {
+  constexpr int UN = BB == 2 ? 8 : 4, FE = BB == 2 ? 4 : 2, GI = kTileCols / BB;
+  extern __shared__ __align__(16) unsigned char smem_g[];
+  const int i0 = blockIdx.y * ig, gn = min(ig, d.n_inst - i0), gw = gn * BB;  // the group's instances, columns
+  double2* wl = reinterpret_cast<double2*>(smem_g);     // [rows][gw]: W_loc of the tile
+  double2* lc = wl + kTileElems;                        // [l*BB + p][gw]
+  __shared__ int s_nb[GI], s_jloc[GI], s_c0[GI];
+  __shared__ unsigned long long s_lnz[GI];
+  __shared__ double s_sig[kTileCols];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid < gn) {
+    const int* stt = st.state + (i0 + tid) * kStateInts;
+    const int nb = stt[S_NB];
+    const bool act = stt[S_ACTIVE] && !(pass == 2 && stt[S_ONEPASS]) && nb <= d.n_slots;
+    s_nb[tid] = act ? nb : -1;
+    s_jloc[tid] = (act && pass == 1 && nb >= 2 && (st.reserved & kFlagSinglePass)) ? nb - 1 : 0;
+    s_c0[tid] = st.inst_col0[i0 + tid];
+  }
+  __syncthreads();
+  int nbmax = -1;
+  for (int i = 0; i < gn; ++i) nbmax = max(nbmax, s_nb[i]);
+  if (nbmax < 0) return;  // no instance of the group has work in this pass
+  // the known part of the recurrence, as in k_lz_gram_stream; warps take
+  // instances
+  for (int i = warp; i < gn; i += 8) {
+    const int jl = s_jloc[i];
+    unsigned long long m = 0;
+    const double2* Pi = reinterpret_cast<const double2*>(st.P) + (int64_t)(i0 + i) * d.pm * d.pm;
+    for (int e = lane; e < jl * BB * BB; e += 32) {
+      const double2 v = Pi[(int64_t)(jl * BB + e % BB) * d.pm + e / BB];
+      lc[(size_t)(e / BB) * gw + i * BB + e % BB] = cconj(v);
+      if (v.x != 0.0 || v.y != 0.0) m |= 1ull << (e / (BB * BB));
+    }
+    for (int o = 16; o > 0; o >>= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
+    if (lane == 0) s_lnz[i] = m;
+    if (jl > 0 && lane < BB) s_sig[i * BB + lane] = Pi[(int64_t)((jl - 1) * BB + lane) * d.pm + (jl - 1) * BB + lane].x;
+  }
+  __syncthreads();
+  const double2* V = reinterpret_cast<const double2*>(st.V);
+  const double2* W = reinterpret_cast<const double2*>(st.W);
+  const int64_t ld = d.ld, slot_stride = d.n_orb * ld;
+  // rows of a warp step, steps of a tile, this warp's units; the last slot
+  // stands for W_loc itself
+  const int rpw = 32 / gw, tile_rows = kTileElems / gw / rpw * rpw, steps = tile_rows / rpw;
+  const int units = (nbmax + 1) * steps;
+  const int u0 = units * warp / 8, u1 = units * (warp + 1) / 8, seg0 = u0 / steps;
+  // this lane's row of a step, local column, instance (number of blocks, W_loc
+  // columns) and column
+  const int lr = lane / gw, lcol = lane % gw;
+  const int lnb = lr < rpw ? s_nb[lcol / BB] : -1, lc0 = lcol / BB * BB;
+  const int64_t gcol = s_c0[lcol / BB] + lcol % BB;
+  // this thread's column and first row of W_loc
+  const int frows = 256 / gw, fcol = tid % gw, fi = fcol / BB;
+  const int frow = tid < frows * gw ? tid / gw : tile_rows;
+  const bool fact = s_nb[fi] >= 0;
+  const int fjl = s_jloc[fi];
+  const double fsig = fjl > 0 ? s_sig[fcol] : 0.0;
+  const int64_t fc0 = s_c0[fi], fgcol = fc0 + fcol % BB;
+  double2 acc[NS][BB];
+#pragma unroll
+  for (int k = 0; k < NS; ++k)
+#pragma unroll
+    for (int q = 0; q < BB; ++q) acc[k][q] = make_double2(0.0, 0.0);
+  for (int64_t r0 = (int64_t)blockIdx.x * tile_rows; r0 < d.n_orb; r0 += (int64_t)gridDim.x * tile_rows) {
+    const int rows = (int)min((int64_t)tile_rows, d.n_orb - r0);
+    __syncthreads();  // the previous tile is done with
+    for (int f0 = frow; f0 < tile_rows; f0 += FE * frows) {
+      double2 w[FE];
+#pragma unroll
+      for (int h = 0; h < FE; ++h) {
+        const int r = f0 + h * frows;
+        w[h] = r < rows && fact ? W[(r0 + r) * ld + fgcol] : make_double2(0.0, 0.0);
+      }
+      if (fjl > 0) {
+        const double2* Vj = V + (int64_t)fjl * slot_stride + r0 * ld + fgcol;
+        double2 x[FE];
+#pragma unroll
+        for (int h = 0; h < FE; ++h) {
+          const int r = f0 + h * frows;
+          x[h] = r < rows ? Vj[r * ld] : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int h = 0; h < FE; ++h) {
+          w[h].x -= fsig * x[h].x;
+          w[h].y -= fsig * x[h].y;
+        }
+        for (unsigned long long m = s_lnz[fi]; m; m &= m - 1) {
+          const int l = __ffsll((long long)m) - 1;
+          const double2* Vl = V + (int64_t)l * slot_stride + r0 * ld + fc0;
+          const double2* Lc = lc + (size_t)l * BB * gw + fcol;
+          double2 v[FE][BB];
+#pragma unroll
+          for (int h = 0; h < FE; ++h)
+#pragma unroll
+            for (int p = 0; p < BB; ++p) {
+              const int r = f0 + h * frows;
+              v[h][p] = r < rows ? Vl[r * ld + p] : make_double2(0.0, 0.0);
+            }
+#pragma unroll
+          for (int p = 0; p < BB; ++p) {
+            const double2 k = Lc[p * gw];
+#pragma unroll
+            for (int h = 0; h < FE; ++h) w[h] = csub(w[h], cmul(v[h][p], k));
+          }
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < FE; ++h)
+        if (f0 + h * frows < tile_rows) wl[(f0 + h * frows) * gw + fcol] = w[h];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+      const int s = seg0 + k;
+      const int t0 = max(u0 - s * steps, 0), t1 = min(u1 - s * steps, steps);
+      // an instance's own last slot is W_loc (the instances of a batch may hold
+      // different numbers of blocks)
+      if (t0 >= t1 || s > lnb) continue;
+      const bool own = s == lnb;
+      const double2* Y = V + (int64_t)(own ? 0 : s) * slot_stride + r0 * ld + gcol;
+      for (int t = t0; t < t1; t += UN) {
+        double2 y[UN];
+#pragma unroll
+        for (int u = 0; u < UN; ++u) {
+          const int r = (t + u) * rpw + lr;
+          y[u] = make_double2(0.0, 0.0);
+          if (t + u < t1 && r < rows) y[u] = own ? wl[r * gw + lcol] : Y[r * ld];
+        }
+#pragma unroll
+        for (int u = 0; u < UN; ++u) {
+          const int r = min((t + u) * rpw + lr, tile_rows - 1);
+          const double2* wr = wl + r * gw + lc0;
+#pragma unroll
+          for (int q = 0; q < BB; ++q) acc[k][q] = cadd(acc[k][q], cdotc(y[u], wr[q]));
+        }
+      }
+    }
+  }
+  // the row lanes of a column, then the warps of a slot in order
+  for (int w = 0; w < 8; ++w) {
+    __syncthreads();
+    if (w != warp) continue;
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+      const int s = seg0 + k;
+      const int t0 = max(u0 - s * steps, 0), t1 = min(u1 - s * steps, steps);
+      if (t0 >= t1) continue;  // the same for all lanes
+      double2 sum[BB];
+#pragma unroll
+      for (int q = 0; q < BB; ++q) {
+        sum[q] = acc[k][q];
+        for (int h = 1; h < rpw; ++h) {
+          const double vx = __shfl_sync(0xffffffffu, acc[k][q].x, (lane + h * gw) & 31);
+          const double vy = __shfl_sync(0xffffffffu, acc[k][q].y, (lane + h * gw) & 31);
+          sum[q] = cadd(sum[q], make_double2(vx, vy));
+        }
+      }
+      if (lr > 0 || s > lnb) continue;
+      double2* out = reinterpret_cast<double2*>(st.partial) +
+                     (((int64_t)blockIdx.x * d.n_inst + i0 + lcol / BB) * d.pslots + s) * kBMax * kBMax +
+                     lcol % BB * kBMax;
+#pragma unroll
+      for (int q = 0; q < BB; ++q) out[q] = t0 == 0 ? sum[q] : cadd(out[q], sum[q]);
+    }
+  }
+}
+
 // Finalisation of the streamed Gram partials, one block per instance (the
 // same arithmetic as the last block of k_lz_reduce).
-__global__ void __launch_bounds__(kRT) k_lz_finalize(rsed_lanczos_t st, LzDims d, int pass) {
+constexpr int kFT = 1024;  // threads of k_lz_finalize
+__global__ void __launch_bounds__(kFT) k_lz_finalize(rsed_lanczos_t st, LzDims d, int pass) {
   const int inst = blockIdx.x;
   int* stt = st.state + inst * kStateInts;
   if (pass == 1 && threadIdx.x == 0) stt[S_RESTART_NB] = 0;
@@ -3055,7 +3222,9 @@ bool stream_config(const rsed_lanczos_t& st, const LzDims& d, StreamConfig* c) {
   // (one sector of block 1 or 2: the per-instance kernel is faster)
   // and below ~32k rows the ring's fill latency outweighs the streaming (a
   // 892-row batch: 12.8 vs 8 ms per step), so small bases keep it too
-  if (d.ld < 16 || d.ld > 64 || d.n_inst > kStreamInstMax || d.n_orb < 32768) return false;
+  // above 32 columns a lane would hold two columns' sums: 778 us on 84,576 rows
+  // of 56 columns against 353 us with one instance per block
+  if (d.ld < 16 || d.ld > 32 || d.n_inst > kStreamInstMax || d.n_orb < 32768) return false;
   const int crows = st.n_slots * st.bmax;
   constexpr size_t kBudget = 104 * 1024;  // dynamic shared memory per block (two blocks per SM)
   c->pr = kPanelElems / d.ld;
@@ -3079,16 +3248,16 @@ bool stream_config(const rsed_lanczos_t& st, const LzDims& d, StreamConfig* c) {
   return true;
 }
 
-template <int BB, int CPL>
+template <int BB>
 int launch_gram_stream(const rsed_lanczos_t& st, const LzDims& d, int pass, const StreamConfig& c,
                        cudaStream_t stream) {
   static bool attr_set = false;
   if (!attr_set) {
-    RSED_TRY_CUDA(cudaFuncSetAttribute(k_lz_gram_stream<BB, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    RSED_TRY_CUDA(cudaFuncSetAttribute(k_lz_gram_stream<BB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        110 * 1024));
     attr_set = true;
   }
-  k_lz_gram_stream<BB, CPL><<<(unsigned)c.grid, kSThreads, c.smem_gram, stream>>>(
+  k_lz_gram_stream<BB><<<(unsigned)c.grid, kSThreads, c.smem_gram, stream>>>(
       st, d, pass, c.ns_gram, c.pr, st.n_slots * st.bmax);
   RSED_CHECK_LAUNCH();
   return RSED_OK;
@@ -3100,19 +3269,12 @@ int launch_pass_stream(const rsed_lanczos_t& st, const LzDims& d, int pass, cons
   ds.n_chunks = c.grid;  // one Gram partial per streaming block
   const int bb = st.bmax <= 1 ? 1 : st.bmax <= 2 ? 2 : st.bmax <= 4 ? 4 : 8;
   int rc;
-  if (d.ld <= 32) {
-    rc = bb == 1   ? launch_gram_stream<1, 1>(st, ds, pass, c, stream)
-         : bb == 2 ? launch_gram_stream<2, 1>(st, ds, pass, c, stream)
-         : bb == 4 ? launch_gram_stream<4, 1>(st, ds, pass, c, stream)
-                   : launch_gram_stream<8, 1>(st, ds, pass, c, stream);
-  } else {
-    rc = bb == 1   ? launch_gram_stream<1, 2>(st, ds, pass, c, stream)
-         : bb == 2 ? launch_gram_stream<2, 2>(st, ds, pass, c, stream)
-         : bb == 4 ? launch_gram_stream<4, 2>(st, ds, pass, c, stream)
-                   : launch_gram_stream<8, 2>(st, ds, pass, c, stream);
-  }
+  rc = bb == 1   ? launch_gram_stream<1>(st, ds, pass, c, stream)
+       : bb == 2 ? launch_gram_stream<2>(st, ds, pass, c, stream)
+       : bb == 4 ? launch_gram_stream<4>(st, ds, pass, c, stream)
+                 : launch_gram_stream<8>(st, ds, pass, c, stream);
   if (rc != RSED_OK) return rc;
-  k_lz_finalize<<<(unsigned)d.n_inst, kRT, 0, stream>>>(st, ds, pass);
+  k_lz_finalize<<<(unsigned)d.n_inst, kFT, 0, stream>>>(st, ds, pass);
   RSED_CHECK_LAUNCH();
   if (st.reserved & kFlagNoStreamUpdate) return launch_update(st, d, pass, stream);
   static bool attr_set = false;
@@ -3126,7 +3288,60 @@ int launch_pass_stream(const rsed_lanczos_t& st, const LzDims& d, int pass, cons
   return RSED_OK;
 }
 
+// Instances of one group of the tiled reduction: at most 32 columns, the groups
+// as equal as can be.
+int tile_group(const rsed_lanczos_t& st, const LzDims& d) {
+  const int most = kTileCols / st.bmax, groups = (d.n_inst + most - 1) / most;
+  return (d.n_inst + groups - 1) / groups;
+}
+
+template <int BB, int NS>
+int launch_gram_tiles(const rsed_lanczos_t& st, const LzDims& d, int pass, cudaStream_t stream) {
+  auto kern = k_lz_gram_tiles<BB, NS>;
+  const int ig = tile_group(st, d), gw = ig * BB, groups = (d.n_inst + ig - 1) / ig;
+  const size_t smem = sizeof(double2) * (kTileElems + (size_t)st.n_slots * BB * gw);
+  if (smem > 40 * 1024)  // beside the static tables
+    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int rpw = 32 / gw, rows = kTileElems / gw / rpw * rpw;
+  const int64_t tiles = (d.n_orb + rows - 1) / rows;
+  int64_t grid = 0;
+  int rc = wave_grid((const void*)kern, smem, tiles * groups, &grid);
+  if (rc) return rc;
+  grid = (grid + groups - 1) / groups;
+  if (grid > kTileGridMax) grid = kTileGridMax;
+  if (grid > tiles) grid = tiles;
+  kern<<<dim3((unsigned)grid, (unsigned)groups), 256, smem, stream>>>(st, d, pass, ig);
+  RSED_CHECK_LAUNCH();
+  LzDims ds = d;
+  ds.n_chunks = (int)grid;  // one Gram partial per block and group
+  k_lz_finalize<<<(unsigned)d.n_inst, kFT, 0, stream>>>(st, ds, pass);
+  RSED_CHECK_LAUNCH();
+  return launch_update(st, d, pass, stream);
+}
+
+// Slots that one of eight warps touches at most, over the numbers of blocks a
+// basis of n_slots can hold.
+int tile_segments(int n_slots) {
+  int most = 0;
+  for (int segs = 1; segs <= n_slots + 1; ++segs)
+    for (int w = 0; w < 8; ++w) {
+      const int n = (segs * (w + 1) + 7) / 8 - segs * w / 8;
+      if (n > most) most = n;
+    }
+  return most;
+}
+
 int launch_pass(const rsed_lanczos_t& st, const LzDims& d, int pass, cudaStream_t stream) {
+  // the tiled reduction from 64k (row, instance) pairs; one or a few narrow
+  // sectors only from 2^18 rows (one sector of 112,720 rows, blocks of 2: 24 us
+  // with the per-instance reduction, 40 us tiled; of 657,756 rows: 90 and 80)
+  if (!(st.reserved & kFlagNoStream) && (st.reserved & kFlagNoStreamUpdate) && d.uniform &&
+      (st.bmax == 2 || st.bmax == 4) && d.n_orb * d.n_inst >= kOwnPairs && (d.ld >= 6 || d.n_orb >= (1 << 18))) {
+    const int segs = tile_segments(st.n_slots);
+    if (st.bmax == 2 && segs <= 3) return launch_gram_tiles<2, 3>(st, d, pass, stream);
+    if (st.bmax == 2 && segs <= 5) return launch_gram_tiles<2, 5>(st, d, pass, stream);
+    if (st.bmax == 4 && segs <= 3) return launch_gram_tiles<4, 3>(st, d, pass, stream);
+  }
   StreamConfig sc;
   if (stream_config(st, d, &sc)) return launch_pass_stream(st, d, pass, sc, stream);
   k_lz_reduce<<<(unsigned)(d.n_chunks * d.n_inst), kRT, 0, stream>>>(st, d, pass);
@@ -3186,7 +3401,7 @@ __global__ void k_scatter_block(int64_t n_rows, const int32_t* orbit_of_row, con
 extern "C" int64_t rsed_lanczos_partial_len(int64_t n_orbits, int32_t chunk_rows, int32_t n_inst,
                                             int32_t n_slots) {
   int64_t n_chunks = (n_orbits + chunk_rows - 1) / chunk_rows;
-  if (n_chunks < kStreamGridMax) n_chunks = kStreamGridMax;  // the streaming reduction's partials
+  if (n_chunks < kStreamGridMax) n_chunks = kStreamGridMax;  // the partials of the streamed and tiled reductions
   const int64_t lz = (int64_t)(n_slots + 3) * kBMax * kBMax * 2;
   const int64_t rr = (int64_t)kRRMax * kRRMax * 2;
   return n_chunks * n_inst * (lz > rr ? lz : rr);

@@ -59,7 +59,7 @@ class LanczosParams:
     precision: int = 64
     apply_variant: int = 0
     single_pass: bool = True  # skip the second Gram-Schmidt pass when pass 1 lost little norm
-    stream: bool = True  # Gram-Schmidt kernels stream whole-row panels by bulk copies (batches with ld <= 64)
+    stream: bool = True  # tiled or streamed Gram reduction over whole rows; False: one instance per block
     # the update streams too; off by default: on the 32-site workload the
     # row-group update takes 615 us per launch, the streamed one 727 us
     stream_update: bool = False
