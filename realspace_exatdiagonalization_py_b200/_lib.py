@@ -181,6 +181,7 @@ SIGNATURES = {
                                        c_void_p, c_int32, c_void_p, c_int32, c_void_p, c_void_p, c_size_t,
                                        c_void_p]),
     "rsed_obdm_scratch_bytes": (c_size_t, [c_int32]),
+    "rsed_obdm_states_bytes": (c_size_t, [c_int64]),
     "rsed_one_body_density": (c_int, [POINTER(RsedGroup), c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
                                       c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "rsed_density_pairs_scratch_bytes": (c_size_t, [c_int32]),

@@ -91,7 +91,12 @@ def one_body_density_matrix(basis, c, *, stream=None) -> np.ndarray:
     x = _orbit_vector(basis, c)
     sset = basis.sector_set
     rho = torch.empty((n, n), dtype=torch.complex128, device=x.device)
-    scratch = torch.empty(int(lib.rsed_obdm_scratch_bytes(n)), dtype=torch.uint8, device=x.device)
+    nbytes = int(lib.rsed_obdm_scratch_bytes(n))
+    try:  # room for the states' amplitudes, written once
+        scratch = torch.empty(nbytes + int(lib.rsed_obdm_states_bytes(cat.n_states)), dtype=torch.uint8,
+                              device=x.device)
+    except torch.cuda.OutOfMemoryError:
+        scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
     _lib.check(lib.rsed_one_body_density(ctypes.byref(cat.dgroup.c), _lib.ptr(cat.table), cat.n_orbits,
                                          _lib.ptr(cat.repr_masks), _lib.ptr(cat.stab_mask), _lib.ptr(sset.member),
                                          int(basis.sector_index), _lib.ptr(sset.chi[basis.sector_index].contiguous()),

@@ -43,8 +43,16 @@ int one_wave(const void* fn, size_t smem) {
 // the 256 threads add the tile's outer products, each owning RT x RT entries.
 // Two-species bases run the particle taken from species A and from species B
 // as two sets of states n; hops between the species stay zero.
+//
+// With scratch for it (32 B a state) K and B of every state are written once
+// (k_obdm_states) and a lookup is one 32-B read (DENSE); otherwise each lookup
+// evaluates its state from the table, the representative's mask, coefficient,
+// stabilizer and membership.  The diagonal comes from the orbits alone
+// (k_obdm_diag).
 // 32 sites, 8 bosons, 10.5 million states: 120.6 ms with one rank, table and
-// coefficient chain per hop and thread, 7.0 ms in this form.
+// coefficient chain per hop and thread; 6.5 ms evaluating each lookup (a state
+// k times; 24 % occupancy, latency of the dependent loads); @MS@ with the
+// states written first.
 template <int NP>
 struct ObdmTile {
   static constexpr int TN = NP == 32 ? 32 : 16;       // states n of one tile
@@ -54,7 +62,7 @@ struct ObdmTile {
 };
 
 struct ObdmLayout {
-  size_t binom, eta, chi, perm, tile, diag, total;
+  size_t binom, eta, chi, perm, tile, total;
 };
 
 ObdmLayout obdm_layout(int n_site, int n_filled, int n_group) {
@@ -68,8 +76,6 @@ ObdmLayout obdm_layout(int n_site, int n_filled, int n_group) {
   off += sizeof(double2) * (size_t)n_group;
   l.binom = off;
   off += sizeof(int64_t) * (size_t)(n_site + 1) * (n_filled + 1);
-  l.diag = off;
-  off += sizeof(double) * (kCT / 32) * 64;
   l.perm = off;
   off += align_up((size_t)n_group * n_site, 16);
   l.total = off;
@@ -90,14 +96,137 @@ __device__ __forceinline__ int64_t rank_with(uint64_t n, int i, const int64_t* _
   return r;
 }
 
-template <int NP>
-__global__ void __launch_bounds__(kCT, 2) k_obdm_part(rsed_group_t grp, const int4* __restrict__ table,
+struct KetBra {
+  double2 ket, bra;
+};
+
+// Ket amplitude and bra coefficient of the state m with table entry e.
+__device__ __forceinline__ KetBra ket_bra(const int4 e, uint64_t s, uint64_t m, double2 c, double2 ph, uint64_t stab,
+                                          bool member, const rsed_group_t& grp, const uint8_t* perm,
+                                          const double2* eta, const double2* chi) {
+  KetBra o;
+  o.ket = o.bra = make_double2(0.0, 0.0);
+  if (c.x == 0.0 && c.y == 0.0) return o;
+  const double S = (double)__popcll(stab);
+  const double norm = 1.0 / sqrt((double)grp.n_group * S);
+  o.ket = rsed_state_amplitude(s, m, e.y, ph, stab, grp, perm, eta, chi, make_double2(c.x * norm, c.y * norm));
+  if (member) {
+    const double2 ch = chi[e.y];
+    const double2 pc = cmul(make_double2((double)__int_as_float(e.z), (double)__int_as_float(e.w)),
+                            make_double2(ch.x, -ch.y));
+    const double sr = S * norm;  // sqrt(S / |G|)
+    o.bra = cmul(c, make_double2(sr * pc.x, -sr * pc.y));
+  }
+  return o;
+}
+
+__device__ __forceinline__ bool stage_phases(const rsed_group_t& grp, const double2* chi_g, double2* eta, uint8_t* perm,
+                                             double2* chi) {
+  bool twisted = false;
+  for (int i = threadIdx.x; i < grp.n_group * grp.n_site; i += kCT) {
+    const double2 v = reinterpret_cast<const double2*>(grp.eta)[i];
+    twisted |= v.x != 1.0 || v.y != 0.0;
+    eta[i] = v;
+    perm[i] = grp.perm[i];
+  }
+  for (int i = threadIdx.x; i < grp.n_group; i += kCT) chi[i] = chi_g[i];
+  return __syncthreads_or(twisted) == 0;  // all site phases exactly 1
+}
+
+// K and B of every state, in rank order.
+__global__ void __launch_bounds__(kCT) k_obdm_states(rsed_group_t grp, const int4* __restrict__ table,
+                                                     const uint64_t* __restrict__ repr_masks,
+                                                     const uint64_t* __restrict__ stab_mask,
+                                                     const uint64_t* __restrict__ member, int sector,
+                                                     const double2* __restrict__ chi_g, const double2* __restrict__ x,
+                                                     ObdmLayout lay, KetBra* __restrict__ out) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  double2* eta = reinterpret_cast<double2*>(smem + lay.eta);
+  double2* chi = reinterpret_cast<double2*>(smem + lay.chi);
+  uint8_t* perm = smem + lay.perm;
+  const bool unit = stage_phases(grp, chi_g, eta, perm, chi);
+  const int N = grp.n_site;
+  for (int64_t r = (int64_t)blockIdx.x * kCT + threadIdx.x; r < grp.n_states; r += (int64_t)gridDim.x * kCT) {
+    const int4 e = __ldg(table + r);
+    KetBra o;
+    o.ket = o.bra = make_double2(0.0, 0.0);
+    if (e.x >= 0) {
+      const double2 c = __ldg(x + e.x);
+      const uint64_t s[1] = {__ldg(repr_masks + e.x)};
+      const uint64_t stab = __ldg(stab_mask + e.x);
+      const bool mem = (__ldg(member + e.x) >> sector) & 1ull;
+      const int g[1] = {e.y};
+      double2 ph[1];
+      rsed_phases<1>(s, g, N, grp.n_filled, perm, eta, grp.fermionic, unit, ph);
+      const uint64_t m = __popcll(stab) > 1 ? rsed_permute(s[0], perm + e.y * N) : 0;
+      o = ket_bra(e, s[0], m, c, ph[0], stab, mem, grp, perm, eta, chi);
+    }
+    out[r] = o;
+  }
+}
+
+// Sum over the orbits of |c|^2 per occupied site of the representative, lane =
+// site (and site + 32); one partial per block.
+__global__ void __launch_bounds__(kCT) k_obdm_diag(int64_t n_orbits, const uint64_t* __restrict__ repr_masks,
+                                                   const double2* __restrict__ x, double* __restrict__ part) {
+  __shared__ double sums[kCT / 32][64];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double lo = 0.0, hi = 0.0;
+  for (int64_t o0 = ((int64_t)blockIdx.x * (kCT / 32) + warp) * 32; o0 < n_orbits;
+       o0 += (int64_t)gridDim.x * kCT) {
+    const int64_t o = o0 + lane;
+    uint64_t m = 0;
+    double w = 0.0;
+    if (o < n_orbits) {
+      const double2 c = __ldg(x + o);
+      m = __ldg(repr_masks + o);
+      w = c.x * c.x + c.y * c.y;
+    }
+    for (int q = 0; q < 32; ++q) {
+      const uint64_t mq = __shfl_sync(0xffffffffu, m, q);
+      const double wq = __shfl_sync(0xffffffffu, w, q);
+      if ((mq >> lane) & 1ull) lo += wq;
+      if ((mq >> (lane + 32)) & 1ull) hi += wq;
+    }
+  }
+  sums[warp][lane] = lo;
+  sums[warp][lane + 32] = hi;
+  __syncthreads();
+  if (threadIdx.x < 64) {
+    double s = 0.0;
+    for (int w = 0; w < kCT / 32; ++w) s += sums[w][threadIdx.x];
+    part[blockIdx.x * 64 + threadIdx.x] = s;
+  }
+}
+
+// rho[j][j] = (1/|G|) sum_g D[a] with g(a) = j, D the block partials' sum; one
+// block of 64 threads.
+__global__ void k_obdm_rotate(rsed_group_t grp, const double* __restrict__ part, int n_blocks,
+                              double2* __restrict__ rho) {
+  __shared__ double D[64];
+  const int t = threadIdx.x, N = grp.n_site;
+  double s = 0.0;
+#pragma unroll 8
+  for (int b = 0; b < n_blocks; ++b) s += part[b * 64 + t];
+  D[t] = s;
+  __syncthreads();
+  if (t >= N) return;
+  double d = 0.0;
+  for (int g = 0; g < grp.n_group; ++g)
+    for (int a = 0; a < N; ++a)
+      if (grp.perm[g * N + a] == t) d += D[a];
+  rho[t * N + t] = make_double2(d / (double)grp.n_group, 0.0);
+}
+
+template <int NP, bool DENSE>
+__global__ void __launch_bounds__(kCT, DENSE && NP == 32 ? 3 : 2) k_obdm_part(rsed_group_t grp, const int4* __restrict__ table,
                                                       const uint64_t* __restrict__ repr_masks,
                                                       const uint64_t* __restrict__ stab_mask,
                                                       const uint64_t* __restrict__ member, int sector,
                                                       const double2* __restrict__ chi_g,
                                                       const double2* __restrict__ x, int per_warp,
                                                       int64_t n_a, int64_t n_b, ObdmLayout lay,
+                                                      const KetBra* __restrict__ states,
                                                       double2* __restrict__ part) {
   using T = ObdmTile<NP>;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -106,35 +235,26 @@ __global__ void __launch_bounds__(kCT, 2) k_obdm_part(rsed_group_t grp, const in
   double2* eta = reinterpret_cast<double2*>(smem + lay.eta);
   double2* chi = reinterpret_cast<double2*>(smem + lay.chi);
   int64_t* binom = reinterpret_cast<int64_t*>(smem + lay.binom);
-  double* diag = reinterpret_cast<double*>(smem + lay.diag);
   uint8_t* perm = smem + lay.perm;
-  const int N = grp.n_site, ng = grp.n_group, kp1 = grp.n_filled + 1;
+  const int N = grp.n_site, kp1 = grp.n_filled + 1;
   for (int i = threadIdx.x; i < (N + 1) * kp1; i += kCT) binom[i] = grp.binom[i];
-  bool twisted = false;
-  for (int i = threadIdx.x; i < ng * N; i += kCT) {
-    const double2 v = reinterpret_cast<const double2*>(grp.eta)[i];
-    twisted |= v.x != 1.0 || v.y != 0.0;
-    eta[i] = v;
-    perm[i] = grp.perm[i];
-  }
-  for (int i = threadIdx.x; i < ng; i += kCT) chi[i] = chi_g[i];
-  const bool unit = __syncthreads_or(twisted) == 0;
+  bool unit = false;
+  if constexpr (DENSE)
+    __syncthreads();
+  else
+    unit = stage_phases(grp, chi_g, eta, perm, chi);
   const uint64_t first = (1ull << grp.n_filled) - 1ull;  // stands in for missing states (N <= 63)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const bool fermion = grp.fermionic != 0;
   const uint64_t sb = grp.species_b;
   const int64_t cb = sb ? binom[__popcll(sb) * kp1 + grp.n_filled_b] : 1;
-  const double inv_ng = 1.0 / (double)ng;
   const uint64_t all = (1ull << N) - 1ull;
   double2 acc[T::RT][T::RT];
 #pragma unroll
   for (int a = 0; a < T::RT; ++a)
 #pragma unroll
     for (int b = 0; b < T::RT; ++b) acc[a][b] = make_double2(0.0, 0.0);
-  double dacc[NP / 32];
-#pragma unroll
-  for (int h = 0; h < NP / 32; ++h) dacc[h] = 0.0;
   const int64_t per_chunk = (int64_t)(kCT / 32) * per_warp;
   const int64_t chunks_a = (n_a + per_chunk - 1) / per_chunk, chunks_b = (n_b + per_chunk - 1) / per_chunk;
   for (int64_t ch = blockIdx.x; ch < chunks_a + chunks_b; ch += gridDim.x) {
@@ -166,52 +286,48 @@ __global__ void __launch_bounds__(kCT, 2) k_obdm_part(rsed_group_t grp, const in
         if (ok[u]) idx[u] = sb ? rsed_rank2(nn | (1ull << i), binom, kp1, sb, cb) : rank_with(nn, i, binom, kp1);
         ok[u] = ok[u] && idx[u] >= 0 && idx[u] < grp.n_states;
       }
-      int4 e[T::U];
+      KetBra kb[T::U];
+      if constexpr (DENSE) {
 #pragma unroll
-      for (int u = 0; u < T::U; ++u) e[u] = ok[u] ? __ldg(table + idx[u]) : make_int4(-1, 0, 0, 0);
-      double2 c[T::U], ph[T::U];
-      uint64_t s[T::U], st[T::U], mem[T::U];
-      int ge[T::U];
-#pragma unroll
-      for (int u = 0; u < T::U; ++u) {
-        c[u] = make_double2(0.0, 0.0);
-        s[u] = first;
-        st[u] = mem[u] = 0;
-        ge[u] = e[u].y;
-        if (e[u].x >= 0) {
-          c[u] = __ldg(x + e[u].x);
-          s[u] = __ldg(repr_masks + e[u].x);
-          st[u] = __ldg(stab_mask + e[u].x);
-          mem[u] = __ldg(member + e[u].x);
+        for (int u = 0; u < T::U; ++u) {
+          kb[u].ket = kb[u].bra = make_double2(0.0, 0.0);
+          if (ok[u])
+            asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                : "=d"(kb[u].ket.x), "=d"(kb[u].ket.y), "=d"(kb[u].bra.x), "=d"(kb[u].bra.y)
+                : "l"(states + idx[u]));
         }
+      } else {
+        int4 e[T::U];
+#pragma unroll
+        for (int u = 0; u < T::U; ++u) e[u] = ok[u] ? __ldg(table + idx[u]) : make_int4(-1, 0, 0, 0);
+        double2 c[T::U], ph[T::U];
+        uint64_t s[T::U], st[T::U], mem[T::U];
+        int ge[T::U];
+#pragma unroll
+        for (int u = 0; u < T::U; ++u) {
+          c[u] = make_double2(0.0, 0.0);
+          s[u] = first;
+          st[u] = mem[u] = 0;
+          ge[u] = e[u].y;
+          if (e[u].x >= 0) {
+            c[u] = __ldg(x + e[u].x);
+            s[u] = __ldg(repr_masks + e[u].x);
+            st[u] = __ldg(stab_mask + e[u].x);
+            mem[u] = __ldg(member + e[u].x);
+          }
+        }
+        rsed_phases<T::U>(s, ge, N, grp.n_filled, perm, eta, fermion, unit, ph);
+#pragma unroll
+        for (int u = 0; u < T::U; ++u)
+          kb[u] = ket_bra(e[u], s[u], n[u / (NP / 32)] | (1ull << ((lane + 32 * (u % (NP / 32))) & 63)), c[u], ph[u], st[u],
+                          (mem[u] >> sector) & 1ull, grp, perm, eta, chi);
       }
-      rsed_phases<T::U>(s, ge, N, grp.n_filled, perm, eta, fermion, unit, ph);
 #pragma unroll
       for (int u = 0; u < T::U; ++u) {
-        const int i = lane + 32 * (u % (NP / 32));
-        const uint64_t nn = n[u / (NP / 32)];
-        double2 K = make_double2(0.0, 0.0), B = make_double2(0.0, 0.0);
-        if (e[u].x >= 0 && (c[u].x != 0.0 || c[u].y != 0.0)) {
-          const double S = (double)__popcll(st[u]);
-          const double norm = 1.0 / sqrt((double)ng * S);
-          K = rsed_state_amplitude(s[u], nn | (1ull << i), e[u].y, ph[u], st[u], grp, perm, eta, chi,
-                                   make_double2(c[u].x * norm, c[u].y * norm));
-          if ((mem[u] >> sector) & 1ull) {
-            const double2 ch = chi[e[u].y];
-            const double2 pc = cmul(make_double2((double)__int_as_float(e[u].z), (double)__int_as_float(e[u].w)),
-                                    make_double2(ch.x, -ch.y));
-            const double sr = S * norm;  // sqrt(S / |G|)
-            B = cmul(c[u], make_double2(sr * pc.x, -sr * pc.y));
-          }
-          if (fermion && (__popcll(nn & ((1ull << i) - 1ull)) & 1)) {
-            K = make_double2(-K.x, -K.y);
-            B = make_double2(-B.x, -B.y);
-          }
-          dacc[u % (NP / 32)] += (c[u].x * c[u].x + c[u].y * c[u].y) * S * inv_ng;
-        }
-        const int q = warp * T::NW + u / (NP / 32);
-        Kt[q * NP + i] = K;
-        Bt[q * NP + i] = B;
+        const int i = lane + 32 * (u % (NP / 32)), q = warp * T::NW + u / (NP / 32);
+        const bool flip = fermion && (__popcll(n[u / (NP / 32)] & ((1ull << i) - 1ull)) & 1);
+        Kt[q * NP + i] = flip ? make_double2(-kb[u].ket.x, -kb[u].ket.y) : kb[u].ket;
+        Bt[q * NP + i] = flip ? make_double2(-kb[u].bra.x, -kb[u].bra.y) : kb[u].bra;
       }
       __syncthreads();
 #pragma unroll 4
@@ -232,22 +348,13 @@ __global__ void __launch_bounds__(kCT, 2) k_obdm_part(rsed_group_t grp, const in
       __syncthreads();
     }
   }
-#pragma unroll
-  for (int h = 0; h < NP / 32; ++h) diag[warp * 64 + lane + 32 * h] = dacc[h];
-  __syncthreads();
-  double2* out = part + (int64_t)blockIdx.x * N * N;
+  double2* out = part + (int64_t)blockIdx.x * N * N;  // the diagonal is overwritten later
 #pragma unroll
   for (int a = 0; a < T::RT; ++a)
 #pragma unroll
     for (int b = 0; b < T::RT; ++b) {
       const int i = ty + 16 * a, j = tx + 16 * b;
-      if (i >= N || j >= N) continue;
-      double2 v = acc[a][b];
-      if (i == j) {
-        v = make_double2(0.0, 0.0);
-        for (int w = 0; w < kCT / 32; ++w) v.x += diag[w * 64 + i];
-      }
-      out[i * N + j] = v;
+      if (i < N && j < N) out[i * N + j] = acc[a][b];
     }
 }
 
@@ -328,15 +435,16 @@ int64_t choose(int n, int k) {
   return (int64_t)c;
 }
 
-template <int NP>
+template <int NP, bool DENSE>
 int obdm_launch(const rsed_group_t& grp, const int4* table, const uint64_t* repr_masks, const uint64_t* stab_mask,
                 const uint64_t* member, int sector, const double2* chi, const double2* x, int64_t n_a, int64_t n_b,
-                double2* part, int* grid_out, cudaStream_t stream) {
-  const ObdmLayout lay = obdm_layout(grp.n_site, grp.n_filled, grp.n_group);
+                const KetBra* states, double2* part, int* grid_out, cudaStream_t stream) {
+  auto kern = k_obdm_part<NP, DENSE>;
+  const ObdmLayout lay = obdm_layout(grp.n_site, grp.n_filled, DENSE ? 0 : grp.n_group);
   if (lay.total > 48 * 1024)
-    RSED_TRY_CUDA(cudaFuncSetAttribute(k_obdm_part<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.total));
+    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.total));
   const int n_sm = sm_count();
-  const int wave = one_wave((const void*)k_obdm_part<NP>, lay.total);
+  const int wave = one_wave((const void*)kern, lay.total);
   RSED_REQUIRE(n_sm > 0 && wave > 0, RSED_ECUDA, "no occupancy for the one-body density kernel");
   int64_t grid = wave < n_sm * kObdmBlocksPerSm ? wave : n_sm * kObdmBlocksPerSm;
   // states n per warp: 32 amortise the unranking; fewer when the blocks of one
@@ -346,12 +454,18 @@ int obdm_launch(const rsed_group_t& grp, const int4* table, const uint64_t* repr
   const int64_t pc = 8 * per_warp;
   const int64_t chunks = (n_a + pc - 1) / pc + (n_b + pc - 1) / pc;
   if (grid > chunks) grid = chunks;
-  k_obdm_part<NP><<<(unsigned)grid, kCT, lay.total, stream>>>(grp, table, repr_masks, stab_mask, member, sector, chi,
-                                                              x, per_warp, n_a, n_b, lay, part);
+  kern<<<(unsigned)grid, kCT, lay.total, stream>>>(grp, table, repr_masks, stab_mask, member, sector, chi, x, per_warp,
+                                                   n_a, n_b, lay, states, part);
   RSED_CHECK_LAUNCH();
   *grid_out = (int)grid;
   return RSED_OK;
 }
+
+// Partial matrices, then the diagonal's partials (64 per SM).
+size_t obdm_part_bytes(int n_site, int n_sm) {
+  return align_up(sizeof(double2) * (size_t)n_sm * kObdmBlocksPerSm * n_site * n_site, 256);
+}
+size_t obdm_diag_bytes(int n_sm) { return align_up(sizeof(double) * 64 * (size_t)n_sm, 256); }
 
 int pairs_grid(int n_site, size_t* smem) {
   *smem = sizeof(double) * (size_t)n_site * n_site;
@@ -363,7 +477,11 @@ int pairs_grid(int n_site, size_t* smem) {
 extern "C" size_t rsed_obdm_scratch_bytes(int32_t n_site) {
   const int n_sm = sm_count();
   if (n_sm <= 0) return 0;
-  return sizeof(double2) * (size_t)n_sm * kObdmBlocksPerSm * n_site * n_site;
+  return obdm_part_bytes(n_site, n_sm) + obdm_diag_bytes(n_sm);
+}
+
+extern "C" size_t rsed_obdm_states_bytes(int64_t n_states) {
+  return n_states < 1 ? 0 : sizeof(KetBra) * (size_t)n_states;
 }
 
 extern "C" int rsed_one_body_density(const rsed_group_t* grp, const rsed_entry_t* table, int64_t n_orbits,
@@ -393,15 +511,42 @@ extern "C" int rsed_one_body_density(const rsed_group_t* grp, const rsed_entry_t
     RSED_TRY_CUDA(cudaMemsetAsync(rho, 0, sizeof(double2) * (size_t)nn, stream));
     return RSED_OK;
   }
-  double2* part = reinterpret_cast<double2*>(scratch);
+  const int n_sm = sm_count();
+  RSED_REQUIRE(n_sm > 0, RSED_ECUDA, "no device");
+  char* base = reinterpret_cast<char*>(scratch);
+  double2* part = reinterpret_cast<double2*>(base);
+  double* dpart = reinterpret_cast<double*>(base + obdm_part_bytes(N, n_sm));
   const int4* tb = reinterpret_cast<const int4*>(table);
   const double2* ch = reinterpret_cast<const double2*>(chi);
   const double2* xo = reinterpret_cast<const double2*>(x_orbit);
+  // the caller's scratch decides: the states written once if they fit (32-B
+  // aligned), else evaluated at every lookup
+  KetBra* states = reinterpret_cast<KetBra*>(base + rsed_obdm_scratch_bytes(N));
+  const bool dense = scratch_bytes >= rsed_obdm_scratch_bytes(N) + rsed_obdm_states_bytes(grp->n_states) &&
+                     (reinterpret_cast<uintptr_t>(states) & 31) == 0;
+  if (dense) {
+    const ObdmLayout lay = obdm_layout(N, grp->n_filled, grp->n_group);
+    if (lay.total > 48 * 1024)
+      RSED_TRY_CUDA(cudaFuncSetAttribute(k_obdm_states, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.total));
+    const int wave = one_wave((const void*)k_obdm_states, lay.total);
+    RSED_REQUIRE(wave > 0, RSED_ECUDA, "no occupancy for the state kernel");
+    const int64_t blocks = (grp->n_states + kCT - 1) / kCT;
+    k_obdm_states<<<(unsigned)(blocks < wave ? blocks : wave), kCT, lay.total, stream>>>(
+        *grp, tb, repr_masks, stab_mask, member, sector, ch, xo, lay, states);
+    RSED_CHECK_LAUNCH();
+  }
   int grid = 0;
-  rc = N <= 32 ? obdm_launch<32>(*grp, tb, repr_masks, stab_mask, member, sector, ch, xo, n_a, n_b, part, &grid, stream)
-               : obdm_launch<64>(*grp, tb, repr_masks, stab_mask, member, sector, ch, xo, n_a, n_b, part, &grid, stream);
+  auto launch = N <= 32 ? (dense ? obdm_launch<32, true> : obdm_launch<32, false>)
+                        : (dense ? obdm_launch<64, true> : obdm_launch<64, false>);
+  rc = launch(*grp, tb, repr_masks, stab_mask, member, sector, ch, xo, n_a, n_b, states, part, &grid, stream);
   if (rc) return rc;
   k_sum_blocks<2><<<(nn + 3) / 4, 128, 0, stream>>>(reinterpret_cast<const double*>(part), grid, nn, rho);
+  RSED_CHECK_LAUNCH();
+  const int64_t dblocks = (n_orbits + kCT - 1) / kCT;
+  const int dgrid = (int)(dblocks < n_sm ? dblocks : n_sm);
+  k_obdm_diag<<<dgrid, kCT, 0, stream>>>(n_orbits, repr_masks, xo, dpart);
+  RSED_CHECK_LAUNCH();
+  k_obdm_rotate<<<1, 64, 0, stream>>>(*grp, dpart, dgrid, reinterpret_cast<double2*>(rho));
   RSED_CHECK_LAUNCH();
   return RSED_OK;
 }

@@ -53,8 +53,9 @@ def _vector(n, seed):
     ("checkerboard", (4, 4), 2, None, 9),
     ("checkerboard", (3, 6), 2, (0.1, 0.3), 4),
 ])
-def test_one_body_density_sizes(family, size, nf, theta, sector):
+def test_one_body_density_sizes(family, size, nf, theta, sector, monkeypatch):
     import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import _lib
     from realspace_exatdiagonalization_py_b200 import correlators as cr
 
     data, sset, cat, perm0, eta = _case(family, size, nf, theta)
@@ -70,6 +71,10 @@ def test_one_body_density_sizes(family, size, nf, theta, sector):
     # entries are at most nf and sums of at most a few thousand terms
     np.testing.assert_allclose(rho, ref, atol=1e-12, rtol=0)
     np.testing.assert_array_equal(rho, cr.one_body_density_matrix(basis, c))
+    # without room for the states' amplitudes: evaluated at every lookup
+    lib = _lib.lib()
+    monkeypatch.setattr(lib, "rsed_obdm_states_bytes", lambda n: 0)
+    np.testing.assert_allclose(cr.one_body_density_matrix(basis, c), ref, atol=1e-12, rtol=0)
 
 
 # one state, several blocks' worth of ranks, symmetric orbits (the sum over the
