@@ -51,8 +51,8 @@ int one_wave(const void* fn, size_t smem) {
 // (k_obdm_diag).
 // 32 sites, 8 bosons, 10.5 million states: 120.6 ms with one rank, table and
 // coefficient chain per hop and thread; 6.5 ms evaluating each lookup (a state
-// k times; 24 % occupancy, latency of the dependent loads); @MS@ with the
-// states written first.
+// k times; 24 % occupancy, latency of the dependent loads); 2.62 ms plus 0.25 for
+// the states with the states written first.
 template <int NP>
 struct ObdmTile {
   static constexpr int TN = NP == 32 ? 32 : 16;       // states n of one tile
@@ -200,22 +200,22 @@ __global__ void __launch_bounds__(kCT) k_obdm_diag(int64_t n_orbits, const uint6
 }
 
 // rho[j][j] = (1/|G|) sum_g D[a] with g(a) = j, D the block partials' sum; one
-// block of 64 threads.
-__global__ void k_obdm_rotate(rsed_group_t grp, const double* __restrict__ part, int n_blocks,
-                              double2* __restrict__ rho) {
+// block, 16 lanes per site.
+__global__ void __launch_bounds__(1024) k_obdm_rotate(rsed_group_t grp, const double* __restrict__ part, int n_blocks,
+                                                      double2* __restrict__ rho) {
   __shared__ double D[64];
-  const int t = threadIdx.x, N = grp.n_site;
+  const int t = threadIdx.x / 16, h = threadIdx.x % 16, N = grp.n_site;
   double s = 0.0;
-#pragma unroll 8
-  for (int b = 0; b < n_blocks; ++b) s += part[b * 64 + t];
-  D[t] = s;
+  for (int b = h; b < n_blocks; b += 16) s += part[b * 64 + t];
+  for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (h == 0) D[t] = s;
   __syncthreads();
-  if (t >= N) return;
   double d = 0.0;
-  for (int g = 0; g < grp.n_group; ++g)
-    for (int a = 0; a < N; ++a)
-      if (grp.perm[g * N + a] == t) d += D[a];
-  rho[t * N + t] = make_double2(d / (double)grp.n_group, 0.0);
+  if (t < N)
+    for (int e = h; e < grp.n_group * N; e += 16)
+      if (grp.perm[e] == t) d += D[e % N];
+  for (int o = 8; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+  if (t < N && h == 0) rho[t * N + t] = make_double2(d / (double)grp.n_group, 0.0);
 }
 
 template <int NP, bool DENSE>
@@ -362,38 +362,62 @@ __global__ void __launch_bounds__(kCT, DENSE && NP == 32 ? 3 : 2) k_obdm_part(rs
 //
 // D[a][b] = sum_o |x_o|^2 n_a(s_o) n_b(s_o) over the representatives s_o; the
 // structure factor's C[i][j] = (1/|G|) sum_g D[a][b] at i = g(a), j = g(b)
-// follows from it on the host.
-__global__ void __launch_bounds__(kCT) k_pairs_part(int n_site, int64_t n_orbits,
-                                                    const uint64_t* __restrict__ repr_masks,
-                                                    const double2* __restrict__ x, double* __restrict__ part) {
-  extern __shared__ double dacc[];
-  __shared__ uint64_t sm[kCT];
-  __shared__ double sw[kCT];
-  const int N = n_site, NN = N * N;
-  const int64_t n_chunks = (n_orbits + kCT - 1) / kCT;
-  for (int p = threadIdx.x; p < NN; p += kCT) dacc[p] = 0.0;
-  for (int64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
-    __syncthreads();
-    const int64_t o = ch * kCT + threadIdx.x;
+// follows from it on the host.  A warp takes 32 orbits at a time and adds each
+// to the 32 rows a of its half (blockIdx.y) that are occupied, lane = b (and
+// b + 32), all sums in registers: two instructions per row, no atomics.
+// 657,756 orbits of 8 bosons on 32 sites: 185 us with every thread testing its
+// pairs against every orbit, 255 us with the rows in shared memory (a chain of
+// read-modify-writes), 117 us in this form.
+template <int NH>
+__global__ void __launch_bounds__(NH == 1 ? 256 : 128, NH == 1 ? 2 : 3)
+    k_pairs_part(int n_site, int64_t n_orbits, const uint64_t* __restrict__ repr_masks,
+                 const double2* __restrict__ x, double* __restrict__ part) {
+  constexpr int W = 32 * NH;
+  extern __shared__ double dacc[];  // [warp][32][W]
+  const int N = n_site, warps = blockDim.x >> 5, a0 = 32 * blockIdx.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double acc[NH][32];
+#pragma unroll
+  for (int h = 0; h < NH; ++h)
+#pragma unroll
+    for (int a = 0; a < 32; ++a) acc[h][a] = 0.0;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t o0 = (int64_t)blockIdx.x * blockDim.x + warp * 32; o0 < n_orbits; o0 += step) {
+    const int64_t o = o0 + lane;
+    uint64_t m = 0;
+    double w = 0.0;
     if (o < n_orbits) {
-      const double2 c = x[o];
-      sm[threadIdx.x] = repr_masks[o];
-      sw[threadIdx.x] = c.x * c.x + c.y * c.y;
-    } else {
-      sm[threadIdx.x] = 0;
-      sw[threadIdx.x] = 0.0;
+      const double2 c = __ldg(x + o);
+      m = __ldg(repr_masks + o);
+      w = c.x * c.x + c.y * c.y;
     }
-    __syncthreads();
-    for (int p = threadIdx.x; p < NN; p += kCT) {
-      const uint64_t both = (1ull << (p / N)) | (1ull << (p % N));
-      double d = dacc[p];
-      for (int q = 0; q < kCT; ++q)
-        if ((sm[q] & both) == both) d += sw[q];
-      dacc[p] = d;
+    for (int q = 0; q < 32; ++q) {
+      const uint64_t mq = __shfl_sync(0xffffffffu, m, q);
+      const double wq = __shfl_sync(0xffffffffu, w, q);
+      const uint32_t rows = (uint32_t)(mq >> a0);
+      double wl[NH];
+#pragma unroll
+      for (int h = 0; h < NH; ++h) wl[h] = (mq >> (lane + 32 * h)) & 1ull ? wq : 0.0;
+#pragma unroll
+      for (int a = 0; a < 32; ++a)
+        if (rows & (1u << a)) {
+#pragma unroll
+          for (int h = 0; h < NH; ++h) acc[h][a] += wl[h];
+        }
     }
   }
+  double* D = dacc + (size_t)warp * 32 * W + lane;
+#pragma unroll
+  for (int a = 0; a < 32; ++a)
+#pragma unroll
+    for (int h = 0; h < NH; ++h) D[a * W + 32 * h] = acc[h][a];
   __syncthreads();
-  for (int p = threadIdx.x; p < NN; p += kCT) part[(int64_t)blockIdx.x * NN + p] = dacc[p];
+  const int rows = min(32, N - a0);
+  for (int p = threadIdx.x; p < rows * N; p += blockDim.x) {
+    double s = 0.0;
+    for (int v = 0; v < warps; ++v) s += dacc[((size_t)v * 32 + p / N) * W + p % N];
+    part[((int64_t)blockIdx.x * N + a0) * N + p] = s;
+  }
 }
 
 // out[p] = sum over the blocks' partials, one warp per entry: lane l adds
@@ -466,11 +490,6 @@ size_t obdm_part_bytes(int n_site, int n_sm) {
   return align_up(sizeof(double2) * (size_t)n_sm * kObdmBlocksPerSm * n_site * n_site, 256);
 }
 size_t obdm_diag_bytes(int n_sm) { return align_up(sizeof(double) * 64 * (size_t)n_sm, 256); }
-
-int pairs_grid(int n_site, size_t* smem) {
-  *smem = sizeof(double) * (size_t)n_site * n_site;
-  return one_wave((const void*)k_pairs_part, *smem);
-}
 
 }  // namespace
 
@@ -546,16 +565,15 @@ extern "C" int rsed_one_body_density(const rsed_group_t* grp, const rsed_entry_t
   const int dgrid = (int)(dblocks < n_sm ? dblocks : n_sm);
   k_obdm_diag<<<dgrid, kCT, 0, stream>>>(n_orbits, repr_masks, xo, dpart);
   RSED_CHECK_LAUNCH();
-  k_obdm_rotate<<<1, 64, 0, stream>>>(*grp, dpart, dgrid, reinterpret_cast<double2*>(rho));
+  k_obdm_rotate<<<1, 1024, 0, stream>>>(*grp, dpart, dgrid, reinterpret_cast<double2*>(rho));
   RSED_CHECK_LAUNCH();
   return RSED_OK;
 }
 
 extern "C" size_t rsed_density_pairs_scratch_bytes(int32_t n_site) {
-  size_t smem = 0;
-  const int grid = pairs_grid(n_site, &smem);
-  if (grid <= 0) return 0;
-  return sizeof(double) * (size_t)grid * n_site * n_site;
+  const int n_sm = sm_count();
+  if (n_sm <= 0) return 0;
+  return sizeof(double) * (size_t)(2 * n_sm) * n_site * n_site;
 }
 
 extern "C" int rsed_density_pairs(int32_t n_site, int64_t n_orbits, const uint64_t* repr_masks,
@@ -565,15 +583,21 @@ extern "C" int rsed_density_pairs(int32_t n_site, int64_t n_orbits, const uint64
                RSED_MAX_SITES);
   RSED_REQUIRE(repr_masks && x_orbit && pairs && scratch && n_orbits >= 1, RSED_EINVAL,
                "bad density-pair arguments");
-  size_t smem = 0;
-  const int grid = pairs_grid(n_site, &smem);
-  RSED_REQUIRE(grid > 0, RSED_ECUDA, "no occupancy for the density-pair kernel");
-  RSED_REQUIRE(scratch_bytes >= sizeof(double) * (size_t)grid * n_site * n_site, RSED_ESCRATCH,
+  RSED_REQUIRE(scratch_bytes >= rsed_density_pairs_scratch_bytes(n_site), RSED_ESCRATCH,
                "density-pair scratch too small");
   cudaStream_t stream = as_stream(stream_);
   double* part = reinterpret_cast<double*>(scratch);
-  k_pairs_part<<<grid, kCT, smem, stream>>>(n_site, n_orbits, repr_masks, reinterpret_cast<const double2*>(x_orbit),
-                                           part);
+  const bool wide = n_site > 32;
+  const int threads = wide ? 128 : 256;
+  const size_t smem = sizeof(double) * (size_t)(threads / 32) * 32 * (wide ? 64 : 32);  // 64 KB
+  auto kern = wide ? k_pairs_part<2> : k_pairs_part<1>;
+  RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int n_sm = sm_count();
+  RSED_REQUIRE(n_sm > 0, RSED_ECUDA, "no device");
+  const int64_t blocks = (n_orbits + threads - 1) / threads;
+  const int grid = (int)(blocks < 2 * n_sm ? blocks : 2 * n_sm);
+  kern<<<dim3(grid, wide ? 2 : 1), threads, smem, stream>>>(n_site, n_orbits, repr_masks,
+                                                           reinterpret_cast<const double2*>(x_orbit), part);
   RSED_CHECK_LAUNCH();
   const int nn = n_site * n_site;
   k_sum_blocks<1><<<(nn + 3) / 4, 128, 0, stream>>>(part, grid, nn, pairs);

@@ -259,3 +259,25 @@ def test_restart_sizes(n_site, n_inst, block):
     b.restart()
     # sums of 48 products of size about 10 in another order
     assert (b.V - want).abs().max() < 1e-11
+
+
+# fewer and more than 32 sites, fewer orbits than a warp takes, several blocks
+@pytest.mark.parametrize("family,size,nf", [
+    ("haldane", (2, 3), 0), ("haldane", (2, 3), 12), ("heisenberg", (18, 1), 9), ("checkerboard", (4, 4), 3),
+    ("checkerboard", (3, 6), 3), ("checkerboard", (3, 7), 2),
+])
+def test_density_pairs_sizes(family, size, nf):
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import correlators as cr
+
+    data, sset, cat, _, _ = _case(family, size, nf)
+    n = data.orbit_catalog.n_site
+    s = next(k for k, d in enumerate(sset.dims) if d)
+    basis = ed.Symmetry_Sector_Basis(data.irrep_list[s], data.orbit_catalog, sset, s)
+    c = _vector(basis.dim, 5)
+    masks = np.array([int(cat["reprs"][o]) for o in port.sector_orbits(cat, np.asarray(data.irrep_list[s].values))],
+                     dtype=np.uint64)
+    occ = ((masks[:, None] >> np.arange(n, dtype=np.uint64)) & np.uint64(1)).astype(float)
+    ref = (occ * (np.abs(c) ** 2)[:, None]).T @ occ
+    # sums of weights that add up to 1
+    np.testing.assert_allclose(cr.density_pairs(basis, c), ref, atol=1e-14, rtol=0)
