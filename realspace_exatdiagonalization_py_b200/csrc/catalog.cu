@@ -145,7 +145,7 @@ __device__ bool stage_moves(const rsed_group_t& grp, const uint8_t* perm, GroupM
 // leaving the loop at the first smaller image saved nothing, and the images
 // themselves are the cost.  M = uint32_t up to 32 sites.
 // 10.5 million states, 32 sites, |G| = 16: 865 us with one image per occupied
-// site step and 32 ranks per thread, @MS@ in this form.
+// site step and 32 ranks per thread, 139 us in this form.
 template <typename M, int R>
 __global__ void __launch_bounds__(kFlagThreads) k_rep_flags(rsed_group_t grp, uint32_t* bitmap, int64_t* block_count,
                                                             int per_block, GroupSmemLayout lay) {
