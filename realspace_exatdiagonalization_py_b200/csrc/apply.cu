@@ -382,8 +382,8 @@ static int check_model(const rsed_model_t* md) {
   return RSED_OK;
 }
 
-extern "C" int rsed_apply_h(const rsed_model_t* md, const rsed_sectors_t* sc, const void* x, void* y,
-                            int32_t precision, int32_t variant, void* stream_) {
+int rsed_apply_pairs(const rsed_model_t* md, const rsed_sectors_t* sc, const void* x, void* y, int precision,
+                     int variant, int pairs, void* stream_) {
   int rc = check_model(md);
   if (rc) return rc;
   RSED_REQUIRE(sc && sc->member && sc->sqrt_stab && sc->chi && sc->col_sector, RSED_EINVAL,
@@ -399,13 +399,18 @@ extern "C" int rsed_apply_h(const rsed_model_t* md, const rsed_sectors_t* sc, co
   if (variant == 999) {
     variant = 0;  // automatic on-the-fly mapping even when a projection table is present
   } else if (variant >= 300 || (variant == 0 && have_proj)) {
-    return rsed_proj_apply(*md, *sc, x, reinterpret_cast<double2*>(y), precision, variant, stream);
+    return rsed_proj_apply(*md, *sc, x, reinterpret_cast<double2*>(y), precision, variant, pairs, stream);
   }
   if (precision == 64)
     return dispatch_apply<64>(*md, *sc, x, reinterpret_cast<double2*>(y), variant, stream);
   if (precision == 32)
     return dispatch_apply<32>(*md, *sc, x, reinterpret_cast<double2*>(y), variant, stream);
   return rsed_set_error(RSED_EINVAL, "precision must be 64 or 32");
+}
+
+extern "C" int rsed_apply_h(const rsed_model_t* md, const rsed_sectors_t* sc, const void* x, void* y,
+                            int32_t precision, int32_t variant, void* stream_) {
+  return rsed_apply_pairs(md, sc, x, y, precision, variant, -1, stream_);
 }
 
 extern "C" size_t rsed_triplet_scratch_bytes(int64_t n_rows) {

@@ -71,6 +71,7 @@ struct LzDims {
   int n_chunks;
   int pslots;  // n_slots + 2 reduction slots per instance
   bool uniform;  // every instance has bmax columns, 32-B segments of the rows
+  int pairs;     // columns 2i, 2i + 1 share a sector: 1 yes, 0 no, -1 unknown
 };
 
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
@@ -3020,7 +3021,9 @@ LzDims make_dims(const rsed_model_t* md, const rsed_sectors_t* sc, const rsed_la
   // bmax; with an even ld and aligned buffers a segment of an even block is
   // whole 32-B (V, W) and 16-B (Xf) words
   auto aligned = [](const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; };
-  d.uniform = sc->n_cols == st->n_inst * st->bmax && (d.ld & 1) == 0 && aligned(st->V, 32) && aligned(st->W, 32) &&
+  const bool full = sc->n_cols == st->n_inst * st->bmax;
+  d.pairs = st->bmax == 1 ? 0 : full ? (st->bmax % 2 == 0 ? 1 : 0) : -1;
+  d.uniform = full && (d.ld & 1) == 0 && aligned(st->V, 32) && aligned(st->W, 32) &&
               (st->Xf == nullptr || aligned(st->Xf, 16));
   return d;
 }
@@ -3459,7 +3462,7 @@ static int lz_iterate(const rsed_model_t* md, const rsed_sectors_t* sc, rsed_lan
   const double2* X = reinterpret_cast<const double2*>(st->V) + (int64_t)(st->n_slots + 1) * d.n_orb * d.ld;
   for (int it = 0; it < n_iter; ++it) {
     const void* xin = (st->precision == 32) ? (const void*)st->Xf : (const void*)X;
-    rc = rsed_apply_h(md, sc, xin, st->W, st->precision, apply_variant, stream_);
+    rc = rsed_apply_pairs(md, sc, xin, st->W, st->precision, apply_variant, d.pairs, stream_);
     if (rc) return rc;
     rc = launch_pass(*st, d, 1, stream);
     if (rc) return rc;
@@ -3504,7 +3507,7 @@ extern "C" int rsed_lanczos_rayleigh_ritz(const rsed_model_t* md, const rsed_sec
   const int64_t slot = d.n_orb * d.ld;
   double2* V = reinterpret_cast<double2*>(st->V);
   for (int l = 0; l <= st->keep_blocks; ++l) {
-    rc = rsed_apply_h(md, sc, V + l * slot, V + (st->keep_blocks + 1 + l) * slot, 64, apply_variant, stream_);
+    rc = rsed_apply_pairs(md, sc, V + l * slot, V + (st->keep_blocks + 1 + l) * slot, 64, apply_variant, d.pairs, stream_);
     if (rc) return rc;
   }
   const unsigned g = (unsigned)(d.n_chunks * d.n_inst);

@@ -161,84 +161,178 @@ __device__ __forceinline__ T ld_stream(const T* p) {
   return __ldcs(p);
 }
 
-// The hops of one row for an FP32 lane of 4 columns that form two sector
-// pairs (columns 0-1 in sector s0, 2-3 in s2) when the row belongs to every
-// sector of the warp: no per-column tests, one weight-character product per
-// pair, and the table entries of the next batch loaded while the current
-// batch gathers.  Missing entries past the row's end become (orbit 0,
-// weight 0), so the loop body has no branches (x is finite: the solver's
-// own Lanczos blocks).
-template <int L, int U>
-__device__ __forceinline__ void spmv_row_pairs32(const uint32_t* __restrict__ cgt, const float2* __restrict__ wt,
-                                                 int64_t e0, int64_t e1, int eslot, const char* __restrict__ xl,
-                                                 uint32_t rowb, const float2* ch0, const float2* ch2, int nsec,
-                                                 float2 acc[4]) {
-  constexpr int EPW = 32 / L;
-  constexpr int B = EPW * U;  // hops per batch and warp
-  float2 a0 = make_float2(0.f, 0.f), a1 = a0, a2 = a0, a3 = a0;
-  uint32_t cgn[U];
-  float2 wn[U];
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const int64_t idx = e0 + u * EPW + eslot;
-    const bool ok = idx < e1;
-    cgn[u] = ok ? ld_stream(cgt + idx) : 0u;
-    wn[u] = ok ? ld_stream(wt + idx) : make_float2(0.f, 0.f);
-  }
-  for (int64_t base = e0; base < e1; base += B) {
-    uint32_t cgc[U];
-    float2 wc[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      cgc[u] = cgn[u];
-      wc[u] = wn[u];
-    }
-    if (base + B < e1) {
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int64_t idx = base + B + u * EPW + eslot;
-        const bool ok = idx < e1;
-        cgn[u] = ok ? ld_stream(cgt + idx) : 0u;
-        wn[u] = ok ? ld_stream(wt + idx) : make_float2(0.f, 0.f);
-      }
-    }
-    float4 xa[U], xc[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      // the lane's 32-B segment in one 256-bit load (32-B aligned: see the caller)
-      const char* px = xl + (size_t)(cgc[u] & kOrbitMask) * rowb;
-      asm("{\n\t.reg .u64 ga;\n\tcvta.to.global.u64 ga, %8;\n\t"
-          "ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [ga];\n\t}"
-          : "=f"(xa[u].x), "=f"(xa[u].y), "=f"(xa[u].z), "=f"(xa[u].w), "=f"(xc[u].x), "=f"(xc[u].y),
-            "=f"(xc[u].z), "=f"(xc[u].w)
-          : "l"(px));
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int go = (int)(cgc[u] >> kOrbitBits) * nsec;
-      const float2 c0 = ch0[go], c2 = ch2[go];
-      const float2 w = wc[u];
-      const float p0x = w.x * c0.x - w.y * c0.y, p0y = w.x * c0.y + w.y * c0.x;
-      const float p2x = w.x * c2.x - w.y * c2.y, p2y = w.x * c2.y + w.y * c2.x;
-      a0.x += p0x * xa[u].x - p0y * xa[u].y;
-      a0.y += p0x * xa[u].y + p0y * xa[u].x;
-      a1.x += p0x * xa[u].z - p0y * xa[u].w;
-      a1.y += p0x * xa[u].w + p0y * xa[u].z;
-      a2.x += p2x * xc[u].x - p2y * xc[u].y;
-      a2.y += p2x * xc[u].y + p2y * xc[u].x;
-      a3.x += p2x * xc[u].z - p2y * xc[u].w;
-      a3.y += p2x * xc[u].w + p2y * xc[u].z;
-    }
-  }
-  acc[0] = a0;
-  acc[1] = a1;
-  acc[2] = a2;
-  acc[3] = a3;
+// A lane's 32-B segment of an x row (4 FP32 or 2 FP64 complex values) in one
+// 256-bit load.
+__device__ __forceinline__ void load_segment(const char* p, float2 (&v)[4]) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[2].x), "=f"(v[2].y), "=f"(v[3].x), "=f"(v[3].y)
+      : "l"(p));
+}
+__device__ __forceinline__ void load_segment(const char* p, double2 (&v)[2]) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(v[0].x), "=d"(v[0].y), "=d"(v[1].x), "=d"(v[1].y)
+      : "l"(p));
 }
 
+// The rows r0, r0 + step, ... of lanes whose 32-B segments hold pairs of columns
+// of one sector each (blocks of 2 or 4: FP32 two pairs, FP64 one), as long as
+// they belong to every sector of the warp (`need`); returns the first row that
+// does not (the caller takes it column by column and comes back) or one past
+// the end.
+//
+// The loop is bound by instruction issue and load latency as much as by the
+// gathers (with every target in one L1-sized window the FP32 form ran only 13 %
+// faster), so it is written for few instructions: entries at constant offsets
+// from per-lane pointers, a lane's characters in one shared-memory word
+// chp[g*L], one weight-character product per pair, no per-column tests, missing
+// entries past the row's end as (the row itself, weight 0) -- its x is read for
+// the diagonal anyway, so a non-finite value spreads no further than H takes it --
+// and the slots' sums combined by halving exchanges, so that every lane finishes
+// its share of the row.  The entries of the next batch -- of
+// this row or the next one, whose offsets are loaded a row ahead -- are fetched
+// while the current batch gathers.  U = 2 hops per lane and batch at 4 blocks
+// per SM: more warps hide the gathers better than deeper batches.
+// 36.7 million hops, 32 columns: FP32 1228 us in the per-row form with U = 4 at
+// 3 blocks per SM, 1103 us as here with U = 4, 1017 us with U = 2 (U = 3 at 3
+// blocks: 1035; U = 2 at 5 blocks spills: 1528); FP64 2637 us with per-column
+// tests, 2051 us in this form.
+template <int PREC, int L, int U>
+__device__ __forceinline__ int64_t spmv_rows_pairs(const rsed_model_t& md, const rsed_sectors_t& sc, int64_t r0,
+                                                   int64_t step, uint64_t need, int c0, bool live,
+                                                   const char* __restrict__ xl,
+                                                   const typename ProjTypes<PREC>::W* chp,
+                                                   const typename ProjTypes<PREC>::W* __restrict__ x,
+                                                   double2* __restrict__ y) {
+  using W = typename ProjTypes<PREC>::W;
+  using Real = typename ProjTypes<PREC>::Real;
+  constexpr int CPL = PREC == 32 ? 4 : 2;    // columns of a lane
+  constexpr int EPW = 32 / L;
+  constexpr int B = EPW * U;                 // hops per batch and warp
+  const int lane = threadIdx.x & 31, eslot = lane / L;
+  const uint32_t* __restrict__ cgt = md.proj_cg + eslot;
+  const W* __restrict__ wt =
+      reinterpret_cast<const W*>(PREC == 64 ? (const void*)md.proj_w64 : (const void*)md.proj_w32) + eslot;
+  const int64_t* __restrict__ rp = md.proj_rowptr;
+  const uint32_t rowb = (uint32_t)(sc.ld * sizeof(W));
+  if (r0 >= md.n_orbits || (sc.member[r0] & need) != need) return r0;
+  int64_t e0 = rp[r0];
+  int left = (int)(rp[r0 + 1] - e0);
+  uint32_t cgn[U];
+  W wn[U];
+  auto fetch = [&](int64_t row, int64_t e, int n) {  // the batch at e, n entries of its row left
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool ok = u * EPW + eslot < n;
+      cgn[u] = ok ? ld_stream(cgt + e + u * EPW) : (uint32_t)row;
+      if (ok) {
+        wn[u] = ld_stream(wt + e + u * EPW);
+      } else {
+        wn[u].x = 0;
+        wn[u].y = 0;
+      }
+    }
+  };
+  fetch(r0, e0, left);
+  for (int64_t r = r0;;) {
+    const int64_t rn = r + step;
+    const bool more = rn < md.n_orbits;
+    const uint64_t memn = more ? __ldg(sc.member + rn) : 0ull;
+    const int64_t en = more ? __ldg(rp + rn) : 0;
+    const int leftn = more ? (int)(__ldg(rp + rn + 1) - en) : 0;
+    W a[CPL];
+#pragma unroll
+    for (int j = 0; j < CPL; ++j) a[j].x = a[j].y = 0;
+    do {
+      uint32_t cgc[U];
+      W wc[U], xs[U][CPL];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        cgc[u] = cgn[u];
+        wc[u] = wn[u];
+        load_segment(xl + (uint64_t)(cgc[u] & kOrbitMask) * rowb, xs[u]);
+      }
+      e0 += B;
+      left -= B;
+      if (left > 0)
+        fetch(r, e0, left);
+      else
+        fetch(rn, en, leftn);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const W* ch = chp + (cgc[u] >> kOrbitBits) * (L * CPL / 2);
+#pragma unroll
+        for (int h = 0; h < CPL / 2; ++h) {
+          const W k = ch[h], w = wc[u];
+          const Real px = w.x * k.x - w.y * k.y, py = w.x * k.y + w.y * k.x;
+#pragma unroll
+          for (int j = 2 * h; j < 2 * h + 2; ++j) {
+            a[j].x += px * xs[u][j].x - py * xs[u][j].y;
+            a[j].y += px * xs[u][j].y + py * xs[u][j].x;
+          }
+        }
+      }
+    } while (left > 0);
+    // the slots' sums: halve the columns while there are two, then plain exchanges
+    constexpr int H1 = EPW >= 2, H2 = PREC == 32 && EPW >= 4;
+    if constexpr (H1) {
+      const bool up = lane & 16;
+#pragma unroll
+      for (int j = 0; j < CPL / 2; ++j) {
+        const W lo = a[j], hi = a[j + CPL / 2];
+        a[j].x = (up ? hi.x : lo.x) + __shfl_xor_sync(0xffffffffu, up ? lo.x : hi.x, 16);
+        a[j].y = (up ? hi.y : lo.y) + __shfl_xor_sync(0xffffffffu, up ? lo.y : hi.y, 16);
+      }
+    }
+    if constexpr (H2) {
+      const bool up = lane & 8;
+      const W lo = a[0], hi = a[1];
+      a[0].x = (up ? hi.x : lo.x) + __shfl_xor_sync(0xffffffffu, up ? lo.x : hi.x, 8);
+      a[0].y = (up ? hi.y : lo.y) + __shfl_xor_sync(0xffffffffu, up ? lo.y : hi.y, 8);
+    }
+    constexpr int OWN = CPL >> (H1 + H2);        // columns a lane finishes
+    constexpr int REST = 32 >> (H1 + H2);        // lanes that hold the same columns' parts
+#pragma unroll
+    for (int off = REST / 2; off >= L; off >>= 1) {
+#pragma unroll
+      for (int j = 0; j < OWN; ++j) {
+        a[j].x += __shfl_xor_sync(0xffffffffu, a[j].x, off);
+        a[j].y += __shfl_xor_sync(0xffffffffu, a[j].y, off);
+      }
+    }
+    const int col = c0 + (H1 ? (lane >> 4 & 1) * (CPL / 2) : 0) + (H2 ? (lane >> 3 & 1) : 0);
+    if (live && (lane & (REST - 1)) < L) {
+      const double2 hd = __ldg(reinterpret_cast<const double2*>(md.hdiag) + r);
+      const int64_t at = r * sc.ld + col;
+#pragma unroll
+      for (int j = 0; j < OWN; ++j) {
+        const W xr = __ldg(x + at + j);
+        const double xx = (double)xr.x, xy = (double)xr.y;
+        y[at + j] = make_double2((double)a[j].x + (hd.x * xx + hd.y * xy), (double)a[j].y + (hd.x * xy - hd.y * xx));
+      }
+    }
+    if (!more || (memn & need) != need) return rn;
+    r = rn;
+    e0 = en;
+    left = leftn;
+  }
+}
+
+// Byte offset of the pair table behind a character table of `bytes`.
+__host__ __device__ constexpr size_t pair_table_offset(size_t bytes) { return (bytes + 15) & ~(size_t)15; }
+
+// Whether a lane's segment is 32 B: the form with the pair loop.
+template <int PREC, int CPL>
+constexpr bool kWide = CPL * (PREC == 32 ? 8 : 16) == 32;
+
 template <int PREC, int L, int CPL, int U>
-__global__ void __launch_bounds__(256, 3) k_proj_spmv(rsed_model_t md, rsed_sectors_t sc, const void* __restrict__ xin,
-                                                   double2* __restrict__ y, int chunk0) {
+__global__ void __launch_bounds__(256, kWide<PREC, CPL> ? 4 : 3) k_proj_spmv(rsed_model_t md, rsed_sectors_t sc, const void* __restrict__ xin,
+                                                   double2* __restrict__ y, int chunk0, int guard) {
+  if (guard) {  // run only if the columns are (1) or are not (2) pairs of one sector each
+    bool same = true;
+    for (int c = 2 * (int)threadIdx.x; c < sc.n_cols; c += 2 * (int)blockDim.x)
+      same = same && c + 1 < sc.n_cols && sc.col_sector[c] == sc.col_sector[c + 1];
+    if ((__syncthreads_and(same) != 0) != (guard == 1)) return;
+  }
   using W = typename ProjTypes<PREC>::W;
   using Real = typename ProjTypes<PREC>::Real;
   constexpr int EPW = 32 / L;
@@ -255,6 +349,17 @@ __global__ void __launch_bounds__(256, 3) k_proj_spmv(rsed_model_t md, rsed_sect
     const double2 c = gchi[i];
     chi[g * nsec + s].x = (Real)c.x;
     chi[g * nsec + s].y = (Real)c.y;
+  }
+  // the characters of a lane's sector pairs side by side, [g][lane of the slot][pair]
+  W* chpair = reinterpret_cast<W*>(smem + pair_table_offset(sizeof(W) * (size_t)nchi));
+  if constexpr (kWide<PREC, CPL>) {
+    const int cfirst = (chunk0 + (int)blockIdx.y) * NC;
+    for (int i = threadIdx.x; i < md.n_group * (NC / 2); i += blockDim.x) {
+      const int g = i / (NC / 2), c = cfirst + i % (NC / 2) * 2;
+      const double2 k = gchi[(c < sc.n_cols ? sc.col_sector[c] : 0) * md.n_group + g];
+      chpair[i].x = (Real)k.x;
+      chpair[i].y = (Real)k.y;
+    }
   }
   __syncthreads();
   const W* __restrict__ wt = reinterpret_cast<const W*>(PREC == 64 ? (const void*)md.proj_w64
@@ -277,25 +382,37 @@ __global__ void __launch_bounds__(256, 3) k_proj_spmv(rsed_model_t md, rsed_sect
     fresh[j] = (j == 0) || sec[j] != sec[j - 1];
   }
   const char* xb = reinterpret_cast<const char*>(xin) + (size_t)c0 * sizeof(W);
-  // FP32 lanes of 4 columns in two sector pairs (blocks of 2 or 4 columns):
-  // the branch-free row loop whenever the row is in all of the warp's sectors.
-  // Lanes past the last column run it too, on column 0 of x (in bounds), and
-  // their sums are dropped.
+  // 32-B segments of sector pairs (blocks of 2 or 4 columns): the pair loop over
+  // the rows that are in all of the warp's sectors.  Lanes past the last column
+  // run it too, on column 0 of x (in bounds), and their sums are dropped.
   bool pairs = false;
   const char* xfast = xb;
-  int s0 = 0, s2 = 0;
-  if constexpr (PREC == 32 && CPL == 4) {
-    // a lane's 4 columns start at a multiple of 4: with ld a multiple of 4 too
-    // (and x 32-B aligned) each segment is 32-B aligned for one 256-bit load
-    const bool lane_ok = colv[3] ? (sec[1] == sec[0] && sec[3] == sec[2]) : !colv[0];
-    pairs = __all_sync(0xffffffffu, lane_ok) && (ld % 4) == 0 &&
-            (reinterpret_cast<uintptr_t>(xin) & 31) == 0;
+  uint64_t need = 0;  // the sectors of the warp's columns
+  if constexpr (kWide<PREC, CPL>) {
+    // a lane's segment starts at a multiple of CPL columns: with ld a multiple of
+    // CPL too (and x 32-B aligned) it is 32-B aligned for one 256-bit load
+    bool lane_ok = !colv[0];
+    if (colv[CPL - 1]) {
+      lane_ok = true;
+#pragma unroll
+      for (int j = 0; j < CPL; j += 2) lane_ok = lane_ok && sec[j + 1] == sec[j];
+    }
+    pairs = __all_sync(0xffffffffu, lane_ok) && (ld % CPL) == 0 && (reinterpret_cast<uintptr_t>(xin) & 31) == 0;
     if (!colv[0]) xfast = reinterpret_cast<const char*>(xin);
-    s0 = colv[0] ? sec[0] : 0;
-    s2 = colv[0] ? sec[2] : 0;
+    if (colv[0] && lane_ok)
+#pragma unroll
+      for (int j = 0; j < CPL; j += 2) need |= 1ull << sec[j];
+    for (int o = 16; o > 0; o >>= 1) need |= __shfl_xor_sync(0xffffffffu, need, o);
   }
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < md.n_orbits; r += warps) {
+    if constexpr (kWide<PREC, CPL>) {
+      if (pairs) {
+        r = spmv_rows_pairs<PREC, L, U>(md, sc, r, warps, need, c0, colv[0], xfast, chpair + lane % L * (CPL / 2),
+                                        reinterpret_cast<const W*>(xin), y);
+        if (r >= md.n_orbits) break;
+      }
+    }
     const uint64_t memr = sc.member[r];
     bool on[CPL];
     bool any = false;
@@ -307,17 +424,7 @@ __global__ void __launch_bounds__(256, 3) k_proj_spmv(rsed_model_t md, rsed_sect
     W acc[CPL];
 #pragma unroll
     for (int j = 0; j < CPL; ++j) acc[j].x = acc[j].y = (Real)0;
-    bool done = false;
-    if constexpr (PREC == 32 && CPL == 4) {
-      if (pairs && __all_sync(0xffffffffu, !colv[0] || (on[0] && on[1] && on[2] && on[3]))) {
-        const float2* chb = reinterpret_cast<const float2*>(chi);
-        spmv_row_pairs32<L, U>(cgt, reinterpret_cast<const float2*>(wt), rp[r], rp[r + 1], eslot, xfast,
-                               (uint32_t)(ld * sizeof(float2)), chb + s0, chb + s2, nsec,
-                               reinterpret_cast<float2*>(acc));
-        done = true;
-      }
-    }
-    if (!done && __any_sync(0xffffffffu, any)) {
+    if (__any_sync(0xffffffffu, any)) {
       const int64_t e0 = rp[r], e1 = rp[r + 1];
       for (int64_t base = e0; base < e1; base += EPW * U) {
         uint32_t cgv[U];
@@ -389,12 +496,13 @@ __global__ void __launch_bounds__(256, 3) k_proj_spmv(rsed_model_t md, rsed_sect
 
 template <int PREC, int L, int CPL>
 int launch_spmv(const rsed_model_t& md, const rsed_sectors_t& sc, const void* x, double2* y, bool sequential,
-                cudaStream_t stream) {
+                int guard, cudaStream_t stream) {
   using W = typename ProjTypes<PREC>::W;
-  constexpr int U = 4;
+  constexpr int U = kWide<PREC, CPL> ? 2 : 4;
   constexpr int NC = L * CPL;
   auto kern = k_proj_spmv<PREC, L, CPL, U>;
-  const size_t smem = sizeof(W) * (size_t)sc.n_sectors * md.n_group;
+  size_t smem = sizeof(W) * (size_t)sc.n_sectors * md.n_group;
+  if (kWide<PREC, CPL>) smem = pair_table_offset(smem) + sizeof(W) * (size_t)md.n_group * (NC / 2);
   static int blocks_per_sm[16] = {0};  // per device, computed once
   int dev = 0;
   RSED_TRY_CUDA(cudaGetDevice(&dev));
@@ -412,11 +520,11 @@ int launch_spmv(const rsed_model_t& md, const rsed_sectors_t& sc, const void* x,
   const int64_t gx = row_blocks < (int64_t)n_sm * bps ? row_blocks : (int64_t)n_sm * bps;
   if (sequential) {
     for (int c = 0; c < n_chunks; ++c) {
-      kern<<<dim3((unsigned)gx, 1), 256, smem, stream>>>(md, sc, x, y, c);
+      kern<<<dim3((unsigned)gx, 1), 256, smem, stream>>>(md, sc, x, y, c, guard);
       RSED_CHECK_LAUNCH();
     }
   } else {
-    kern<<<dim3((unsigned)gx, (unsigned)n_chunks), 256, smem, stream>>>(md, sc, x, y, 0);
+    kern<<<dim3((unsigned)gx, (unsigned)n_chunks), 256, smem, stream>>>(md, sc, x, y, 0, guard);
     RSED_CHECK_LAUNCH();
   }
   return RSED_OK;
@@ -434,40 +542,8 @@ int check_proj_model(const rsed_model_t* md) {
   return RSED_OK;
 }
 
-}  // namespace
-
-// Called by rsed_apply_h for variants 0 (with a table present), 3NN-6NN.
-int rsed_proj_apply(const rsed_model_t& md, const rsed_sectors_t& sc, const void* x, double2* y, int precision,
-                    int variant, cudaStream_t stream) {
-  RSED_REQUIRE(md.proj_rowptr && md.proj_cg, RSED_EINVAL, "no projection table in the model");
-  RSED_REQUIRE(precision == 64 ? md.proj_w64 != nullptr : md.proj_w32 != nullptr, RSED_EINVAL,
-               "projection table has no weights for precision %d", precision);
-  RSED_REQUIRE((sc.ld & 1) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0, RSED_EINVAL,
-               "projection apply needs an even leading dimension and a 16-byte aligned x");
-  if (variant == 0) {
-    // Measured on B200 (657,756 orbits, 64 columns): FP32 runs best with a
-    // 32-B x segment per lane (4 columns) and one chunk covering up to 64
-    // columns (3.7 ms vs 4.5 ms with 16-B segments; at 32 columns 1.48 ms in
-    // one chunk vs 1.95 ms in chunks of 16 that keep x in L2); FP64 with
-    // 16-B segments and 16-column chunks, one after another (7.5 ms; wider
-    // segments spill into lower occupancy), except at 17-32 columns.  Small (latency-bound) bases prefer up to 16
-    // columns per chunk with all chunks in one launch, for more warps in flight.
-    if (md.n_orbits < 65536) {
-      int nc = 4;
-      while (nc < sc.n_cols && nc < 16) nc *= 2;  // a narrow block keeps every lane of its slots
-      variant = 400 + nc;
-    } else if (precision == 32) {
-      int nc = 8;
-      while (nc < sc.n_cols && nc < 64) nc *= 2;
-      variant = 500 + nc;
-    } else if (sc.n_cols > 16 && sc.n_cols <= 32) {
-      variant = 632;  // 17-32 FP64 columns: 32-B segments, one launch (3.50 vs 3.76 ms at 32 columns)
-    } else {
-      int nc = 2;
-      while (nc < sc.n_cols && nc < 16) nc *= 2;
-      variant = 300 + nc;
-    }
-  }
+int launch_variant(const rsed_model_t& md, const rsed_sectors_t& sc, const void* x, double2* y, int precision,
+                   int variant, int guard, cudaStream_t stream) {
   const int family = variant / 100;  // 3/4: 16-B segment per lane, 5/6: 32-B segment
   const bool seq = family == 3 || family == 5;
   const bool wide = family >= 5;
@@ -476,46 +552,91 @@ int rsed_proj_apply(const rsed_model_t& md, const rsed_sectors_t& sc, const void
     if (precision == 64) {
       if (!wide) {
         switch (nc) {
-          case 2: return launch_spmv<64, 2, 1>(md, sc, x, y, seq, stream);
-          case 4: return launch_spmv<64, 4, 1>(md, sc, x, y, seq, stream);
-          case 8: return launch_spmv<64, 8, 1>(md, sc, x, y, seq, stream);
-          case 16: return launch_spmv<64, 16, 1>(md, sc, x, y, seq, stream);
-          case 32: return launch_spmv<64, 32, 1>(md, sc, x, y, seq, stream);
+          case 2: return launch_spmv<64, 2, 1>(md, sc, x, y, seq, guard, stream);
+          case 4: return launch_spmv<64, 4, 1>(md, sc, x, y, seq, guard, stream);
+          case 8: return launch_spmv<64, 8, 1>(md, sc, x, y, seq, guard, stream);
+          case 16: return launch_spmv<64, 16, 1>(md, sc, x, y, seq, guard, stream);
+          case 32: return launch_spmv<64, 32, 1>(md, sc, x, y, seq, guard, stream);
           default: break;
         }
       } else {
         switch (nc) {
-          case 4: return launch_spmv<64, 2, 2>(md, sc, x, y, seq, stream);
-          case 8: return launch_spmv<64, 4, 2>(md, sc, x, y, seq, stream);
-          case 16: return launch_spmv<64, 8, 2>(md, sc, x, y, seq, stream);
-          case 32: return launch_spmv<64, 16, 2>(md, sc, x, y, seq, stream);
-          case 64: return launch_spmv<64, 32, 2>(md, sc, x, y, seq, stream);
+          case 4: return launch_spmv<64, 2, 2>(md, sc, x, y, seq, guard, stream);
+          case 8: return launch_spmv<64, 4, 2>(md, sc, x, y, seq, guard, stream);
+          case 16: return launch_spmv<64, 8, 2>(md, sc, x, y, seq, guard, stream);
+          case 32: return launch_spmv<64, 16, 2>(md, sc, x, y, seq, guard, stream);
+          case 64: return launch_spmv<64, 32, 2>(md, sc, x, y, seq, guard, stream);
           default: break;
         }
       }
     } else {
       if (!wide) {
         switch (nc) {
-          case 4: return launch_spmv<32, 2, 2>(md, sc, x, y, seq, stream);
-          case 8: return launch_spmv<32, 4, 2>(md, sc, x, y, seq, stream);
-          case 16: return launch_spmv<32, 8, 2>(md, sc, x, y, seq, stream);
-          case 32: return launch_spmv<32, 16, 2>(md, sc, x, y, seq, stream);
-          case 64: return launch_spmv<32, 32, 2>(md, sc, x, y, seq, stream);
+          case 4: return launch_spmv<32, 2, 2>(md, sc, x, y, seq, guard, stream);
+          case 8: return launch_spmv<32, 4, 2>(md, sc, x, y, seq, guard, stream);
+          case 16: return launch_spmv<32, 8, 2>(md, sc, x, y, seq, guard, stream);
+          case 32: return launch_spmv<32, 16, 2>(md, sc, x, y, seq, guard, stream);
+          case 64: return launch_spmv<32, 32, 2>(md, sc, x, y, seq, guard, stream);
           default: break;
         }
       } else {
         switch (nc) {
-          case 8: return launch_spmv<32, 2, 4>(md, sc, x, y, seq, stream);
-          case 16: return launch_spmv<32, 4, 4>(md, sc, x, y, seq, stream);
-          case 32: return launch_spmv<32, 8, 4>(md, sc, x, y, seq, stream);
-          case 64: return launch_spmv<32, 16, 4>(md, sc, x, y, seq, stream);
-          case 128: return launch_spmv<32, 32, 4>(md, sc, x, y, seq, stream);
+          case 8: return launch_spmv<32, 2, 4>(md, sc, x, y, seq, guard, stream);
+          case 16: return launch_spmv<32, 4, 4>(md, sc, x, y, seq, guard, stream);
+          case 32: return launch_spmv<32, 8, 4>(md, sc, x, y, seq, guard, stream);
+          case 64: return launch_spmv<32, 16, 4>(md, sc, x, y, seq, guard, stream);
+          case 128: return launch_spmv<32, 32, 4>(md, sc, x, y, seq, guard, stream);
           default: break;
         }
       }
     }
   }
   return rsed_set_error(RSED_EINVAL, "projection apply variant %d invalid at precision %d", variant, precision);
+}
+
+}  // namespace
+
+// Called by rsed_apply_h for variants 0 (with a table present), 3NN-6NN.
+// pairs: 1 = the caller knows that columns 2i and 2i + 1 share a sector, 0 = it
+// knows that they do not, -1 = unknown.
+int rsed_proj_apply(const rsed_model_t& md, const rsed_sectors_t& sc, const void* x, double2* y, int precision,
+                    int variant, int pairs, cudaStream_t stream) {
+  RSED_REQUIRE(md.proj_rowptr && md.proj_cg, RSED_EINVAL, "no projection table in the model");
+  RSED_REQUIRE(precision == 64 ? md.proj_w64 != nullptr : md.proj_w32 != nullptr, RSED_EINVAL,
+               "projection table has no weights for precision %d", precision);
+  RSED_REQUIRE((sc.ld & 1) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0, RSED_EINVAL,
+               "projection apply needs an even leading dimension and a 16-byte aligned x");
+  if (variant != 0) return launch_variant(md, sc, x, y, precision, variant, 0, stream);
+  // Pairs of columns of one sector run the pair loop on 32-B segments, one launch
+  // of up to 64 columns per chunk (B200, us, against 16-B segments in chunks of 16;
+  // 657,756 orbits: FP64 32 columns 2051 and 3009, 64 columns 4269 and 5931, 8
+  // columns 671 and 838, FP32 32 columns 995 and 1892; 11,240 orbits, 24 columns:
+  // FP64 31 and 40, FP32 22 and 27).  Few columns fill no 32-B segments of enough
+  // lanes, which pays only where the gathers miss L2 (FP64 4 columns: 657,756
+  // orbits 482 and 521, 112,720 orbits 52 and 47; 2 columns: 445 and 330; FP32 4
+  // columns 385 and 367, 8 columns 415 and 580).  Other columns run best on 16-B
+  // segments (16 columns of 16 sectors: FP64 1470 and 1610, FP32 1062 and 1082; 48
+  // columns, FP64 4470 and 6456), as do the smallest bases, which want the warps of
+  // more chunks.  Where the caller does not know, a large basis launches both
+  // forms and the kernel that does not fit the columns leaves at once (4 us: FP64
+  // from 2^21 elements, about 100 us).
+  const int cpl = precision == 64 ? 2 : 4;
+  const bool fits = sc.ld % cpl == 0 && (reinterpret_cast<uintptr_t>(x) & 31) == 0 && sc.n_cols % 2 == 0;
+  const int64_t elems = md.n_orbits * (int64_t)sc.n_cols;
+  const bool small = md.n_orbits < 65536;
+  const bool gains = precision == 32 ? sc.n_cols >= 8 : sc.n_cols > 16 || (sc.n_cols >= 4 && elems >= (1 << 21));
+  int wide = precision == 64 ? 4 : 8;
+  while (wide < sc.n_cols && wide < 64) wide *= 2;
+  wide += 600;
+  int narrow = small || precision == 32 ? 4 : 2;
+  while (narrow < sc.n_cols && narrow < 16) narrow *= 2;
+  narrow += small || precision == 32 ? 400 : 300;
+  if (!fits || !gains || pairs == 0 || md.n_orbits < 2048 ||
+      (pairs < 0 && (small || (precision == 64 && elems < (1 << 21)))))
+    return launch_variant(md, sc, x, y, precision, narrow, 0, stream);
+  const int rc = launch_variant(md, sc, x, y, precision, wide, pairs < 0 ? 1 : 0, stream);
+  if (rc || pairs > 0) return rc;
+  return launch_variant(md, sc, x, y, precision, narrow, 2, stream);
 }
 
 extern "C" size_t rsed_proj_scratch_bytes(int64_t n_orbits) {

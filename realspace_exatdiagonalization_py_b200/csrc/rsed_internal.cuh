@@ -52,4 +52,8 @@ int check_group(const rsed_group_t* g);
 // Streaming apply over the model's projection table (proj.cu); variant 0
 // picks the column chunk, 3NN / 4NN as documented at rsed_apply_h.
 int rsed_proj_apply(const rsed_model_t& md, const rsed_sectors_t& sc, const void* x, double2* y, int precision,
-                    int variant, cudaStream_t stream);
+                    int variant, int pairs, cudaStream_t stream);
+// rsed_apply_h with what the caller knows of the columns: pairs = 1 if columns
+// 2i and 2i + 1 share a sector for every i, 0 if they do not, -1 unknown.
+int rsed_apply_pairs(const rsed_model_t* md, const rsed_sectors_t* sc, const void* x, void* y, int precision,
+                     int variant, int pairs, void* stream);

@@ -281,3 +281,58 @@ def test_density_pairs_sizes(family, size, nf):
     ref = (occ * (np.abs(c) ** 2)[:, None]).T @ occ
     # sums of weights that add up to 1
     np.testing.assert_allclose(cr.density_pairs(basis, c), ref, atol=1e-14, rtol=0)
+
+
+# the projection matvec by how the columns pair up: pairs (blocks of 2 and 4),
+# pairs broken at one place, single columns, odd counts, more columns than one
+# chunk, leading dimensions that do not hold whole segments; bases around the
+# sizes where the default route changes, with orbits outside some sectors and
+# (all sites taken) rows without a hop.  A non-finite value of x reaches the
+# rows that H takes it to and no other.
+@pytest.mark.parametrize("n_site,nf,blocks,ld", [
+    (16, 8, [2] * 3, 6), (16, 16, [2], 2), (20, 10, [2] * 10, 20), (20, 10, [4] * 17, 68), (20, 10, [2, 1, 2, 2], 8),
+    (20, 10, [1] * 5, 6), (24, 12, [2], 2), (24, 12, [2] * 5, 10), (24, 12, [4] * 5, 22), (24, 12, [3] * 3, 10),
+    (24, 12, [2, 1, 1, 4], 8), (24, 12, [2] * 33, 68),
+])
+def test_projection_products(n_site, nf, blocks, ld):
+    import torch
+
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import models
+
+    m = models.build_heisenberg_second_quantized_model(n_site, 1.0)
+    data = ed.build_ed_data(m, filling_fraction=Fraction(nf, n_site),
+                            symmetry_group=ed.build_translation_group(m.lattice))
+    dm, sset = data._device()
+    n = sum(blocks)
+    cs = torch.tensor([i % sset.n_sectors for i, b in enumerate(blocks) for _ in range(b)], dtype=torch.int32,
+                      device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    X = torch.randn(data.orbit_catalog.n_orbits, ld, dtype=torch.complex128, device="cuda", generator=gen)
+    X[:, :n] *= (sset.member[:, None] >> cs[None, :].long()) & 1
+    Xf = X.to(torch.complex64)
+    want, want32 = torch.zeros_like(X), torch.zeros_like(X)
+    dm.apply_block(sset, cs, X, want)  # without a table: on the fly
+    dm.apply_block(sset, cs, Xf, want32, 32)
+    top = max(1.0, want[:, :n].abs().max().item())
+    dm.build_projection(sset.sqrt_stab, precisions=(64, 32))
+    try:
+        Xn = X.clone()
+        Xn[0, 0] = complex("nan")
+        Yn = torch.zeros_like(X)
+        dm.apply_block(sset, cs, Xn, Yn, 64, 302)
+        reached = torch.isnan(Yn[:, :n].real)
+        for v in (0, 604, 616, 664):
+            Y = torch.zeros_like(X)
+            dm.apply_block(sset, cs, X, Y, 64, v)
+            # the same products in another order: a few ulps of sums of up to 24 hops
+            assert (Y[:, :n] - want[:, :n]).abs().max().item() < 1e-13 * top, v
+            assert not Y[:, n:].any()
+            dm.apply_block(sset, cs, Xn, Y, 64, v)
+            assert torch.equal(torch.isnan(Y[:, :n].real), reached), v
+        for v in (0, 408, 608, 632, 664):
+            Y = torch.zeros_like(X)
+            dm.apply_block(sset, cs, Xf, Y, 32, v)
+            assert (Y[:, :n] - want32[:, :n]).abs().max().item() < 2e-6 * top, v
+    finally:
+        dm.drop_projection()
