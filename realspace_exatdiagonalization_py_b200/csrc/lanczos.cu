@@ -1542,13 +1542,17 @@ __global__ void __launch_bounds__(kSThreads, 2)
 // (full row-major storage, destroyed), one thread block:
 //   1. Householder reduction to a real symmetric tridiagonal T = Q^H A Q
 //      (lower variant of LAPACK zhetd2: reflectors H_k = I - tau_k v v^H
-//      chosen so the sub-diagonal comes out real), ~5 block barriers per column;
-//   2. eigenvalues of T by Sturm-sequence bisection, one thread per eigenvalue;
+//      chosen so the sub-diagonal comes out real), two block barriers per column;
+//   2. eigenvalues of T by Sturm-sequence bisection, 16 threads per eigenvalue;
 //   3. eigenvectors of T by inverse iteration (tridiagonal LU with partial
 //      pivoting, three solves), one thread per eigenvector, then modified
 //      Gram-Schmidt in ascending order (orthonormal bases of degenerate
 //      clusters);
-//   4. back-transformation s = H_0 H_1 ... H_{M-2} z, one warp per vector.
+//   4. back-transformation s = H_0 H_1 ... H_{M-2} z, 16 lanes per vector.
+// All four are serial chains (8 cycles an FMA, 35 an exchange and add, 140 a
+// division), so each keeps its chain in registers.  64 rows, 16 eigenvectors,
+// one instance, us: the matrix in shared memory 330 (140, 70, 72 with the
+// Gram-Schmidt, 45), as here 198 (102, 34, 38, 21).
 __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
@@ -1565,62 +1569,161 @@ __device__ __forceinline__ double warp_sum(double v) {
 // leaves [2^-400, 2^400].  A minor that vanishes against its predecessor,
 // |p_i| < piv |p_{i-1}|, becomes -piv p_{i-1} (the pivmin rule of the ratio
 // form).  piv >= 2^-500 keeps piv |p_{i-1}| a normal number.
+// The chain of dependent operations bounds it, so eight steps run on the FMA
+// alone and integer tests on the high words count the sign changes and ask
+// whether a minor fell below the range or vanished (above it none can get from
+// inside within eight steps of at most a factor 4); if one did, the eight are
+// taken again with the tests after each step (64 rows, 16 eigenvalues: 70 us of
+// tests after each step, 34 us as here, for all counts of one problem).
 __device__ int sturm_count(const double2* de, int M, double x, double piv) {
   double pm = de[0].x - x;  // p_0
   if (fabs(pm) < piv) pm = -piv;
   int c = pm < 0.0;
   double pmm = 1.0;  // p_{-1}
-  for (int i = 1; i < M; ++i) {
-    const double2 v = de[i];
-    const double t = de[i - 1].y * pmm;
-    double p = fma(v.x - x, pm, -t);
-    if (fabs(p) < piv * fabs(pm)) p = -piv * pm;
-    c += (p < 0.0) != (pm < 0.0);
-    pmm = pm;
-    pm = p;
-    if (!(fabs(pm) <= 0x1p400 && fabs(pm) >= 0x1p-400)) {
-      int ex;
-      frexp(pm, &ex);
-      pm = ldexp(pm, -ex);
-      pmm = ldexp(pmm, -ex);
+  constexpr unsigned kLow = (1023u - 400u) << 21, kHigh = (1023u + 400u) << 21;  // high words without the sign
+  int i = 1;
+  while (i < M) {
+    const unsigned h0 = (unsigned)__double2hiint(pm);
+    if (i + 8 <= M && h0 << 1 >= kLow && h0 << 1 < kHigh) {
+      double2 v[9];
+#pragma unroll
+      for (int u = 0; u < 9; ++u) v[u] = de[i - 1 + u];
+      double p1 = pm, p0 = pmm;
+      unsigned signs = h0 >> 31, least = ~0u;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const double p = fma(v[u + 1].x - x, p1, -(v[u].y * p0));
+        const unsigned h = (unsigned)__double2hiint(p);
+        signs = __funnelshift_l(h, signs, 1);
+        least = min(least, h << 1);
+        p0 = p1;
+        p1 = p;
+      }
+      if (least >= kLow) {
+        c += __popc((signs ^ (signs >> 1)) & 0xffu);
+        pmm = p0;
+        pm = p1;
+        i += 8;
+        continue;
+      }
+    }
+    for (const int end = min(i + 8, M); i < end; ++i) {
+      const double2 v = de[i];
+      const double t = de[i - 1].y * pmm;
+      double p = fma(v.x - x, pm, -t);
+      if (fabs(p) < piv * fabs(pm)) p = -piv * pm;
+      c += (p < 0.0) != (pm < 0.0);
+      pmm = pm;
+      pm = p;
+      if (!(fabs(pm) <= 0x1p400 && fabs(pm) >= 0x1p-400)) {
+        int ex;
+        frexp(pm, &ex);
+        pm = ldexp(pm, -ex);
+        pmm = ldexp(pmm, -ex);
+      }
     }
   }
   return c;
 }
 
-// Householder reflector of column c (rows c+1..M-1) by one warp: v (v[c+1] =
-// 1) into A's column c and into vb, tau[c], the off-diagonal ee[c].
-__device__ __forceinline__ void herm_reflector(double2* A, int lda, int M, int c, double2* vb, double2* tau,
-                                               double* ee, int lane) {
+// Householder reflector of a column whose entries c[h] (row lane + 32 h, zero
+// outside rows col+1 .. M-1) one warp holds: v (v[col+1] = 1) into vb and below
+// the diagonal of A's column col, tau[col], the off-diagonal ee[col].
+__device__ __forceinline__ void herm_reflector(const double2 (&c)[2], double2* A, int lda, int M, int col, double2* vb,
+                                               double2* tau, double* ee, int lane) {
+  const int f = col + 1;  // row of the pivot
+  double2 al;
+  al.x = __shfl_sync(0xffffffffu, f < 32 ? c[0].x : c[1].x, f & 31);
+  al.y = __shfl_sync(0xffffffffu, f < 32 ? c[0].y : c[1].y, f & 31);
   double sq = 0.0;
-  for (int i = c + 2 + lane; i < M; i += 32) {
-    const double2 v = A[i * lda + c];
-    sq += v.x * v.x + v.y * v.y;
-  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    if (lane + 32 * h > f) sq += c[h].x * c[h].x + c[h].y * c[h].y;
   sq = warp_sum(sq);
-  const double2 al = A[(c + 1) * lda + c];
   double2 t = make_double2(0.0, 0.0), scl = make_double2(0.0, 0.0);
   double beta = al.x;
   if (sq != 0.0 || al.y != 0.0) {
     beta = -copysign(sqrt(al.x * al.x + al.y * al.y + sq), al.x);
-    const double ib = 1.0 / beta;
-    t = make_double2((beta - al.x) * ib, -al.y * ib);
     const double2 den = make_double2(al.x - beta, al.y);
-    const double idn = 1.0 / (den.x * den.x + den.y * den.y);
+    const double rec = 1.0 / (lane & 1 ? den.x * den.x + den.y * den.y : beta);  // both divisions at once
+    const double ib = __shfl_sync(0xffffffffu, rec, 0), idn = __shfl_sync(0xffffffffu, rec, 1);
+    t = make_double2((beta - al.x) * ib, -al.y * ib);
     scl = make_double2(den.x * idn, -den.y * idn);
   }
-  for (int i = c + 2 + lane; i < M; i += 32) {
-    const double2 v = cmul(A[i * lda + c], scl);
-    A[i * lda + c] = v;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = lane + 32 * h;
+    double2 v = cmul(c[h], scl);
+    if (i == f) v = make_double2(1.0, 0.0);
+    if (i < f) v = make_double2(0.0, 0.0);
     vb[i] = v;
+    if (i >= f && i < M) A[i * lda + col] = v;
   }
   if (lane == 0) {
-    vb[c + 1] = make_double2(1.0, 0.0);
-    A[(c + 1) * lda + c] = make_double2(1.0, 0.0);
-    tau[c] = t;
-    ee[c] = beta;
+    tau[col] = t;
+    ee[col] = beta;
   }
-  __syncwarp();
+}
+
+// One thread's part of a tridiagonalisation step on columns k+1.. (blocks LO ..
+// HI-1 of 16): the rank-2 update of the step before (if there was one), column
+// k+1 into cv, and this step's q = A v into pw.
+constexpr int kNA = kJacobiMax / 16;
+template <int LO, int HI>
+__device__ __forceinline__ void herm_step(double2 (&a)[kNA][kNA], int k, int ty, int tx, const double2* vo,
+                                          const double2* wv, const double2* v, double2* cv, double2* pw) {
+  constexpr int N = HI - LO;
+  if (k > 0) {
+    double2 vj[N], wj[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      vj[q] = vo[tx + 16 * (LO + q)];
+      wj[q] = wv[tx + 16 * (LO + q)];
+    }
+#pragma unroll
+    for (int p = 0; p < N; ++p) {
+      const double2 vi = vo[ty + 16 * (LO + p)], wi = wv[ty + 16 * (LO + p)];
+#pragma unroll
+      for (int q = 0; q < N; ++q) {  // a -= v w^H + w v^H
+        double2& e = a[LO + p][LO + q];
+        e.x -= vi.x * wj[q].x + vi.y * wj[q].y + wi.x * vj[q].x + wi.y * vj[q].y;
+        e.y -= vi.y * wj[q].x - vi.x * wj[q].y + wi.y * vj[q].x - wi.x * vj[q].y;
+      }
+    }
+  }
+  if (tx == ((k + 1) & 15)) {
+#pragma unroll
+    for (int p = LO; p < HI; ++p) cv[ty + 16 * p] = a[p][LO];
+  }
+  double2 s[kNA];
+#pragma unroll
+  for (int p = 0; p < kNA; ++p) s[p] = make_double2(0.0, 0.0);
+#pragma unroll
+  for (int q = LO; q < HI; ++q) {
+    const double2 vj = v[tx + 16 * q];
+#pragma unroll
+    for (int p = LO; p < HI; ++p) {
+      s[p].x += a[p][q].x * vj.x - a[p][q].y * vj.y;
+      s[p].y += a[p][q].x * vj.y + a[p][q].y * vj.x;
+    }
+  }
+  // sums over the 16 threads of a row: halve the rows twice, then exchange
+  const bool u8 = tx & 8, u4 = tx & 4;
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    const double2 l = s[p], h = s[p + 2];
+    s[p].x = (u8 ? h.x : l.x) + __shfl_xor_sync(0xffffffffu, u8 ? l.x : h.x, 8);
+    s[p].y = (u8 ? h.y : l.y) + __shfl_xor_sync(0xffffffffu, u8 ? l.y : h.y, 8);
+  }
+  double2 r;
+  r.x = (u4 ? s[1].x : s[0].x) + __shfl_xor_sync(0xffffffffu, u4 ? s[0].x : s[1].x, 4);
+  r.y = (u4 ? s[1].y : s[0].y) + __shfl_xor_sync(0xffffffffu, u4 ? s[0].y : s[1].y, 4);
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1) {
+    r.x += __shfl_xor_sync(0xffffffffu, r.x, o);
+    r.y += __shfl_xor_sync(0xffffffffu, r.y, o);
+  }
+  if ((tx & 3) == 0) pw[ty + 16 * ((u8 ? 2 : 0) + (u4 ? 1 : 0))] = r;
 }
 
 // iwork: optional shared-memory work area of kHermWork bytes for the inverse
@@ -1632,87 +1735,101 @@ __device__ void herm_lowest(double2* A, int M, int Kp, double* theta, double2* S
   const int tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
   // ---- 1. tridiagonalisation: two barriers per column ----
-  // Warp 0 updates column k+1 itself during step k's rank-2 update and forms
-  // the next reflector at once (look-ahead), while the other warps update the
-  // rest of the trailing matrix; the reflector vectors alternate between two
-  // buffers (vv and the still unused S), so the next one never overwrites the
-  // one being applied.  p^H v is formed redundantly by every warp.
-  double2* vbuf[2] = {vv, S};
-  if (M >= 2 && warp == 0) herm_reflector(A, lda, M, 0, vbuf[0], tau, ee, lane);
-  __syncthreads();
-  for (int k = 0; k < M - 1; ++k) {
-    const double2* v = vbuf[k & 1];
-    const double2 t = tau[k];
-    const bool next = k + 1 < M - 1;
-    if (t.x == 0.0 && t.y == 0.0) {  // H_k = I: nothing to update
-      if (next && warp == 0) herm_reflector(A, lda, M, k + 1, vbuf[(k + 1) & 1], tau, ee, lane);
-      __syncthreads();
-      continue;
-    }
-    // p = tau * A22 v, four lanes per row
-    {
-      const int i = k + 1 + (tid >> 2), sub = tid & 3;
-      double sx = 0.0, sy = 0.0;
-      if (i < M) {
-        const double2* Ar = A + i * lda;
-        for (int j = k + 1 + sub; j < M; j += 4) {
-          const double2 a = Ar[j], vj = v[j];
-          sx += a.x * vj.x - a.y * vj.y;
-          sy += a.x * vj.y + a.y * vj.x;
-        }
+  // The matrix lives in the registers of a 16 x 16 grid of threads, entry (i, j)
+  // in thread (i % 16, j % 16), so that a step reads only vectors from shared
+  // memory.  Step k applies the rank-2 update of step k-1, hands column k+1 out
+  // and multiplies by v_k; then warp 0 alone, two rows a lane, forms w, the
+  // updated column k+1 and its reflector, while the others wait: the chain of
+  // its two sums, square root and divisions is what a step takes.
+  {
+    double2* const wv = S;
+    double2* const cv = S + kJacobiMax;
+    double2* const vbuf[2] = {vv, S + 2 * kJacobiMax};
+    constexpr int NA = kNA;
+    const int ty = (tid >> 4) & 15, tx = tid & 15;
+    double2 a[NA][NA];
+#pragma unroll
+    for (int p = 0; p < NA; ++p)
+#pragma unroll
+      for (int q = 0; q < NA; ++q) {
+        const int i = ty + 16 * p, j = tx + 16 * q;
+        a[p][q] = tid < 256 && i < M && j < M ? A[i * lda + j] : make_double2(0.0, 0.0);
       }
-      sx += __shfl_xor_sync(0xffffffffu, sx, 1);
-      sy += __shfl_xor_sync(0xffffffffu, sy, 1);
-      sx += __shfl_xor_sync(0xffffffffu, sx, 2);
-      sy += __shfl_xor_sync(0xffffffffu, sy, 2);
-      if (i < M && sub == 0) pw[i] = cmul(t, make_double2(sx, sy));
-    }
     __syncthreads();
-    // p^H v in every warp; alpha = -1/2 tau (p^H v); w = p + alpha v
-    double2 alpha;
-    {
-      double sx = 0.0, sy = 0.0;
-      for (int i = k + 1 + lane; i < M; i += 32) {
-        const double2 c = cdotc(pw[i], v[i]);
-        sx += c.x;
-        sy += c.y;
-      }
-      const double2 ta = cmul(t, make_double2(warp_sum(sx), warp_sum(sy)));
-      alpha = make_double2(-0.5 * ta.x, -0.5 * ta.y);
-    }
-    // A22 -= v w^H + w v^H: column k+1 by warp 0 (then the next reflector),
-    // columns k+2.. of every row by the other warps (all warps if there is one)
-    const int c1 = k + 1;
-    const double2 v1 = v[c1];
-    const double2 w1 = cadd(pw[c1], cmul(alpha, v1));
     if (warp == 0) {
-      for (int i = c1 + lane; i < M; i += 32) {
-        const double2 vi = v[i];
-        const double2 wi = cadd(pw[i], cmul(alpha, vi));
-        const double2 u = cadd(make_double2(vi.x * w1.x + vi.y * w1.y, vi.y * w1.x - vi.x * w1.y),
-                               make_double2(wi.x * v1.x + wi.y * v1.y, wi.y * v1.x - wi.x * v1.y));
-        A[i * lda + c1] = csub(A[i * lda + c1], u);
+      double2 c0[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = lane + 32 * h;
+        c0[h] = i >= 1 && i < M ? A[i * lda] : make_double2(0.0, 0.0);
       }
-      __syncwarp();
-      if (next) herm_reflector(A, lda, M, c1, vbuf[c1 & 1], tau, ee, lane);
-    }
-    const int w0 = nwarp > 1 ? 1 : 0, nw = nwarp > 1 ? nwarp - 1 : 1;
-    if (warp >= w0) {
-      for (int i = c1 + (warp - w0); i < M; i += nw) {
-        const double2 vi = v[i];
-        const double2 wi = cadd(pw[i], cmul(alpha, vi));
-        for (int j = c1 + 1 + lane; j < M; j += 32) {
-          const double2 vj = v[j];
-          const double2 wj = cadd(pw[j], cmul(alpha, vj));
-          const double2 u = cadd(make_double2(vi.x * wj.x + vi.y * wj.y, vi.y * wj.x - vi.x * wj.y),
-                                 make_double2(wi.x * vj.x + wi.y * vj.y, wi.y * vj.x - wi.x * vj.y));
-          A[i * lda + j] = csub(A[i * lda + j], u);
-        }
-      }
+      if (lane == 0) dd[0] = A[0].x;
+      if (M >= 2) herm_reflector(c0, A, lda, M, 0, vbuf[0], tau, ee, lane);
     }
     __syncthreads();
+    const int hi = (M + 15) >> 4;  // blocks of 16 rows or columns
+    for (int k = 0; k < M - 1; ++k) {
+      const double2* v = vbuf[k & 1];
+      const double2* vo = vbuf[(k + 1) & 1];  // of step k-1
+      if (tid < 256) {
+        // rows and columns k+1 .. M-1 are alive, in blocks (k+1)/16 .. (M-1)/16
+#define RSED_HERM(LO, HI) herm_step<LO, HI>(a, k, ty, tx, vo, wv, v, cv, pw); break
+        switch ((k + 1) >> 4 | hi << 2) {
+          case 0 | 1 << 2: RSED_HERM(0, 1);
+          case 0 | 2 << 2: RSED_HERM(0, 2);
+          case 1 | 2 << 2: RSED_HERM(1, 2);
+          case 0 | 3 << 2: RSED_HERM(0, 3);
+          case 1 | 3 << 2: RSED_HERM(1, 3);
+          case 2 | 3 << 2: RSED_HERM(2, 3);
+          case 0 | 4 << 2: RSED_HERM(0, 4);
+          case 1 | 4 << 2: RSED_HERM(1, 4);
+          case 2 | 4 << 2: RSED_HERM(2, 4);
+          default: RSED_HERM(3, 4);
+        }
+#undef RSED_HERM
+      }
+      __syncthreads();
+      if (warp == 0) {
+        // w = tau q - 1/2 |tau|^2 (v^H q) v with v^H q = v^H A v real, and column
+        // k+1 of A - v w^H - w v^H (v[k+1] = 1)
+        const double2 t = tau[k];
+        double2 w[2], c[2], vl[2];
+        double sum = 0.0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int i = lane + 32 * h;
+          const bool in = i > k && i < M;
+          vl[h] = in ? v[i] : make_double2(0.0, 0.0);
+          w[h] = in ? pw[i] : make_double2(0.0, 0.0);
+          c[h] = in ? cv[i] : make_double2(0.0, 0.0);
+          sum += vl[h].x * w[h].x + vl[h].y * w[h].y;
+        }
+        const double alpha = -0.5 * (t.x * t.x + t.y * t.y) * warp_sum(sum);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          w[h] = cmul(t, w[h]);
+          w[h].x += alpha * vl[h].x;
+          w[h].y += alpha * vl[h].y;
+        }
+        const int f = k + 1;
+        const double w1x = __shfl_sync(0xffffffffu, f < 32 ? w[0].x : w[1].x, f & 31);
+        const double w1y = __shfl_sync(0xffffffffu, f < 32 ? w[0].y : w[1].y, f & 31);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int i = lane + 32 * h;
+          wv[i] = w[h];
+          c[h].x -= vl[h].x * w1x + vl[h].y * w1y + w[h].x;
+          c[h].y -= vl[h].y * w1x - vl[h].x * w1y + w[h].y;
+          if (i == f) {
+            dd[f] = c[h].x;
+            c[h] = make_double2(0.0, 0.0);
+          }
+        }
+        if (f < M - 1) herm_reflector(c, A, lda, M, f, vbuf[f & 1], tau, ee, lane);
+      }
+      __syncthreads();
+    }
   }
-  for (int k = tid; k < M; k += nt) dd[k] = A[k * lda + k].x;
   if (tid == 0 && M >= 1) ee[M - 1] = 0.0;
   __syncthreads();
   // ---- 2. eigenvalues: 16-way multisection, 16 threads per eigenvalue ----
@@ -1768,7 +1885,7 @@ __device__ void herm_lowest(double2* A, int M, int Kp, double* theta, double2* S
     // j at i * Kp + j (the Kp threads touch consecutive words), else local
     double ldl[kJacobiMax], ldg[kJacobiMax], ldu[kJacobiMax], ldu2[kJacobiMax], lz[kJacobiMax];
     unsigned char lpiv[kJacobiMax];
-    const int sw = iwork ? Kp : 1;
+    const int ws = iwork ? Kp : 1;
     const int mk = kJacobiMax * kKeepMax;
     double* dlp = iwork ? iwork + j : ldl;
     double* dgp = iwork ? iwork + mk + j : ldg;
@@ -1776,68 +1893,88 @@ __device__ void herm_lowest(double2* A, int M, int Kp, double* theta, double2* S
     double* du2p = iwork ? iwork + 3 * mk + j : ldu2;
     double* zp = iwork ? iwork + 4 * mk + j : lz;
     unsigned char* pivp = iwork ? reinterpret_cast<unsigned char*>(iwork + 5 * mk) + j : lpiv;
-#define dl(i) dlp[(i) * sw]
-#define dg(i) dgp[(i) * sw]
-#define du(i) dup[(i) * sw]
-#define du2(i) du2p[(i) * sw]
-#define z(i) zp[(i) * sw]
-#define piv(i) pivp[(i) * sw]
-    for (int i = 0; i < M; ++i) {
-      dg(i) = dd[i] - lam;
-      dl(i) = (i < M - 1) ? ee[i] : 0.0;
-      du(i) = (i < M - 1) ? ee[i] : 0.0;
-      du2(i) = 0.0;
-    }
+#define dl(i) dlp[(i) * ws]
+#define dg(i) dgp[(i) * ws]
+#define du(i) dup[(i) * ws]
+#define du2(i) du2p[(i) * ws]
+#define z(i) zp[(i) * ws]
+#define piv(i) pivp[(i) * ws]
+    // The chains of the factorisation and of the solves stay in registers: the
+    // arrays are written behind them and read ahead of them.
     const double tiny = 1e-15 * fmax(tnorm, 1e-300);
-    for (int i = 0; i < M - 1; ++i) {
-      if (fabs(dg(i)) >= fabs(dl(i))) {
-        piv(i) = 0;
-        if (dg(i) == 0.0) dg(i) = tiny;
-        const double f = dl(i) / dg(i);
+    {
+      double d0 = dd[0] - lam, u0 = M > 1 ? ee[0] : 0.0;  // row i as the steps before left it
+      for (int i = 0; i < M - 1; ++i) {
+        const double l = ee[i], d1 = dd[i + 1] - lam, u1 = i < M - 2 ? ee[i + 1] : 0.0;
+        const bool swap = !(fabs(d0) >= fabs(l));  // row i+1 has the larger pivot
+        if (d0 == 0.0) d0 = tiny;
+        const double pv = swap ? l : d0, pu = swap ? d1 : u0, pu2 = swap ? u1 : 0.0;
+        const double r = 1.0 / pv, f = (swap ? d0 : l) * r;
+        piv(i) = swap;
         dl(i) = f;
-        dg(i + 1) -= f * du(i);
-      } else {
-        piv(i) = 1;
-        const double f = dg(i) / dl(i);
-        dg(i) = dl(i);
-        dl(i) = f;
-        const double tmp = du(i);
-        du(i) = dg(i + 1);
-        dg(i + 1) = tmp - f * dg(i + 1);
-        if (i < M - 2) {
-          du2(i) = du(i + 1);
-          du(i + 1) = -f * du(i + 1);
-        }
+        dg(i) = r;  // reciprocal pivots, and the rows above scaled by them
+        du(i) = pu * r;
+        du2(i) = pu2 * r;
+        d0 = (swap ? u0 : d1) - f * pu;
+        u0 = swap ? -f * u1 : u1;
       }
+      if (d0 == 0.0) d0 = tiny;
+      dg(M - 1) = 1.0 / d0;
     }
-    if (dg(M - 1) == 0.0) dg(M - 1) = tiny;
-    for (int i = 0; i < M; ++i) dg(i) = 1.0 / dg(i);  // reciprocal pivots: the solves multiply
     unsigned h = 2166136261u ^ (unsigned)(j * 16777619u);
     for (int i = 0; i < M; ++i) {
       h = h * 1664525u + 1013904223u;
       z(i) = ((h >> 8) * (1.0 / 16777216.0)) - 0.5;
     }
+    double inv = 1.0;
     for (int rep = 0; rep < 3; ++rep) {
-      for (int i = 0; i < M - 1; ++i) {
-        if (piv(i) == 0) {
-          z(i + 1) -= dl(i) * z(i);
-        } else {
-          const double tmp = z(i);
-          z(i) = z(i + 1);
-          z(i + 1) = tmp - dl(i) * z(i);
+      double zc = z(0) * inv;
+      for (int i0 = 0; i0 < M - 1; i0 += 8) {  // eight rows' loads before their stores
+        double zn[8], l[8], g[8];
+        bool sw[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int i = min(i0 + u, M - 2);
+          zn[u] = z(i + 1) * inv;
+          l[u] = dl(i);
+          g[u] = dg(i);
+          sw[u] = piv(i);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (i0 + u >= M - 1) break;
+          const double top = sw[u] ? zn[u] : zc;
+          zc = (sw[u] ? zc : zn[u]) - l[u] * top;
+          z(i0 + u) = top * g[u];
         }
       }
-      z(M - 1) *= dg(M - 1);
-      if (M > 1) z(M - 2) = (z(M - 2) - du(M - 2) * z(M - 1)) * dg(M - 2);
-      for (int i = M - 3; i >= 0; --i) z(i) = (z(i) - du(i) * z(i + 1) - du2(i) * z(i + 2)) * dg(i);
-      double nrm = 0.0;
-      for (int i = 0; i < M; ++i) nrm = fmax(nrm, fabs(z(i)));
-      const double inv = nrm > 0.0 ? 1.0 / nrm : 1.0;
-      for (int i = 0; i < M; ++i) z(i) *= inv;
+      double z1 = zc * dg(M - 1), z2 = 0.0, nrm = fabs(z1);
+      z(M - 1) = z1;
+      for (int i0 = M - 2; i0 >= 0; i0 -= 8) {
+        double zr[8], u1[8], u2[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int i = max(i0 - u, 0);
+          zr[u] = z(i);
+          u1[u] = du(i);
+          u2[u] = du2(i);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (i0 - u < 0) break;
+          const double zi = fma(-u1[u], z1, zr[u] - u2[u] * z2);
+          z(i0 - u) = zi;
+          z2 = z1;
+          z1 = zi;
+          nrm = fmax(nrm, fabs(zi));
+        }
+      }
+      inv = nrm > 0.0 ? 1.0 / nrm : 1.0;
     }
+    for (int i = 0; i < M; ++i) z(i) *= inv;
     double n2 = 0.0;
     for (int i = 0; i < M; ++i) n2 += z(i) * z(i);
-    const double inv = 1.0 / sqrt(n2);
+    inv = 1.0 / sqrt(n2);
     for (int i = 0; i < M; ++i) Z[i * Kp + j] = z(i) * inv;
 #undef dl
 #undef dg
@@ -1885,67 +2022,43 @@ __device__ void herm_lowest(double2* A, int M, int Kp, double* theta, double2* S
     __syncthreads();
   }
   // ---- 4. back-transformation: S = H_0 H_1 ... H_{M-2} Z ----
-  // Reflectors in blocks of nbw, the last block first.  A block's product is
-  // H_k0 ... H_k1-1 = I - V T V^H with T^-1 = diag(1/tau) + strict_upper(V^H V)
-  // (the "UT transform" of compact WY), so S <- S - V T (V^H S) needs only the
-  // block's Gram matrix G = V^H V: Y = V^H S, then T Y by back-substitution,
-  // Y'_c = tau_c (Y_c - sum_{b > c} G_cb Y'_b) (tau_c = 0 gives 0, as it must),
-  // then S -= V Y'.  G and Y live in Z's space (kJacobiMax x kKeepMax doubles
-  // in every caller), free once S holds Z; nbw is the largest block (<= 16)
-  // that fits there.
-  for (int i = tid; i < M * Kp; i += nt) S[i] = make_double2(Z[i], 0.0);
-  __syncthreads();
-  int nbw = 16;
-  while (nbw > 1 && 2 * nbw * (nbw + Kp) > kJacobiMax * kKeepMax) --nbw;
-  double2* Gv = reinterpret_cast<double2*>(Z);  // nbw x nbw, strict upper part
-  double2* Yv = Gv + nbw * nbw;                 // nbw x Kp
-  for (int k1 = M - 1; k1 > 0; k1 -= nbw) {     // reflectors k0 .. k1-1
-    const int k0 = max(0, k1 - nbw);
-    const int nb = k1 - k0;
-    // v_c (reflector k = k0 + c) at row r: 0 for r <= k, 1 at r = k + 1, A[r][k] below.
-    // One thread per output entry, a serial dot over the rows: G[a][c] =
-    // v_a^H v_c (a < c) for the first nb*nb entries, Y[c][j] = v_c^H s_j after
-    for (int e = tid; e < nb * nb + nb * Kp; e += nt) {
-      double2 acc = make_double2(0.0, 0.0);
-      if (e < nb * nb) {
-        const int ga = e / nb, gc = e % nb;
-        if (ga >= gc) continue;
-        const int ka = k0 + ga, kc = k0 + gc;
-        acc = cconj(A[(kc + 1) * lda + ka]);  // v_c's unit entry; v_a there and below is A[r][ka]
-        for (int r = kc + 2; r < M; ++r) acc = cadd(acc, cdotc(A[r * lda + ka], A[r * lda + kc]));
-        Gv[ga * nbw + gc] = acc;
-      } else {
-        const int f = e - nb * nb;
-        const int c = f / Kp, j = f % Kp;
-        const int k = k0 + c;
-        acc = S[(k + 1) * Kp + j];
-        for (int r = k + 2; r < M; ++r) acc = cadd(acc, cdotc(A[r * lda + k], S[r * Kp + j]));
-        Yv[f] = acc;
+  // 16 lanes per vector, its rows sub + 16 q in registers, one reflector after
+  // the other without barriers.  v is zero above its unit entry.
+  {
+    const int j = tid >> 4, sub = tid & 15;
+    constexpr int NA = kJacobiMax / 16;
+    double2 s[NA];
+#pragma unroll
+    for (int q = 0; q < NA; ++q) {
+      const int r = sub + 16 * q;
+      s[q] = make_double2(j < Kp && r < M ? Z[r * Kp + j] : 0.0, 0.0);
+    }
+    __syncwarp();
+    if ((tid & ~31) < Kp * 16) {  // the same for every lane of a warp
+      for (int k = M - 2; k >= 0; --k) {
+        double2 v[NA], y = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int q = 0; q < NA; ++q) {
+          const int r = sub + 16 * q;
+          v[q] = r > k && r < M ? A[r * lda + k] : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int q = 0; q < NA; ++q) y = cadd(y, cdotc(v[q], s[q]));
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+          y.x += __shfl_xor_sync(0xffffffffu, y.x, o);
+          y.y += __shfl_xor_sync(0xffffffffu, y.y, o);
+        }
+        y = cmul(tau[k], y);
+#pragma unroll
+        for (int q = 0; q < NA; ++q) s[q] = csub(s[q], cmul(v[q], y));
       }
     }
-    __syncthreads();
-    // Y <- T Y by back-substitution, one thread per column j (rows descending)
-    for (int j = tid; j < Kp; j += nt) {
-      for (int c = nb - 1; c >= 0; --c) {
-        double2 acc = Yv[c * Kp + j];
-        for (int bb = c + 1; bb < nb; ++bb) acc = csub(acc, cmul(Gv[c * nbw + bb], Yv[bb * Kp + j]));
-        Yv[c * Kp + j] = cmul(tau[k0 + c], acc);
-      }
+#pragma unroll
+    for (int q = 0; q < NA; ++q) {
+      const int r = sub + 16 * q;
+      if (j < Kp && r < M) S[r * Kp + j] = s[q];
     }
-    __syncthreads();
-    // S -= V Y on rows k0+1 .. M-1
-    for (int e = tid; e < (M - k0 - 1) * Kp; e += nt) {
-      const int r = k0 + 1 + e / Kp, j = e % Kp;
-      double2 acc = make_double2(0.0, 0.0);
-      for (int c = 0; c < nb; ++c) {
-        const int k = k0 + c;
-        if (r <= k) break;
-        const double2 vr = (r == k + 1) ? make_double2(1.0, 0.0) : A[r * lda + k];
-        acc = cadd(acc, cmul(vr, Yv[c * Kp + j]));
-      }
-      S[r * Kp + j] = csub(S[r * Kp + j], acc);
-    }
-    __syncthreads();
   }
   __syncthreads();
 }

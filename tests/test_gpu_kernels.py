@@ -336,3 +336,71 @@ def test_projection_products(n_site, nf, blocks, ld):
             assert (Y[:, :n] - want32[:, :n]).abs().max().item() < 2e-6 * top, v
     finally:
         dm.drop_projection()
+
+
+# the projected eigenproblem at the edges of its 16-row blocks, with clusters,
+# exact degeneracies, zero rows (no reflector), decoupled parts and scales at
+# which the Sturm minors leave their range.  The matrix is planted in P; a step
+# on a basis of zeros but for its last block leaves all but the last block's
+# column of it, and the eigen-solve of the full basis follows (no restart: none
+# is allowed)
+@pytest.mark.parametrize("block,slots,kind", [
+    (1, 4, "random"), (1, 15, "random"), (1, 16, "random"), (1, 17, "graded"), (1, 33, "degenerate"),
+    (2, 16, "random"), (2, 24, "large"), (2, 24, "small"), (2, 32, "random"), (3, 11, "degenerate"), (3, 16, "random"),
+    (4, 12, "decoupled"), (4, 16, "random"), (4, 16, "diagonal"), (4, 16, "degenerate"), (4, 16, "graded"),
+])
+def test_projected_eigenproblem(block, slots, kind):
+    import torch
+
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import _lib, models
+    from realspace_exatdiagonalization_py_b200.lanczos import S_NB, S_STATUS, LanczosBatch
+
+    m = models.build_heisenberg_second_quantized_model(16, 1.0)
+    data = ed.build_ed_data(m, filling_fraction=Fraction(1, 2), symmetry_group=ed.build_translation_group(m.lattice))
+    dm, sset = data._device()
+    b = LanczosBatch(dm, sset, [0, 1], 2, ed.LanczosParams(block=block, n_slots=slots, tol=0.0, max_restarts=0))
+    b.load_start(None)
+    b.start()
+    M = slots * block
+    rng = np.random.default_rng(M)
+    P = torch.zeros_like(b.P)
+    for i in range(2):
+        A = rng.standard_normal((M, M)) + 1j * rng.standard_normal((M, M))
+        if kind == "diagonal":
+            A = np.diag(rng.standard_normal(M))
+        elif kind == "degenerate":
+            q, _ = np.linalg.qr(A)
+            A = (q * np.repeat(np.arange((M + 3) // 4) - 5.0, 4)[:M]) @ q.conj().T
+        elif kind == "graded":
+            s = 10.0 ** -np.linspace(0, 12, M)
+            A = A * s[:, None] * s[None, :]
+        elif kind == "decoupled":
+            A[: M // 2, M // 2:] = 0
+            A[M // 2:, : M // 2] = 0
+        elif kind in ("large", "small"):
+            A = A * (1e60 if kind == "large" else 1e-60)
+        P[i, :M, :M] = torch.from_numpy(A + A.conj().T)
+    b.P.copy_(P)
+    b.V[slots - 1].copy_(b.V[0])
+    b.V[: slots - 1].zero_()
+    st = b.state.cpu()
+    st[:, S_NB] = slots
+    b.state.copy_(st)
+    b.iterate_span(1, True)
+    if kind == "large":  # the step's own block is nothing beside the planted coupling: reported, not solved
+        assert (b.status()[:, S_STATUS] == _lib.RSED_EBREAKDOWN).all()
+        return
+    K = b.keep * block
+    for i in range(2):
+        A = b.P[i, :M, :M].cpu().numpy()
+        A = 0.5 * (A + A.conj().T)
+        assert np.abs(A).max() > 0
+        S = b.ritz_vec[i, :M, :K].cpu().numpy()
+        th = b.ritz_val[i, :K].cpu().numpy()
+        # a backward-stable reduction: a few ulps of the norm per row; the cluster
+        # gap of the Gram-Schmidt, 1e-3 of the norm, loses three digits
+        scale = np.linalg.norm(A, 2)
+        np.testing.assert_allclose(th, np.linalg.eigvalsh(A)[:K], atol=1e-15 * M * scale, rtol=0)
+        assert np.abs(A @ S - S * th).max() <= 1e-14 * M * scale
+        assert np.abs(S.conj().T @ S - np.eye(K)).max() < 1e-11
