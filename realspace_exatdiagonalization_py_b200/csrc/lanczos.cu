@@ -2489,8 +2489,13 @@ __global__ void k_rr_prepare(rsed_lanczos_t st) {
   }
 }
 
-// Each task (row r of T, column block l2) is split over NP = blockDim / tasks
-// row phases (interleaved rows), summed in phase order in shared memory.
+// Block (row chunk, instance): kRRRows rows of Q and H Q at a time in shared
+// memory, each read once, and T in 2 x 2 tiles of registers, a tile's rows split
+// over the NP = 256 / tiles threads that share it and summed in phase order at
+// the end: 16 FMA per four 16-B loads, where one column against a block of two
+// straight from global memory took a load per three (16 instances of 12 columns,
+// 657,756 rows: 6.8 -> 1.9 ms; 4 GB, 0.65 ms at the measured copy rate).
+constexpr int kRRRows = 32;
 __global__ void __launch_bounds__(256) k_rr_gram(rsed_lanczos_t st, LzDims d) {
   const int chunk = blockIdx.x / d.n_inst;
   const int inst = blockIdx.x % d.n_inst;
@@ -2507,50 +2512,54 @@ __global__ void __launch_bounds__(256) k_rr_gram(rsed_lanczos_t st, LzDims d) {
   double2* part = reinterpret_cast<double2*>(st.partial);
   const int64_t pbase = ((int64_t)chunk * d.n_inst + inst) * (int64_t)kRRMax * kRRMax;
   __shared__ int s_last;
-  // thread task: (row of T, column block l2, row phase) -> b accumulators
-  __shared__ double2 red[256][kBMax];
-  const int n_tasks = M * nq;
-  const int NP = n_tasks >= (int)blockDim.x ? 1 : (int)blockDim.x / n_tasks;
-  for (int t0 = 0; t0 < n_tasks * NP; t0 += blockDim.x) {  // one pass when NP > 1
-    const int t = t0 + (int)threadIdx.x;
-    const bool act = t < n_tasks * NP;
-    const int task = t % n_tasks, ph = t / n_tasks;
-    const int r = task / nq, l2 = task % nq;
-    double2 acc[kBMax];
+  __shared__ double2 tile[kRRRows][2 * kRRMax + 1];  // Q at 0, H Q at kRRMax; the odd stride spreads the banks
+  const int H = (M + 1) / 2, n_tiles = H * H;
+  const int NP = n_tiles >= 256 ? 1 : 256 / n_tiles;
+  const int tl = threadIdx.x % n_tiles, ph = threadIdx.x / n_tiles;
+  const int tr = tl / H * 2, tc = tl % H * 2;
+  double2 acc[2][2];
 #pragma unroll
-    for (int q = 0; q < kBMax; ++q) acc[q] = make_double2(0.0, 0.0);
-    if (act) {
-      const double2* Q = V + (int64_t)(r / b) * slot_stride + c0 + (r % b);
-      const double2* Z = V + (int64_t)(nq + l2) * slot_stride + c0;
+  for (int p = 0; p < 4; ++p) acc[p / 2][p % 2] = make_double2(0.0, 0.0);
+  for (int i = threadIdx.x; i < kRRRows * (2 * kRRMax + 1); i += 256)  // an odd M's last tile reads a zero column
+    (&tile[0][0])[i] = make_double2(0.0, 0.0);
+  const int lanes = 256 / b, lq = threadIdx.x % b, lw = threadIdx.x / b;
+  for (int64_t t0 = r0; t0 < r1; t0 += kRRRows) {
+    const int nr = (int)min((int64_t)kRRRows, r1 - t0);
+    __syncthreads();
+    if (lw < lanes) {
 #pragma unroll 4
-      for (int64_t row = r0 + ph; row < r1; row += NP) {
-        const double2 qv = Q[row * d.ld];
-#pragma unroll
-        for (int q = 0; q < kBMax; ++q)
-          if (q < b) acc[q] = cadd(acc[q], cdotc(qv, Z[row * d.ld + q]));
+      for (int w = lw; w < 2 * nq * kRRRows; w += lanes) {
+        // consecutive threads: a slot's columns, then the rows, then the slots
+        const int rr = w % kRRRows, l = w / kRRRows;
+        if (rr < nr)
+          tile[rr][(l < nq ? l * b : kRRMax + (l - nq) * b) + lq] =
+              V[(int64_t)l * slot_stride + (t0 + rr) * d.ld + c0 + lq];
       }
     }
-    if (NP == 1) {
-      if (act) {
-#pragma unroll
-        for (int q = 0; q < kBMax; ++q)
-          if (q < b) part[pbase + r * kRRMax + l2 * b + q] = acc[q];
+    __syncthreads();
+    if (ph < NP)
+#pragma unroll 2
+      for (int rr = ph; rr < nr; rr += NP) {
+        const double2 q0 = tile[rr][tr], q1 = tile[rr][tr + 1];
+        const double2 z0 = tile[rr][kRRMax + tc], z1 = tile[rr][kRRMax + tc + 1];
+        acc[0][0] = cadd(acc[0][0], cdotc(q0, z0));
+        acc[0][1] = cadd(acc[0][1], cdotc(q0, z1));
+        acc[1][0] = cadd(acc[1][0], cdotc(q1, z0));
+        acc[1][1] = cadd(acc[1][1], cdotc(q1, z1));
       }
-    } else {
+  }
+  // the row phases' sums, in phase order
+  double2* red = &tile[0][0];  // at least 4 x 256 entries
+  __syncthreads();
 #pragma unroll
-      for (int q = 0; q < kBMax; ++q) red[threadIdx.x][q] = acc[q];
-      __syncthreads();
-      if ((int)threadIdx.x < n_tasks) {
-#pragma unroll
-        for (int q = 0; q < kBMax; ++q) {
-          if (q >= b) continue;
-          double2 a = make_double2(0.0, 0.0);
-          for (int h = 0; h < NP; ++h) a = cadd(a, red[threadIdx.x + h * n_tasks][q]);
-          part[pbase + r * kRRMax + l2 * b + q] = a;
-        }
-      }
-      __syncthreads();
-    }
+  for (int p = 0; p < 4; ++p) red[p * 256 + threadIdx.x] = acc[p / 2][p % 2];
+  __syncthreads();
+  for (int e = threadIdx.x; e < 4 * n_tiles; e += 256) {
+    const int p = e / n_tiles, t = e % n_tiles;
+    const int r = t / H * 2 + p / 2, cc = t % H * 2 + p % 2;
+    double2 a = make_double2(0.0, 0.0);
+    for (int h = 0; h < NP; ++h) a = cadd(a, red[p * 256 + h * n_tiles + t]);
+    if (r < M && cc < M) part[pbase + r * kRRMax + cc] = a;
   }
   __threadfence();
   __syncthreads();
@@ -2586,7 +2595,9 @@ __global__ void __launch_bounds__(256) k_rr_gram(rsed_lanczos_t st, LzDims d) {
   }
 }
 
-// True FP64 residual norms of the nev refined pairs.
+// True FP64 residual norms of the nev refined pairs (16 instances of 12 columns,
+// 657,756 rows, 4 pairs: 3.9 -> 1.5 ms against one pair per walk over the basis
+// with the coefficients from global memory).
 __global__ void __launch_bounds__(128) k_rr_resid(rsed_lanczos_t st, LzDims d) {
   const int chunk = blockIdx.x / d.n_inst;
   const int inst = blockIdx.x % d.n_inst;
@@ -2605,19 +2616,38 @@ __global__ void __launch_bounds__(128) k_rr_resid(rsed_lanczos_t st, LzDims d) {
   const double* th = st.ritz_val + (int64_t)inst * d.pm;
   double* part = st.partial;
   __shared__ double red[kKeepMax][128];
+  __shared__ double2 sS[kRRMax][kKeepMax];  // the Ritz coefficients
   __shared__ int s_last;
+  for (int i = threadIdx.x; i < M * nev; i += blockDim.x) sS[i / nev][i % nev] = S[(int64_t)(i / nev) * d.pm + i % nev];
   for (int j = 0; j < nev; ++j) red[j][threadIdx.x] = 0.0;
+  __syncthreads();
+  // four pairs at a time: a row's entries of Q and H Q are read once for them
   for (int64_t row = r0 + threadIdx.x; row < r1; row += blockDim.x) {
-    for (int j = 0; j < nev; ++j) {
-      double2 hu = make_double2(0.0, 0.0), u = make_double2(0.0, 0.0);
-      for (int l = 0; l < M; ++l) {
-        const double2 sj = S[(int64_t)l * d.pm + j];
-        const int64_t off = row * d.ld + c0 + (l % b);
-        u = cadd(u, cmul(V[(int64_t)(l / b) * slot_stride + off], sj));
-        hu = cadd(hu, cmul(V[(int64_t)(nq + l / b) * slot_stride + off], sj));
+    for (int j0 = 0; j0 < nev; j0 += 4) {
+      double2 hu[4], u[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) hu[j] = u[j] = make_double2(0.0, 0.0);
+      for (int l = 0; l < nq; ++l) {
+        const double2* Q = V + (int64_t)l * slot_stride + row * d.ld + c0;
+        const double2* Z = Q + (int64_t)nq * slot_stride;
+#pragma unroll 2
+        for (int q = 0; q < b; ++q) {
+          const double2 vq = Q[q], vz = Z[q];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const double2 sj = sS[l * b + q][min(j0 + j, nev - 1)];
+            u[j] = cadd(u[j], cmul(vq, sj));
+            hu[j] = cadd(hu[j], cmul(vz, sj));
+          }
+        }
       }
-      const double2 r = make_double2(hu.x - th[j] * u.x, hu.y - th[j] * u.y);
-      red[j][threadIdx.x] += r.x * r.x + r.y * r.y;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (j0 + j >= nev) break;
+        const double t = th[j0 + j];
+        const double2 r = make_double2(hu[j].x - t * u[j].x, hu[j].y - t * u[j].y);
+        red[j0 + j][threadIdx.x] += r.x * r.x + r.y * r.y;
+      }
     }
   }
   __syncthreads();

@@ -404,3 +404,43 @@ def test_projected_eigenproblem(block, slots, kind):
         np.testing.assert_allclose(th, np.linalg.eigvalsh(A)[:K], atol=1e-15 * M * scale, rtol=0)
         assert np.abs(A @ S - S * th).max() <= 1e-14 * M * scale
         assert np.abs(S.conj().T @ S - np.eye(K)).max() < 1e-11
+
+
+# the FP64 refinement (Gram over the restart basis, residuals) of FP32 solves:
+# even and odd blocks and bases, a mixed batch, more pairs than one group of
+# four, by H's own action on the vectors
+@pytest.mark.parametrize("n_site,blocks,nev,keep", [
+    (16, [1], 1, 0), (16, [1, 1], 5, 7), (16, [2] * 3, 4, 0), (16, [3, 3], 3, 2), (16, [4, 2, 1], 2, 4), (16, [5], 6, 3),
+    (16, [8], 8, 2), (18, [2] * 9, 9, 5), (20, [4] * 2, 4, 4),
+])
+def test_refinement_blocks(n_site, blocks, nev, keep):
+    import torch
+
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import models
+    from realspace_exatdiagonalization_py_b200.lanczos import LanczosBatch
+
+    m = models.build_heisenberg_second_quantized_model(n_site, 1.0)
+    data = ed.build_ed_data(m, filling_fraction=Fraction(1, 2), symmetry_group=ed.build_translation_group(m.lattice))
+    dm, sset = data._device()
+    dm.build_projection(sset.sqrt_stab, precisions=(64, 32))
+    slots = min(64 // max(blocks), 2 * (keep or 4) + 8)
+    b = LanczosBatch(dm, sset, list(range(len(blocks))), nev,
+                     ed.LanczosParams(block=max(blocks), n_slots=slots, keep_blocks=keep, precision=32),
+                     block_sizes=blocks)
+    b.load_start(None)
+    b.start()
+    b.run()
+    b.rayleigh_ritz()
+    U, res, th = b.ritz_vectors_orbit(), b.residuals(), b.ritz_val[:, :nev].cpu().numpy()
+    ld = nev + nev % 2
+    for i in range(len(blocks)):
+        X = torch.zeros(U.shape[2], ld, dtype=torch.complex128, device="cuda")
+        X[:, :nev] = U[i].T
+        Y = torch.zeros_like(X)
+        dm.apply_block(sset, torch.full((nev,), i, dtype=torch.int32, device="cuda"), X, Y)
+        R = Y[:, :nev] - X[:, :nev] * torch.from_numpy(th[i]).cuda()
+        # rounding of H (norm below n_site) on unit vectors
+        assert np.abs(torch.linalg.norm(R, dim=0).cpu().numpy() - res[i]).max() < 1e-13 * n_site
+        T = X[:, :nev].conj().T @ Y[:, :nev]
+        assert (T - torch.diag(torch.from_numpy(th[i]).cuda())).abs().max().item() < 1e-13 * n_site
