@@ -58,7 +58,7 @@ WORKLOADS = {
 # (dram__bytes_read.sum + dram__bytes_write.sum); the capture commands and the
 # workloads are in the named profiles/ summaries.
 NCU_TRAFFIC: dict = {
-    ("haldane32", "k_proj_spmv<32>"): {"bytes_per_launch": 2.93e9 + 0.32535e9,
+    ("haldane32", "k_proj_spmv<32>"): {"bytes_per_launch": 2.677e9 + 0.329e9,
                                        "profile": "profiles/k_proj_spmv_fp32_haldane32_bench.md"},
 }
 
@@ -1061,10 +1061,10 @@ def run_b200(args):
                 "alg_bytes_per_launch": proj_apply_unique_bytes(nh, n_orb, b.n_cols, args.precision),
                 "unit_bytes": "per hop 4 + 8 B table, per row 8 + 8 + 16 B, per element x 8 B + y 16 B, once each"}
         lb = lanczos_step_bytes(n_orb, b, st_prof)
-        # the streamed forms: k_lz_gram_stream + k_lz_finalize (reduction),
-        # k_lz_update_stream (update); the per-instance forms k_lz_reduce,
-        # k_lz_update / k_lz_update_rows
-        for key, fam, extra_fam in (("reduce", "k_lz_reduce", ("k_lz_gram_stream", "k_lz_finalize")),
+        # the tiled and streamed forms: k_lz_gram_tiles, k_lz_gram_stream +
+        # k_lz_finalize (reduction), k_lz_update_stream (update); the others
+        # k_lz_reduce, k_lz_update / k_lz_update_rows / k_lz_update_own
+        for key, fam, extra_fam in (("reduce", "k_lz_reduce", ("k_lz_gram_tiles", "k_lz_gram_stream", "k_lz_finalize")),
                                     ("update", "k_lz_update", ())):
             n_k, us_k = _family(agg, fam)
             names = [fam + "*"] if n_k else []
