@@ -62,11 +62,17 @@ __global__ void __launch_bounds__(kFT, 6) k_fock_amps(rsed_group_t grp, const in
     inv[i + 1] = 1.0 / sqrt((double)grp.n_group * (double)(i + 1));
   }
   const bool unit = __syncthreads_or(twisted) == 0;
-  // |z| > atol by its square, the square root only next to the threshold
+  // |z| against atol by its square, the square root only next to the threshold
   const double sure = 1.0001 * atol * atol;
   auto above = [&](double2 z) {
     const double q = z.x * z.x + z.y * z.y;
     return q > sure || sqrt(q) > atol;
+  };
+  // not the negation of `above`: an infinite coefficient makes the amplitude NaN,
+  // which has to stay, so that the norm turns NaN and the state is refused
+  auto below = [&](double2 z) {
+    const double q = z.x * z.x + z.y * z.y;
+    return q <= sure && sqrt(q) <= atol;
   };
   double n2 = 0.0;
   for (int64_t r = (int64_t)blockIdx.x * kFChunk + threadIdx.x;
@@ -85,7 +91,7 @@ __global__ void __launch_bounds__(kFT, 6) k_fock_amps(rsed_group_t grp, const in
         rsed_phases<1>(s, g, N, grp.n_filled, perm, eta, grp.fermionic, unit, ph);
         sum = rsed_state_amplitude(s[0], m, e.y, ph[0], stab, grp, perm, eta, chi,
                                    make_double2(co.x * inv[order], co.y * inv[order]));
-        if (!above(sum)) sum = make_double2(0.0, 0.0);
+        if (below(sum)) sum = make_double2(0.0, 0.0);
       }
     }
     amp[r] = sum;

@@ -73,3 +73,26 @@ def test_fock_expansion_rejects_zero_state(golden):
     basis = ed.Symmetry_Sector_Basis(data.irrep_list[0], data.orbit_catalog, sset, 0)
     with pytest.raises(ValueError):
         ed.expand_sector_state_to_fock_amplitudes(np.zeros(basis.dim), basis, None)
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, complex(0.0, np.inf)])
+@pytest.mark.parametrize("case", ["haldane12_flux", "checkerboard12_flux", "hubbard12"])
+def test_fock_expansion_rejects_infinite_coefficients(golden, case, value):
+    """An infinite coefficient leaves no state to normalise, whether its orbit
+    has one group element per state or several; in every form of the call."""
+    import realspace_exatdiagonalization_py_b200 as ed
+
+    g = golden(case)
+    data = ed_data_for(case, g)
+    dm, sset = data._device()
+    order = np.array(data.orbit_catalog.stabilizer_order_list)
+    s = next(k for k, d in enumerate(sset.dims) if d > 1)
+    basis = ed.Symmetry_Sector_Basis(data.irrep_list[s], data.orbit_catalog, sset, s)
+    stab = order[basis.orbit_of_row.cpu().numpy()]
+    for row in {int(np.argmin(stab)), int(np.argmax(stab))}:
+        c = np.full(basis.dim, 0.1, dtype=np.complex128)
+        c[row] = value
+        with pytest.raises(ValueError):
+            ed.expand_sector_state_to_fock_amplitudes(c, basis, None)
+        with pytest.raises(ValueError):
+            ed.expand_sector_state_to_fock_dense(c, basis)
