@@ -15,6 +15,7 @@ measurement.
 
 from __future__ import annotations
 
+import copy
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -173,6 +174,21 @@ def ensure_projection(model: DeviceModel, sset: SectorSet, precision: int) -> No
         model.build_projection(sset.sqrt_stab, precisions=projection_precisions(model, precision))
     except torch.cuda.OutOfMemoryError:
         model.drop_projection()
+
+
+def streaming_view(model: DeviceModel, sset: SectorSet, precision: int) -> DeviceModel:
+    """``model`` with a projection table for one solve, where there is room for
+    it: a copy of the descriptor, whose table goes with it.  The model itself
+    stays as it is: solves of other sectors may run on it from other threads
+    and streams, its catalog may move to another flux point in place, and the
+    table's memory is the caller's again after the solve."""
+    view = copy.copy(model)
+    view.refresh()
+    try:
+        ensure_projection(view, sset, precision)
+    except ValueError:
+        view.drop_projection()  # beyond the table's limits (2^26 orbits, 48 KB of terms): on the fly
+    return view
 
 
 def plan_waves(n_orbits: int, block_sizes: list[int], budget: int, n_slots: int = 16,

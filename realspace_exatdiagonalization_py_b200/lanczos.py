@@ -516,21 +516,20 @@ def diagonalize_block_dense(H, *, nev: int = 5):
 
 
 def _solve_sector(model: DeviceModel, sset: SectorSet, s: int, nev: int, params: LanczosParams):
-    from .batched import APPLY_AUTO, ensure_projection
+    from .batched import APPLY_AUTO, streaming_view
 
-    if params.apply_variant == APPLY_AUTO:
-        # the table costs one or two products and serves every step and the
-        # model's other sectors
-        try:
-            ensure_projection(model, sset, params.precision)
-        except ValueError:
-            model.drop_projection()  # beyond the table's limits (2^26 orbits, 48 KB of terms): on the fly
+    # the solver's own buffers first: the table, which costs one or two products
+    # and serves every step, takes what room is left, and goes before the vectors
+    # are gathered
     b = LanczosBatch(model, sset, [s], nev, params)
     b.load_start(None)
+    if params.apply_variant == APPLY_AUTO:
+        b.model = streaming_view(model, sset, params.precision)
     b.start()
     b.run_aligned(graph=False)
     if params.precision == 32:
         refine(b)
+    b.model = model
     vals = b.eigenvalues()[0]
     vecs = b.eigenvectors()[0]
     return vals, vecs
