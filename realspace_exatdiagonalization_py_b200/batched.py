@@ -109,6 +109,20 @@ class BatchedSectorSolver:
         else:
             b.run(poll=poll, graph=False)
 
+    def _current_table(self) -> None:
+        """A table of the catalog's amplitudes as they are now: one that was
+        built before an in-place update of the catalog is built again (on the
+        fly where there is no room for it)."""
+        m, proj = self.model, self.model.proj
+        if proj is not None and proj["table_version"] == m.catalog.version:
+            return
+        m.refresh()
+        try:
+            m.build_projection(self.sset.sqrt_stab, precisions=proj["precisions"] if proj is not None else
+                               projection_precisions(m, self.precision))
+        except torch.cuda.OutOfMemoryError:
+            m.drop_projection()
+
     def solve(self, start_blocks=None, *, vectors: bool = True, host: bool = True, seeds=None):
         """Solve every sector; ``start_blocks`` and ``seeds`` (per instance, for
         the seeded blocks drawn where ``start_blocks`` is None) as in
@@ -119,6 +133,8 @@ class BatchedSectorSolver:
         ``None`` when ``vectors`` is false).
         """
         b = self.batch
+        if self.config.projection:
+            self._current_table()
         b.load_start(start_blocks, seeds)
         self._run(b, self.poll)
         if self.precision == 32:

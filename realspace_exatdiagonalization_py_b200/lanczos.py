@@ -187,6 +187,7 @@ class LanczosBatch:
         self._graph_iters = None
         self._spans = None  # restart-aligned graphs: ((head, launches), (cycle, launches))
         self._aligned_runs = 0
+        self._captured = None  # the table the graphs read: (addresses, its tensors)
 
     @property
     def n_inst(self) -> int:
@@ -285,10 +286,25 @@ class LanczosBatch:
     def done(self) -> bool:
         return not bool(self.state[:, S_ACTIVE].any().item())
 
+    def _table(self):
+        """(addresses, tensors) of the projection table that a step reads now."""
+        v = self.p.apply_variant
+        reads = v == 0 or 300 <= v < 999  # rsed_apply_h: the others run on the fly
+        proj = (getattr(self.model, "proj", None) or {}) if reads else {}
+        own = [proj.get(k) for k in ("rowptr", "cg", f"w{self.p.precision}")]
+        return [_lib.ptr(t) for t in own], own
+
+    def _check_graphs(self) -> None:
+        """Graphs hold the addresses of the table they were captured with (and
+        keep its tensors alive): they go when the model's table is another."""
+        if self._captured is not None and self._captured[0] != self._table()[0]:
+            self._graph = self._spans = self._captured = None
+
     def run(self, max_iter: int = 12000, poll: int = 8, graph: bool = False, stream=None) -> np.ndarray:
         """Iterate until every instance converged or failed; returns the state."""
         it = 0
         g = None
+        self._check_graphs()
         if graph:
             if getattr(self, "_graph", None) is None or self._graph_iters != poll:
                 self._graph = self.capture(poll)
@@ -326,6 +342,7 @@ class LanczosBatch:
         check_inside = self.periodic_check_in
         if h < 1 or period < 1 or check_inside(1, h):
             return self.run(max_iter, poll, graph=graph)
+        self._check_graphs()
         if graph and self._spans is None and self._aligned_runs > 0:
             # every kernel has run before the captures
             self._spans = (self.capture_span(h, False), self.capture_span(period, True))
@@ -401,6 +418,7 @@ class LanczosBatch:
         return self._capture(lambda st: self.iterate_span(n_iter, ritz_last, st), sync)
 
     def _capture(self, launch, sync: bool):
+        self._captured = self._table()
         s = torch.cuda.Stream()
         s.wait_stream(torch.cuda.current_stream())
         g = torch.cuda.CUDAGraph()
