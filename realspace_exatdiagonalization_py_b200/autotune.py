@@ -115,10 +115,10 @@ class Autotuner:
             os.replace(tmp, self.cache_path)
 
     def _projection_ok(self, dm: DeviceModel, precision: int) -> bool:
-        if dm.proj is not None:
+        if dm.has_weights(precision):
             return True
         free, _ = torch.cuda.mem_get_info(dm.hdiag.device)
-        need = dm.projection_bytes((64, 32) if precision == 32 else (64,))
+        need = dm.missing_projection_bytes((64, 32) if precision == 32 else (64,))
         return need <= self.memory_fraction * free
 
     def tune(self, dm: DeviceModel, sset: SectorSet, sectors: list[int], nev: int, precision: int = 32,

@@ -28,7 +28,7 @@ from .sector import SectorSet
 # rsed_apply_h variants: 0 = automatic (projection table when present),
 # 999 = automatic on-the-fly mapping
 APPLY_AUTO, APPLY_ON_THE_FLY = 0, 999
-# largest basis of the persistent path's automatic use (an explicit cluster size)
+# largest basis of the persistent path: an explicit cluster size asks for it up to here
 PERSISTENT_MAX_ORBITS = 1 << 16
 
 
@@ -88,8 +88,13 @@ class BatchedSectorSolver:
             raise ValueError("config.block_sizes needs one entry per sector")
         if config.persistent and not persistent_ok(config.block_sizes):
             raise ValueError("the persistent path needs uniform blocks of 1, 2 or 4 columns")
-        if config.projection and model.proj is None:
-            model.build_projection(sset.sqrt_stab, precisions=projection_precisions(model, precision))
+        if config.projection and not model.has_weights(precision):
+            try:
+                model.build_projection(sset.sqrt_stab, precisions=projection_precisions(model, precision))
+            except torch.cuda.OutOfMemoryError:
+                if model.proj is None:
+                    raise
+                # a table of the other precision: its products stream, these run on the fly
         p = LanczosParams(**{**p.__dict__, "n_slots": config.n_slots,
                              "apply_variant": APPLY_AUTO if config.projection else APPLY_ON_THE_FLY})
         self.config = config
@@ -166,30 +171,36 @@ class BatchedSectorSolver:
         return int(sum(t.numel() * t.element_size() for t in tensors if t is not None))
 
 
-def projection_precisions(model: DeviceModel, precision: int, fraction: float = 0.25) -> tuple[int, ...]:
+def projection_precisions(model: DeviceModel, precision: int, fraction: float = 0.25,
+                          free: int | None = None) -> tuple[int, ...]:
     """Weights to build: an FP32 solve also streams FP64 weights in its
-    refinement when both fit in ``fraction`` of the free device memory;
-    otherwise the refinement's few FP64 products run on the fly."""
+    refinement when both fit in ``fraction`` of the free device memory
+    (``free``, asked for if not given); otherwise the refinement's few FP64
+    products run on the fly."""
     if precision == 64:
         return (64,)
-    free, _ = torch.cuda.mem_get_info(model.hdiag.device)
-    return (64, 32) if model.projection_bytes((64, 32)) <= fraction * free else (32,)
+    if free is None:
+        free, _ = torch.cuda.mem_get_info(model.hdiag.device)
+    return (64, 32) if model.missing_projection_bytes((64, 32)) <= fraction * free else (32,)
 
 
-def ensure_projection(model: DeviceModel, sset: SectorSet, precision: int) -> None:
-    """Build the model's projection table unless it has one, it takes more than
-    half the free memory (asked only for tables above 1 GiB: the query can
-    stall for 100 ms), or there is no room for it; without it the products
-    run on the fly."""
-    if model.proj is not None:
-        return
-    nbytes = model.projection_bytes((precision,))
-    if nbytes > 1 << 30 and nbytes > 0.5 * torch.cuda.mem_get_info(model.hdiag.device)[0]:
+def ensure_projection(model: DeviceModel, sset: SectorSet, precision: int, free: int | None = None) -> None:
+    """Build the model's projection table with weights of ``precision``, or
+    what of it is missing, unless that takes more than half the ``free`` device
+    memory or there is no room for it; without them the products run on the
+    fly.  Without ``free`` (the query can stall for 100 ms) the memory is only
+    asked for above 1 GiB and for the second precision of an FP32 solve."""
+    if model.has_weights(precision):
         return
     try:
-        model.build_projection(sset.sqrt_stab, precisions=projection_precisions(model, precision))
+        nbytes = model.missing_projection_bytes((precision,))
+        if free is None and nbytes > 1 << 30:
+            free = torch.cuda.mem_get_info(model.hdiag.device)[0]
+        if free is not None and nbytes > 0.5 * free:
+            return
+        model.build_projection(sset.sqrt_stab, precisions=projection_precisions(model, precision, free=free))
     except torch.cuda.OutOfMemoryError:
-        model.drop_projection()
+        pass  # the model is as it was
 
 
 def streaming_view(model: DeviceModel, sset: SectorSet, precision: int) -> DeviceModel:

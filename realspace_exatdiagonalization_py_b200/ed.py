@@ -212,8 +212,6 @@ def solve_sectors_batched(ed_data, sector_ids: list[int], *, nev: int = 5, preci
         from .batched import ensure_projection, lanczos_footprint_bytes, plan_waves
 
         p = params or LanczosParams(precision=precision)
-        if config is None or config.projection:
-            ensure_projection(dm, sset, precision)  # the streaming matvec, when its table fits
         cache = ed_data.__dict__.setdefault("_solvers", {})
         resident = None
         if not (config is None and autotune):
@@ -226,6 +224,12 @@ def solve_sectors_batched(ed_data, sector_ids: list[int], *, nev: int = 5, preci
             waves = [list(range(len(big)))]
         else:
             free, _ = torch.cuda.mem_get_info()
+            if config is None or config.projection:
+                # the streaming matvec, when its table fits; the buffers are
+                # planned for what it leaves
+                reserved = torch.cuda.memory_reserved()
+                ensure_projection(dm, sset, precision, free)
+                free += reserved - torch.cuda.memory_reserved()
             n_orb = ed_data.orbit_catalog.n_orbits
             bs = list(config.block_sizes) if config is not None else [p.block] * len(big)
             budget = int(0.7 * free)

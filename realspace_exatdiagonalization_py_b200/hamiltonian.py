@@ -137,6 +137,12 @@ class DeviceModel:
         return 8 * (self.catalog.n_orbits + 1) + n * (4 + (16 if 64 in precisions else 0)
                                                       + (8 if 32 in precisions else 0))
 
+    def missing_projection_bytes(self, precisions) -> int:
+        """Device bytes that ``build_projection`` would still allocate."""
+        if self.proj is None:
+            return self.projection_bytes(precisions)
+        return self.proj["n_hops"] * sum({64: 16, 32: 8}[p] for p in set(precisions) - set(self.proj["precisions"]))
+
     def count_hops(self, stream=None) -> int:
         """Hops over all orbit rows (the projection table's entry count)."""
         lib = _lib.lib()
@@ -159,36 +165,45 @@ class DeviceModel:
         (a copy moved to another flux point by ``update_orbit_stabilizer_phases``
         keeps every target orbit and group element); its ``rowptr`` and ``cg``
         are reused and only the weights are computed."""
-        lib = _lib.lib()
         want = tuple(sorted(set(precisions)))
-        if self.proj is not None and self.proj["table_version"] == self.catalog.version and \
-                set(want) <= set(self.proj["precisions"]):
+        have = self.proj
+        if have is not None and have["table_version"] != self.catalog.version:
+            have = None
+        if have is not None and set(want) <= set(have["precisions"]):
             return
-        if share is not None and share["terms"] != self._term_key:
-            share = None  # other hops: a table of its own
-        if share is not None:
-            rowptr, cg, n = share["rowptr"], share["cg"], share["n_hops"]
-            dev = rowptr.device
-            w64 = torch.empty(max(n, 1), dtype=torch.complex128, device=dev) if 64 in want else None
-            w32 = torch.empty(max(n, 1), dtype=torch.complex64, device=dev) if 32 in want else None
-            _lib.check(lib.rsed_proj_fill(ctypes.byref(self.c), _lib.ptr(sqrt_stab), _lib.ptr(rowptr), None,
-                                          _lib.ptr(w64), _lib.ptr(w32), _lib.stream_ptr(stream)))
+        # the weights of another precision join a table that is there: its arrays
+        # stay where they are, captured graphs hold their addresses
+        base = have if have is not None else share
+        if base is not None and base["terms"] != self._term_key:
+            base = None  # other hops: a table of its own
+        if base is not None:
+            rowptr, cg, n = base["rowptr"], base["cg"], base["n_hops"]
+        else:
+            if self._hops is None:
+                self.count_hops(stream)
+            n, rowptr = self._hops
+            cg = torch.empty(max(n, 1), dtype=torch.int32, device=rowptr.device)
+        missing = set(want) - set(have["precisions"] if have is not None else ())
+        w64 = torch.empty(max(n, 1), dtype=torch.complex128, device=rowptr.device) if 64 in missing else None
+        w32 = torch.empty(max(n, 1), dtype=torch.complex64, device=rowptr.device) if 32 in missing else None
+        _lib.check(_lib.lib().rsed_proj_fill(ctypes.byref(self.c), _lib.ptr(sqrt_stab), _lib.ptr(rowptr),
+                                             None if base is not None else _lib.ptr(cg), _lib.ptr(w64), _lib.ptr(w32),
+                                             _lib.stream_ptr(stream)))
+        if have is not None:
+            self.proj = {**have, "w64": have["w64"] if w64 is None else w64,
+                         "w32": have["w32"] if w32 is None else w32,
+                         "precisions": tuple(sorted(set(want) | set(have["precisions"])))}
+        else:
             self.proj = {"rowptr": rowptr, "cg": cg, "w64": w64, "w32": w32, "n_hops": n, "precisions": want,
-                         "terms": self._term_key, "table_version": self.catalog.version, "shared": True}
-            self.refresh()
-            return
-        if self._hops is None:
-            self.count_hops(stream)
-        n, rowptr = self._hops
-        dev = rowptr.device
-        cg = torch.empty(max(n, 1), dtype=torch.int32, device=dev)
-        w64 = torch.empty(max(n, 1), dtype=torch.complex128, device=dev) if 64 in want else None
-        w32 = torch.empty(max(n, 1), dtype=torch.complex64, device=dev) if 32 in want else None
-        _lib.check(lib.rsed_proj_fill(ctypes.byref(self.c), _lib.ptr(sqrt_stab), _lib.ptr(rowptr),
-                                      _lib.ptr(cg), _lib.ptr(w64), _lib.ptr(w32), _lib.stream_ptr(stream)))
-        self.proj = {"rowptr": rowptr, "cg": cg, "w64": w64, "w32": w32, "n_hops": n,
-                     "precisions": want, "terms": self._term_key, "table_version": self.catalog.version}
+                         "terms": self._term_key, "table_version": self.catalog.version}
+            if base is not None:
+                self.proj["shared"] = True
         self.refresh()
+
+    def has_weights(self, precision: int) -> bool:
+        """Whether products of that precision can stream the table."""
+        return (self.proj is not None and precision in self.proj["precisions"]
+                and self.proj["table_version"] == self.catalog.version)
 
     def drop_projection(self) -> None:
         self.proj = None
