@@ -61,6 +61,8 @@ struct ObdmTile {
   static constexpr int RT = NP / 16;                  // outputs per thread and dimension
 };
 
+// Launches that need more than 48 KB allow the kernel what the largest group
+// takes, not what they take themselves: host threads share the attribute.
 struct ObdmLayout {
   size_t binom, eta, chi, perm, tile, total;
 };
@@ -466,7 +468,8 @@ int obdm_launch(const rsed_group_t& grp, const int4* table, const uint64_t* repr
   auto kern = k_obdm_part<NP, DENSE>;
   const ObdmLayout lay = obdm_layout(grp.n_site, grp.n_filled, DENSE ? 0 : grp.n_group);
   if (lay.total > 48 * 1024)
-    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.total));
+    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)obdm_layout(RSED_MAX_SITES, RSED_MAX_SITES, DENSE ? 0 : RSED_MAX_GROUP).total));
   const int n_sm = sm_count();
   const int wave = one_wave((const void*)kern, lay.total);
   RSED_REQUIRE(n_sm > 0 && wave > 0, RSED_ECUDA, "no occupancy for the one-body density kernel");
@@ -546,7 +549,8 @@ extern "C" int rsed_one_body_density(const rsed_group_t* grp, const rsed_entry_t
   if (dense) {
     const ObdmLayout lay = obdm_layout(N, grp->n_filled, grp->n_group);
     if (lay.total > 48 * 1024)
-      RSED_TRY_CUDA(cudaFuncSetAttribute(k_obdm_states, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.total));
+      RSED_TRY_CUDA(cudaFuncSetAttribute(k_obdm_states, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)obdm_layout(RSED_MAX_SITES, RSED_MAX_SITES, RSED_MAX_GROUP).total));
     const int wave = one_wave((const void*)k_obdm_states, lay.total);
     RSED_REQUIRE(wave > 0, RSED_ECUDA, "no occupancy for the state kernel");
     const int64_t blocks = (grp->n_states + kCT - 1) / kCT;

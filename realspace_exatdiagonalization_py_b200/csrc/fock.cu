@@ -151,8 +151,9 @@ extern "C" int rsed_fock_expand(const rsed_group_t* grp, const rsed_entry_t* tab
   cudaStream_t stream = as_stream(stream_);
   const int64_t n_blocks = (grp->n_states + kFChunk - 1) / kFChunk;
   const FockLayout lay = fock_layout(grp->n_site, grp->n_group);
-  if (lay.total > 40 * 1024)  // beside the static tables
-    RSED_TRY_CUDA(cudaFuncSetAttribute(k_fock_amps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.total));
+  if (lay.total > 40 * 1024)  // beside the static tables; the limit of every group: threads share the attribute
+    RSED_TRY_CUDA(cudaFuncSetAttribute(k_fock_amps, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)fock_layout(RSED_MAX_SITES, RSED_MAX_GROUP).total));
   double* bn = reinterpret_cast<double*>(scratch);
   double* nrm = bn + n_blocks;
   k_fock_amps<<<(unsigned)n_blocks, kFT, lay.total, stream>>>(

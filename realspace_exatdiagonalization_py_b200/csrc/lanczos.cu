@@ -3226,6 +3226,11 @@ int check_lz(const rsed_model_t* md, const rsed_sectors_t* sc, const rsed_lanczo
 
 // (row, instance) pairs from which the register forms of update and restart are used
 constexpr int64_t kOwnPairs = 65536;
+// Their shared memory at most: two blocks per SM.  The attribute that allows a
+// kernel more than 48 KB belongs to the kernel, so every launch sets the kernel's
+// own limit, never what this launch takes: another host thread may launch the
+// same kernel with more between the two statements.
+constexpr size_t kOwnSmem = 100 * 1024;
 
 // One wave of blocks of 256 threads over `units` block-sized pieces of work.
 int wave_grid(const void* kern, size_t smem, int64_t units, int64_t* grid) {
@@ -3243,7 +3248,7 @@ int launch_restart_own(const rsed_lanczos_t& st, const LzDims& d, int ig, cudaSt
   auto kern = k_lz_restart_own<BB, KM, US>;
   const size_t smem = sizeof(double2) * (size_t)st.n_slots * BB * st.keep_blocks * BB * ig;
   if (smem > 48 * 1024)
-    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOwnSmem));
   const int rows_pg = 256 / ig, groups = (d.n_inst + ig - 1) / ig;
   int64_t grid = 0;
   const int rc = wave_grid((const void*)kern, smem, (d.n_orb + rows_pg - 1) / rows_pg * groups, &grid);
@@ -3273,14 +3278,14 @@ int launch_restart_rows(const rsed_lanczos_t& st, const LzDims& d, int64_t grid,
 // up to 115 KB, one up to 220 KB), else the per-instance form.
 int launch_restart(const rsed_lanczos_t& st, const LzDims& d, cudaStream_t stream) {
   // one even block size for all instances: registers only, no barriers; groups
-  // of instances whose coefficients fit 100 KB (two blocks per SM).  Below 64k
+  // of instances whose coefficients fit kOwnSmem.  Below 64k
   // (row, instance) pairs the staging outweighs it (12 instances of 892 rows:
   // 44 us in the forms below, 57 us in this one)
   if (!(st.reserved & kFlagNoRowRestart) && d.uniform && (st.bmax == 2 || st.bmax == 4) &&
       d.n_orb * d.n_inst >= kOwnPairs) {
     const int K = st.keep_blocks * st.bmax;
     const size_t per = sizeof(double2) * (size_t)st.n_slots * st.bmax * K;  // <= 16 KB
-    int ig = (int)(100 * 1024 / per);
+    int ig = (int)(kOwnSmem / per);
     if (ig > 64) ig = 64;
     if (ig > d.n_inst) ig = d.n_inst;
     const int groups = (d.n_inst + ig - 1) / ig;
@@ -3344,7 +3349,7 @@ template <int BB, int RG, int US>
 int launch_update_own(const rsed_lanczos_t& st, const LzDims& d, int pass, size_t smem, cudaStream_t stream) {
   auto kern = k_lz_update_own<BB, RG, US>;
   if (smem > 48 * 1024)
-    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOwnSmem));
   const int rows = 256 / d.n_inst * RG;
   int64_t grid = 0;
   const int rc = wave_grid((const void*)kern, smem, (d.n_orb + rows - 1) / rows, &grid);
@@ -3360,7 +3365,7 @@ int launch_update(const rsed_lanczos_t& st, const LzDims& d, int pass, cudaStrea
   // (below 64k (row, instance) pairs the per-instance form has more blocks than
   // this one has coefficient copies to stage: 5.6 against 10.5 us for 12
   // instances of 892 rows)
-  if (d.uniform && (st.bmax == 2 || st.bmax == 4) && d.n_inst <= 256 && own <= 100 * 1024 &&
+  if (d.uniform && (st.bmax == 2 || st.bmax == 4) && d.n_inst <= 256 && own <= kOwnSmem &&
       d.n_orb * d.n_inst >= kOwnPairs)
     return st.bmax == 2 ? launch_update_own<2, 2, 3>(st, d, pass, own, stream)
                         : launch_update_own<4, 2, 2>(st, d, pass, own, stream);
@@ -3477,8 +3482,10 @@ int launch_gram_tiles(const rsed_lanczos_t& st, const LzDims& d, int pass, cudaS
   auto kern = k_lz_gram_tiles<BB, NS>;
   const int ig = tile_group(st, d), gw = ig * BB, groups = (d.n_inst + ig - 1) / ig;
   const size_t smem = sizeof(double2) * (kTileElems + (size_t)st.n_slots * BB * gw);
-  if (smem > 40 * 1024)  // beside the static tables
-    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 40 * 1024) {  // beside the static tables
+    constexpr size_t most = sizeof(double2) * (kTileElems + kJacobiMax * kTileCols);  // n_slots * BB <= kJacobiMax
+    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+  }
   const int rpw = 32 / gw, rows = kTileElems / gw / rpw * rpw;
   const int64_t tiles = (d.n_orb + rows - 1) / rows;
   int64_t grid = 0;

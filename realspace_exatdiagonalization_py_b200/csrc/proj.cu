@@ -507,8 +507,12 @@ int launch_spmv(const rsed_model_t& md, const rsed_sectors_t& sc, const void* x,
   int dev = 0;
   RSED_TRY_CUDA(cudaGetDevice(&dev));
   int& bps = blocks_per_sm[dev & 15];
-  if (smem > 48 * 1024)
-    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) {
+    // the limit of every model, not this call's size: host threads share the attribute
+    constexpr size_t chars = sizeof(W) * 64 * RSED_MAX_GROUP;
+    constexpr size_t most = kWide<PREC, CPL> ? pair_table_offset(chars) + sizeof(W) * RSED_MAX_GROUP * (NC / 2) : chars;
+    RSED_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+  }
   if (bps == 0) {
     RSED_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, 256, smem));
     if (bps < 1) bps = 1;
