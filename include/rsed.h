@@ -356,7 +356,11 @@ typedef struct {
   int32_t reserved;      /* bit 0: adaptive single Gram-Schmidt pass (pass 1 removes the part of
                           * the recurrence known from the projected matrix; pass 2 is skipped per
                           * instance when no Cholesky pivot of pass 1 lost more than 7/8 of its
-                          * column's norm^2) */
+                          * column's norm^2); bit 4: every instance has bmax columns and instance i
+                          * starts at column i * bmax, so that the kernels made for packed blocks
+                          * may run (without it any inst_col0 and any inst_b <= bmax are taken,
+                          * with columns between the instances); bits 1-3 choose kernel forms,
+                          * 0 = the default */
   double tol;            /* converged when ||r_j|| <= tol * max(1, |theta_j|) for j < nev */
   const int32_t* inst_col0;  /* n_inst: first column of each instance */
   const int32_t* inst_b;     /* n_inst: block size of each instance */

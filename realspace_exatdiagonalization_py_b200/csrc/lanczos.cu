@@ -60,6 +60,7 @@ constexpr int S_NB = 0, S_STATUS = 1, S_RESTARTS = 2, S_ITERS = 3, S_ACTIVE = 4,
 // single pass allowed when every Cholesky pivot^2 >= G_qq / kOnePassKappa2
 constexpr double kOnePassKappa2 = 8.0;
 constexpr int kFlagSinglePass = 1;
+constexpr int kFlagPacked = 16;  // st.reserved bit 4: instance i has bmax columns, from column i * bmax
 
 struct LzDims {
   int64_t n_orb;
@@ -3191,11 +3192,11 @@ LzDims make_dims(const rsed_model_t* md, const rsed_sectors_t* sc, const rsed_la
   d.chunk_rows = st->chunk_rows;
   d.n_chunks = (int)((d.n_orb + d.chunk_rows - 1) / d.chunk_rows);
   d.pslots = st->n_slots + 3;
-  // blocks of bmax columns that fill the columns in use lie at multiples of
-  // bmax; with an even ld and aligned buffers a segment of an even block is
-  // whole 32-B (V, W) and 16-B (Xf) words
+  // packed blocks of bmax columns (the caller says so: inst_b and inst_col0 are
+  // device arrays) that fill the columns in use; with an even ld and aligned
+  // buffers a segment of an even block is whole 32-B (V, W) and 16-B (Xf) words
   auto aligned = [](const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; };
-  const bool full = sc->n_cols == st->n_inst * st->bmax;
+  const bool full = (st->reserved & kFlagPacked) && sc->n_cols == st->n_inst * st->bmax;
   d.pairs = st->bmax == 1 ? 0 : full ? (st->bmax % 2 == 0 ? 1 : 0) : -1;
   d.uniform = full && (d.ld & 1) == 0 && aligned(st->V, 32) && aligned(st->W, 32) &&
               (st->Xf == nullptr || aligned(st->Xf, 16));

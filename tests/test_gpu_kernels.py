@@ -444,3 +444,46 @@ def test_refinement_blocks(n_site, blocks, nev, keep):
         assert np.abs(torch.linalg.norm(R, dim=0).cpu().numpy() - res[i]).max() < 1e-13 * n_site
         T = X[:, :nev].conj().T @ Y[:, :nev]
         assert (T - torch.diag(torch.from_numpy(th[i]).cuda())).abs().max().item() < 1e-13 * n_site
+
+
+# a caller of the C interface may leave columns free: instances of one column in
+# places of two or four, between full ones; they read as zero and stay so
+@pytest.mark.parametrize("n_site,wide,blocks", [(20, 2, [1, 2] * 6), (20, 4, [4, 2, 3, 1] * 3), (24, 2, [1, 2, 1])])
+def test_padded_column_layout(n_site, wide, blocks):
+    import torch
+
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import models
+    from realspace_exatdiagonalization_py_b200.lanczos import S_STATUS, LanczosBatch
+
+    m = models.build_heisenberg_second_quantized_model(n_site, 1.0)
+    data = ed.build_ed_data(m, filling_fraction=Fraction(1, 2), symmetry_group=ed.build_translation_group(m.lattice))
+    dm, sset = data._device()
+    dm.build_projection(sset.sqrt_stab, precisions=(64,))
+    n_inst, nev = len(blocks), 1
+    b = LanczosBatch(dm, sset, list(range(n_inst)), nev, ed.LanczosParams(block=wide, n_slots=12))
+    assert b.n_orb * n_inst >= 65536
+    b.c.reserved &= ~16  # not packed
+    b.inst_b.copy_(torch.tensor(blocks, dtype=torch.int32))
+    used = torch.zeros(b.ld, dtype=torch.bool, device="cuda")
+    for c0, k in zip(b.col0, blocks):
+        used[int(c0): int(c0) + k] = True
+    b.load_start(None)
+    b.W[:, ~used] = 0
+    b.start()
+    b.iterate_span(12, True)  # with a restart
+    assert not (b.status()[:, S_STATUS] < 0).any()
+    assert not b.V[: b.keep + 1][:, :, ~used].any()
+    n = b.keep
+    HV = torch.empty_like(b.V[: n + 1])
+    for s in range(n + 1):
+        dm.apply_block(sset, b.col_sector, b.V[s], HV[s], 64)
+    for i, (c0, k) in enumerate(zip(b.col0, blocks)):
+        Q = torch.cat([b.V[s][:, c0: c0 + k] for s in range(n + 1)], 1)
+        Z = torch.cat([HV[s][:, c0: c0 + k] for s in range(n + 1)], 1)
+        G = (Q.conj().T @ Q).cpu()
+        # a few ulps per Gram-Schmidt step and restart, sums of up to 112,720 products
+        assert (G - torch.eye(G.shape[0], dtype=G.dtype)).abs().max() < 2e-13
+        # the restart basis holds Ritz vectors
+        T = (Q.conj().T @ Z).cpu()[: n * k, : n * k]
+        assert (T - torch.diag(b.ritz_val[i, : n * k].cpu())).abs().max() < 1e-12 * n_site
