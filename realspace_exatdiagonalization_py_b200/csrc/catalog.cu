@@ -59,8 +59,8 @@ __device__ GroupView stage_group(const rsed_group_t& g, unsigned char* smem, siz
 // form a class, and the image of a mask is the union of its classes, each
 // rotated by its distance.  A translation of a periodic lattice has two classes
 // per wrapped direction at most (4 in two dimensions), so an image takes 4
-// and-rotate-or steps instead of one table step per occupied site.  Groups with
-// an element of more than kClasses distances take the images bit by bit.
+// and-rotate-or steps instead of one table step per occupied site.  Elements of
+// more than kClasses distances (reflections, rotations) take the image bit by bit.
 constexpr int kClasses = 8;
 
 template <typename M>
@@ -111,14 +111,23 @@ __device__ __forceinline__ I rank_of(M m, const I* binom, int kp1, M sb, I cb) {
   return sb ? ra * cb + rb : ra;
 }
 
-// Fills `mv` from the staged permutations; false if some element has more than
-// kClasses classes.  All threads of the block call it.
+// Image of m under the site permutation perm, bit by bit.
 template <typename M>
-__device__ bool stage_moves(const rsed_group_t& grp, const uint8_t* perm, GroupMoves<M>& mv) {
+__device__ __forceinline__ M permuted(M m, const uint8_t* perm) {
+  M img = 0;
+  for (; m; m &= m - 1) img |= (M)1 << perm[low_bit(m)];
+  return img;
+}
+
+// Fills `mv` from the staged permutations; the elements with more than kClasses
+// classes (theirs are incomplete), as a bitmask.  All threads of the block call it.
+template <typename M>
+__device__ uint64_t stage_moves(const rsed_group_t& grp, const uint8_t* perm, GroupMoves<M>& mv) {
   constexpr int W = 8 * sizeof(M) - 1;
+  __shared__ unsigned long long many;
+  if (threadIdx.x == 0) many = 0;
   for (int g = threadIdx.x; g < grp.n_group; g += blockDim.x) mv.n[g] = 0;
   __syncthreads();
-  bool fits = true;
   for (int t = threadIdx.x; t < grp.n_group * grp.n_site; t += blockDim.x) {
     const int g = t / grp.n_site, i = t % grp.n_site;
     const uint8_t* pg = perm + g * grp.n_site;
@@ -133,19 +142,25 @@ __device__ bool stage_moves(const rsed_group_t& grp, const uint8_t* perm, GroupM
     if (at < kClasses)
       mv.cls[g][at] = MoveClass<M>{mask, (M)d};
     else
-      fits = false;
+      atomicOr(&many, 1ull << g);
   }
-  return __syncthreads_and(fits);
+  __syncthreads();
+  return many;
 }
 
 // Pass 1: representative flags as a bitmap (symmetry_resolved_ed.py:519-528).
-// A thread tests R consecutive ranks (32 / R lanes share a bitmap word) against
-// all |G| images at once, each move class loaded once for the R masks.  Bound by
-// integer issue: some lane of a warp nearly always holds a representative, so
-// leaving the loop at the first smaller image saved nothing, and the images
-// themselves are the cost.  M = uint32_t up to 32 sites.
+// A thread tests R consecutive ranks (32 / R lanes share a bitmap word), first
+// against the images by move classes, each class loaded once for the R masks.
+// Bound by integer issue: some lane of a warp nearly always holds a
+// representative, so leaving that loop at the first smaller image saved nothing,
+// and the images themselves are the cost.  The elements without few classes come
+// after, for the ranks that are left, up to the first smaller image: their images
+// cost a step per occupied site.  M = uint32_t up to 32 sites.
 // 10.5 million states, 32 sites, |G| = 16: 865 us with one image per occupied
-// site step and 32 ranks per thread, 139 us in this form.
+// site step and 32 ranks per thread, 139 us in this form.  Dihedral group of 26
+// sites, 10.4 million states, half of 52 elements bit by bit: 2.46 ms with 32
+// ranks per thread and an exit at the first smaller image, 7.0 ms with every
+// element of the group bit by bit and no exit, 0.67 ms as here.
 template <typename M, int R>
 __global__ void __launch_bounds__(kFlagThreads) k_rep_flags(rsed_group_t grp, uint32_t* bitmap, int64_t* block_count,
                                                             int per_block, GroupSmemLayout lay) {
@@ -153,7 +168,7 @@ __global__ void __launch_bounds__(kFlagThreads) k_rep_flags(rsed_group_t grp, ui
   __shared__ GroupMoves<M> mv;
   __shared__ int warp_sums[kFlagThreads / 32];
   GroupView gv = stage_group(grp, smem, lay.binom_off, lay.perm_off, 0, 0, false, false);
-  const bool moves = stage_moves<M>(grp, gv.perm, mv);
+  const uint64_t many = stage_moves<M>(grp, gv.perm, mv);
   const int kp1 = grp.n_filled + 1;
   int count = 0;
   for (int t = 0; t < per_block; t += kFlagThreads * R) {
@@ -172,22 +187,27 @@ __global__ void __launch_bounds__(kFlagThreads) k_rep_flags(rsed_group_t grp, ui
       if (i + 1 < R && r0 + i + 1 < grp.n_states) w.next();
     }
     for (int g = 0; g < grp.n_group; ++g) {
+      if ((many >> g) & 1ull) continue;
       M img[R];
 #pragma unroll
       for (int i = 0; i < R; ++i) img[i] = 0;
-      if (moves) {
-        for (int c = 0; c < mv.n[g]; ++c) {
-          const MoveClass<M> cl = mv.cls[g][c];
+      for (int c = 0; c < mv.n[g]; ++c) {
+        const MoveClass<M> cl = mv.cls[g][c];
 #pragma unroll
-          for (int i = 0; i < R; ++i) img[i] |= rotl(m[i] & cl.mask, cl.rot);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < R; ++i) img[i] = (M)rsed_permute(m[i], gv.perm + g * grp.n_site);
+        for (int i = 0; i < R; ++i) img[i] |= rotl(m[i] & cl.mask, cl.rot);
       }
 #pragma unroll
       for (int i = 0; i < R; ++i)
         if (img[i] < m[i]) bits &= ~(1u << i);
+    }
+    if (many) {
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        for (uint64_t h = (bits >> i) & 1u ? many : 0; h; h &= h - 1)
+          if (permuted(m[i], gv.perm + (__ffsll((long long)h) - 1) * grp.n_site) < m[i]) {
+            bits &= ~(1u << i);
+            break;
+          }
     }
     count += __popc(bits);
     // the 32 / R lanes of a word put their bits together

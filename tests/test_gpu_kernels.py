@@ -487,3 +487,32 @@ def test_padded_column_layout(n_site, wide, blocks):
         # the restart basis holds Ritz vectors
         T = (Q.conj().T @ Z).cpu()[: n * k, : n * k]
         assert (T - torch.diag(b.ritz_val[i, : n * k].cpu())).abs().max() < 1e-12 * n_site
+
+
+# groups with some, none or only elements of few move distances, in both widths
+# of the masks and with one and eight ranks per thread
+@pytest.mark.parametrize("n,nf,kind", [
+    (12, 6, "dihedral"), (18, 9, "dihedral"), (23, 11, "dihedral"), (23, 11, "reflection"), (18, 9, "shuffled"),
+    (23, 11, "shuffled"), (36, 4, "reflection"), (36, 5, "shuffled"), (40, 5, "reflection"), (16, 16, "dihedral"),
+])
+def test_catalog_of_groups_with_many_distances(n, nf, kind):
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import models
+
+    if kind == "shuffled":  # a cyclic group on relabelled sites
+        lab = np.random.default_rng(n).permutation(n)
+        perms = [[0] * n for _ in range(n // 2)]
+        for s in range(n // 2):
+            for i in range(n):  # two cycles of n // 2 sites, a fixed site if n is odd
+                c, k = divmod(i, n // 2)
+                perms[s][lab[i]] = int(lab[i] if c == 2 else lab[c * (n // 2) + (k + s) % (n // 2)])
+    else:
+        turns = range(n) if kind == "dihedral" else [0]
+        perms = [[(i + s) % n for i in range(n)] for s in turns] + [[(s - 1 - i) % n for i in range(n)] for s in turns]
+    m = models.build_heisenberg_second_quantized_model(n, 1.0)
+    G = ed.Finite_Symmetry_Group(kind, [ed.Symmetry_Operation(str(s), [v + 1 for v in p])
+                                        for s, p in enumerate(perms)], identity_idx=0)
+    cat = ed.build_symmetry_orbit_catalog(second_quantized_model=m, n_filled=nf, symmetry_group=G,
+                                          particle_statistics=m.particle_statistics)
+    perm0, eta = port.group_arrays(G)
+    _check_catalog(cat, port.catalog(n, nf, perm0, eta, False))
