@@ -516,3 +516,61 @@ def test_catalog_of_groups_with_many_distances(n, nf, kind):
                                           particle_statistics=m.particle_statistics)
     perm0, eta = port.group_arrays(G)
     _check_catalog(cat, port.catalog(n, nf, perm0, eta, False))
+
+
+# the projected eigenproblem where its counts leave their range inside a group
+# of eight steps and at scales far from one: tridiagonal matrices of nearly equal
+# diagonal entries and couplings from small to below the square root of the
+# smallest number, diagonals on the interval's bisection points, large and small
+# norms.  Planted as above; with two Gram-Schmidt passes the step takes nothing
+# from P, so that its own block stays beside any scale
+@pytest.mark.parametrize("block,slots,kind,size", [
+    (1, 33, "clusters", 1e-8), (1, 33, "clusters", 1e-20), (2, 24, "clusters", 1e-70), (4, 16, "clusters", 1e-160),
+    (4, 16, "clusters", 0.0), (1, 49, "dyadic", 1e-3), (4, 16, "dyadic", 1e-20), (2, 32, "dyadic", 0.0),
+    (2, 24, "random", 1e60), (4, 16, "random", 1e100), (1, 20, "random", 1e60),
+])
+def test_projected_eigenproblem_ranges(block, slots, kind, size):
+    import torch
+
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import _lib, models
+    from realspace_exatdiagonalization_py_b200.lanczos import S_NB, S_STATUS, LanczosBatch
+
+    m = models.build_heisenberg_second_quantized_model(16, 1.0)
+    data = ed.build_ed_data(m, filling_fraction=Fraction(1, 2), symmetry_group=ed.build_translation_group(m.lattice))
+    dm, sset = data._device()
+    b = LanczosBatch(dm, sset, [0, 1], 2, ed.LanczosParams(block=block, n_slots=slots, tol=0.0, max_restarts=0,
+                                                           single_pass=False))
+    b.load_start(None)
+    b.start()
+    M = slots * block
+    rng = np.random.default_rng(M)
+    P = torch.zeros_like(b.P)
+    for i in range(2):
+        if kind == "random":
+            A = rng.standard_normal((M, M)) + 1j * rng.standard_normal((M, M))
+            A = size * (A + A.conj().T)
+        else:
+            d = np.full(M, -30.0) if kind == "clusters" else -32.0 + rng.integers(0, 3, M) * 2.0 ** -4
+            d[rng.permutation(M)[: M // 8]] = rng.uniform(-20, 20, M // 8)
+            A = np.diag(d) + size * (np.diag(np.ones(M - 1), 1) + np.diag(np.ones(M - 1), -1))
+        P[i, :M, :M] = torch.from_numpy(A)
+    b.P.copy_(P)
+    b.V[slots - 1].copy_(b.V[0])
+    b.V[: slots - 1].zero_()
+    st = b.state.cpu()
+    st[:, S_NB] = slots
+    b.state.copy_(st)
+    b.iterate_span(1, True)
+    K = b.keep * block
+    for i in range(2):
+        A = b.P[i, :M, :M].cpu().numpy()
+        A = 0.5 * (A + A.conj().T)
+        scale = np.linalg.norm(A, 2)
+        assert scale > 20 and int(b.status()[i, S_STATUS]) != _lib.RSED_EBREAKDOWN
+        S = b.ritz_vec[i, :M, :K].cpu().numpy()
+        th = b.ritz_val[i, :K].cpu().numpy()
+        # as for the cases above
+        np.testing.assert_allclose(th, np.linalg.eigvalsh(A)[:K], atol=1e-15 * M * scale, rtol=0)
+        assert np.abs(A @ S - S * th).max() <= 1e-14 * M * scale
+        assert np.abs(S.conj().T @ S - np.eye(K)).max() < 1e-11
