@@ -21,7 +21,16 @@
 namespace {
 
 constexpr int kFT = 256;
-constexpr int64_t kFChunk = 8 * kFT;  // ranks per block
+
+// Ranks per block: up to 8 per thread, so that a block's group tables serve 2048
+// states, as long as the blocks still fill the device (888 are resident); small
+// bases take one rank per thread.  Two expansions, us, with 8 ranks and as here:
+// 10,626 states 45 and 14, 134,596 states 67 and 29, 705,432 states 77 and 67
+// (30, 48 and 558 with every state's |G| images).
+int64_t fock_chunk(int64_t n_states) {
+  const int64_t per = n_states / (888 * kFT);
+  return kFT * (per < 1 ? 1 : per > 8 ? 8 : per);
+}
 
 struct FockLayout {
   size_t eta, chi, perm, total;
@@ -42,7 +51,8 @@ __global__ void __launch_bounds__(kFT, 6) k_fock_amps(rsed_group_t grp, const in
                                                       const double2* __restrict__ xo,
                                                       const double2* __restrict__ chi_g, double atol,
                                                       double2* __restrict__ amp, uint64_t* __restrict__ masks,
-                                                      double* __restrict__ block_norm2, FockLayout lay) {
+                                                      double* __restrict__ block_norm2, int64_t chunk,
+                                                      FockLayout lay) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[kFT / 32];
   __shared__ double inv[RSED_MAX_GROUP + 1];  // 1 / sqrt(|G| |Stab|)
@@ -75,8 +85,8 @@ __global__ void __launch_bounds__(kFT, 6) k_fock_amps(rsed_group_t grp, const in
     return q <= sure && sqrt(q) <= atol;
   };
   double n2 = 0.0;
-  for (int64_t r = (int64_t)blockIdx.x * kFChunk + threadIdx.x;
-       r < min(grp.n_states, ((int64_t)blockIdx.x + 1) * kFChunk); r += kFT) {
+  for (int64_t r = (int64_t)blockIdx.x * chunk + threadIdx.x;
+       r < min(grp.n_states, ((int64_t)blockIdx.x + 1) * chunk); r += kFT) {
     const int4 e = __ldg(table + r);
     double2 sum = make_double2(0.0, 0.0);
     uint64_t m = 0;
@@ -134,7 +144,7 @@ __global__ void k_fock_scale(double2* __restrict__ amp, int64_t n, const double*
 }  // namespace
 
 extern "C" size_t rsed_fock_scratch_bytes(int64_t n_states) {
-  const int64_t n_blocks = (n_states + kFChunk - 1) / kFChunk;
+  const int64_t chunk = fock_chunk(n_states), n_blocks = (n_states + chunk - 1) / chunk;
   return sizeof(double) * (size_t)(n_blocks + 2);
 }
 
@@ -149,7 +159,7 @@ extern "C" int rsed_fock_expand(const rsed_group_t* grp, const rsed_entry_t* tab
   RSED_REQUIRE(grp->eta != nullptr, RSED_EINVAL, "Fock expansion needs the group's eta phases");
   RSED_REQUIRE(scratch_bytes >= rsed_fock_scratch_bytes(grp->n_states), RSED_ESCRATCH, "Fock scratch too small");
   cudaStream_t stream = as_stream(stream_);
-  const int64_t n_blocks = (grp->n_states + kFChunk - 1) / kFChunk;
+  const int64_t chunk = fock_chunk(grp->n_states), n_blocks = (grp->n_states + chunk - 1) / chunk;
   const FockLayout lay = fock_layout(grp->n_site, grp->n_group);
   if (lay.total > 40 * 1024)  // beside the static tables; the limit of every group: threads share the attribute
     RSED_TRY_CUDA(cudaFuncSetAttribute(k_fock_amps, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -158,7 +168,7 @@ extern "C" int rsed_fock_expand(const rsed_group_t* grp, const rsed_entry_t* tab
   double* nrm = bn + n_blocks;
   k_fock_amps<<<(unsigned)n_blocks, kFT, lay.total, stream>>>(
       *grp, reinterpret_cast<const int4*>(table), repr_masks, stab_mask, reinterpret_cast<const double2*>(x_orbit),
-      reinterpret_cast<const double2*>(chi), atol, reinterpret_cast<double2*>(amp), masks, bn, lay);
+      reinterpret_cast<const double2*>(chi), atol, reinterpret_cast<double2*>(amp), masks, bn, chunk, lay);
   RSED_CHECK_LAUNCH();
   k_fock_norm<<<1, kFT, 0, stream>>>(bn, n_blocks, nrm);
   RSED_CHECK_LAUNCH();

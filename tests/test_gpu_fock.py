@@ -96,3 +96,28 @@ def test_fock_expansion_rejects_infinite_coefficients(golden, case, value):
             ed.expand_sector_state_to_fock_amplitudes(c, basis, None)
         with pytest.raises(ValueError):
             ed.expand_sector_state_to_fock_dense(c, basis)
+
+
+# below, at and above the sizes where a thread takes another rank: the norm's
+# partial sums cover every state once
+@pytest.mark.parametrize("n,nf", [(4, 2), (10, 5), (19, 9), (20, 10), (21, 10), (22, 11), (24, 12)])
+def test_fock_norm_over_block_sizes(n, nf):
+    from fractions import Fraction
+
+    import torch
+
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import models
+
+    m = models.build_heisenberg_second_quantized_model(n, 1.0)
+    data = ed.build_ed_data(m, filling_fraction=Fraction(nf, n), symmetry_group=ed.build_translation_group(m.lattice))
+    _, sset = data._device()
+    basis = ed.Symmetry_Sector_Basis(data.irrep_list[0], data.orbit_catalog, sset, 0)
+    c = torch.full((basis.dim,), 2.0, dtype=torch.complex128, device="cuda")
+    a = ed.expand_sector_state_to_fock_dense(c, basis)
+    # the zero-momentum sector of bosons: |c| = 2 / sqrt(orbit length) on each state of an orbit
+    cat = data.orbit_catalog
+    length = n / torch.from_numpy(np.array(cat.stabilizer_order_list, dtype=np.float64)).cuda()
+    want = (2.0 / torch.sqrt(length))[cat.table[:, 0].long()]
+    want /= torch.linalg.vector_norm(want)
+    assert (a - want).abs().max().item() < 1e-14
