@@ -598,6 +598,39 @@ int launch_variant(const rsed_model_t& md, const rsed_sectors_t& sc, const void*
   return rsed_set_error(RSED_EINVAL, "projection apply variant %d invalid at precision %d", variant, precision);
 }
 
+// Hops of a row on average: occupied sites times the terms of a site with an
+// empty target.
+double mean_hops(const rsed_model_t& md) {
+  const double N = md.n_site, k = md.n_filled;
+  return N > 1 ? md.n_terms * k * (N - k) / (N * (N - 1)) : 0.0;
+}
+
+// The variant for columns that do not pair up: 16-B segments, in the chunks that
+// leave the fewest columns of the last one empty, the wider ones first (each chunk
+// reads the table again and pays a row's fixed cost).  Rings, 13 hops a row, us:
+//   112,720 orbits, 24 columns: chunks of 16 / 32 167 / 133 FP64, 125 / 98 FP32
+//   400,024 orbits, 64 columns: 1248 / 961 FP64, chunks of 16 / 32 / 64 1059 / 750 / 605 FP32
+//   657,756 orbits of 56 hops: 24 columns 2925 / 2890 FP64, 2140 / 1890 FP32
+// 11,240 orbits of 56 hops lack the warps for it (24 columns: 55 / 57 FP64).  With a
+// third of a chunk empty the table counts against the padding: FP32, 18 columns,
+// chunks of 16 / 32: 56,742 orbits of 60 hops 178 / 183; 40 columns, chunks of 16 / 64: 291 / 288 with 25 hops a row, 383 / 412 with 37
+// (112,720 orbits), 1147 / 1079 with 27 and 1501 / 1563 with 41 (400,024 orbits).
+// Several FP64 chunks go one after another, so that a chunk of x stays in L2, only
+// on the largest bases (48 columns: 657,756 orbits 4434 against 4750 in one
+// launch, 400,024 orbits 1456 against 1430, 112,720 orbits 255 against 241).
+int narrow_variant(const rsed_model_t& md, int n_cols, int precision) {
+  const auto last = [&](int nc) { return (n_cols - 1) % nc + 1; };  // columns of the last chunk
+  const bool few_hops = mean_hops(md) < 28.0;
+  int nc = 2;
+  while (nc < n_cols && nc < 16) nc *= 2;
+  if (md.n_orbits >= (1 << 14) && n_cols > 16) {
+    if (last(32) > (precision == 32 && !few_hops ? 21 : 16)) nc = 32;
+    if (precision == 32 && n_cols > 32 && last(64) > (few_hops ? 32 : 48)) nc = 64;
+  }
+  if (precision == 32 || md.n_orbits < 65536) return 400 + (nc < 4 ? 4 : nc);
+  return (md.n_orbits < (1 << 19) ? 400 : 300) + nc;
+}
+
 }  // namespace
 
 // Called by rsed_apply_h for variants 0 (with a table present), 3NN-6NN.
@@ -621,9 +654,11 @@ int rsed_proj_apply(const rsed_model_t& md, const rsed_sectors_t& sc, const void
   // columns 385 and 367, 8 columns 415 and 580).  Other columns run best on 16-B
   // segments (16 columns of 16 sectors: FP64 1470 and 1610, FP32 1062 and 1082; 48
   // columns, FP64 4470 and 6456), as do the smallest bases, which want the warps of
-  // more chunks.  Where the caller does not know, a large basis launches both
-  // forms and the kernel that does not fit the columns leaves at once (4 us: FP64
-  // from 2^21 elements, about 100 us).
+  // more chunks: see narrow_variant.  Where the caller does not know, a large basis
+  // launches both forms and the kernel that does not fit the columns leaves at once:
+  // 4 us, FP64 from 2^25 hops of all columns on (about 250 us; ring of 400,024
+  // orbits, 12 columns: pairs 291 instead of 320 us, single columns 327 instead of
+  // 323; ring of 112,720 orbits, 36 columns: pairs 173 instead of 240).
   const int cpl = precision == 64 ? 2 : 4;
   const bool fits = sc.ld % cpl == 0 && (reinterpret_cast<uintptr_t>(x) & 31) == 0 && sc.n_cols % 2 == 0;
   const int64_t elems = md.n_orbits * (int64_t)sc.n_cols;
@@ -632,11 +667,9 @@ int rsed_proj_apply(const rsed_model_t& md, const rsed_sectors_t& sc, const void
   int wide = precision == 64 ? 4 : 8;
   while (wide < sc.n_cols && wide < 64) wide *= 2;
   wide += 600;
-  int narrow = small || precision == 32 ? 4 : 2;
-  while (narrow < sc.n_cols && narrow < 16) narrow *= 2;
-  narrow += small || precision == 32 ? 400 : 300;
+  const int narrow = narrow_variant(md, sc.n_cols, precision);
   if (!fits || !gains || pairs == 0 || md.n_orbits < 2048 ||
-      (pairs < 0 && (small || (precision == 64 && elems < (1 << 21)))))
+      (pairs < 0 && (small || (precision == 64 && elems * mean_hops(md) < (1 << 25)))))
     return launch_variant(md, sc, x, y, precision, narrow, 0, stream);
   const int rc = launch_variant(md, sc, x, y, precision, wide, pairs < 0 ? 1 : 0, stream);
   if (rc || pairs > 0) return rc;

@@ -574,3 +574,44 @@ def test_projected_eigenproblem_ranges(block, slots, kind, size):
         np.testing.assert_allclose(th, np.linalg.eigvalsh(A)[:K], atol=1e-15 * M * scale, rtol=0)
         assert np.abs(A @ S - S * th).max() <= 1e-14 * M * scale
         assert np.abs(S.conj().T @ S - np.eye(K)).max() < 1e-11
+
+
+# the default route of columns that do not pair up, by the chunks it takes: up to
+# 16, 17 to 32, a third chunk, a full 64, more; rows of few and of many hops, small
+# and larger bases
+@pytest.mark.parametrize("n_site,reach", [(18, 1), (20, 1), (22, 1), (22, 3), (24, 1), (24, 4)])
+@pytest.mark.parametrize("n", [5, 16, 17, 21, 22, 32, 33, 40, 49, 64, 65, 100])
+def test_projection_products_of_single_columns(n_site, reach, n):
+    import torch
+
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import models
+
+    m = models.build_heisenberg_second_quantized_model(n_site, 1.0)
+    data = ed.build_ed_data(m, filling_fraction=Fraction(1, 2), symmetry_group=ed.build_translation_group(m.lattice))
+    sset = ed.SectorSet(data.orbit_catalog, data.irrep_list)
+    terms = [(i + 1, (i + s * k) % n_site + 1, 0.5 / k) for i in range(n_site) for k in range(1, reach + 1)
+             for s in (1, -1)]
+    dm = ed.DeviceModel(data.orbit_catalog, terms, m.density_density_terms)
+    dm.build_projection(sset.sqrt_stab, precisions=(64, 32))
+    cs = torch.arange(n, dtype=torch.int32, device="cuda") % n_site
+    ld = n + n % 2
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    X = torch.randn(data.orbit_catalog.n_orbits, ld, dtype=torch.complex128, device="cuda", generator=gen)
+    X[:, :n] *= (sset.member[:, None] >> cs[None, :].long()) & 1
+    for prec, x, tol in ((64, X, 1e-13), (32, X.to(torch.complex64), 2e-6)):
+        # on the fly, 32 columns at a time
+        want = torch.zeros_like(X)
+        for c in range(0, n, 32):
+            w = min(32, n - c)
+            xs = torch.zeros(x.shape[0], w + w % 2, dtype=x.dtype, device="cuda")
+            xs[:, :w] = x[:, c: c + w]
+            ys = torch.zeros_like(xs, dtype=torch.complex128)
+            dm.apply_block(sset, cs[c: c + w].contiguous(), xs, ys, prec, 999)
+            want[:, c: c + w] = ys[:, :w]
+        Y = torch.zeros_like(X)
+        dm.apply_block(sset, cs, x, Y, prec)
+        top = max(1.0, want[:, :n].abs().max().item())
+        # the same products in another order: a few ulps of sums of up to 50 hops
+        assert (Y[:, :n] - want[:, :n]).abs().max().item() < tol * top
+        assert not Y[:, n:].any()
