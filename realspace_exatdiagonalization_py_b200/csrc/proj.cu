@@ -651,8 +651,11 @@ int rsed_proj_apply(const rsed_model_t& md, const rsed_sectors_t& sc, const void
   // FP64 31 and 40, FP32 22 and 27).  Few columns fill no 32-B segments of enough
   // lanes, which pays only where the gathers miss L2 (FP64 4 columns: 657,756
   // orbits 482 and 521, 112,720 orbits 52 and 47; 2 columns: 445 and 330; FP32 4
-  // columns 385 and 367, 8 columns 415 and 580).  Other columns run best on 16-B
-  // segments (16 columns of 16 sectors: FP64 1470 and 1610, FP32 1062 and 1082; 48
+  // columns 385 and 367, 8 columns 415 and 580).  80 columns go in chunks of 32, not
+  // of 64 (84,576 orbits: FP64 567 and 628, FP32 291 and 335).  A table of fewer than
+  // 2^16 hops has too few rows or hops for it (48 columns, FP64: 892 orbits of 42
+  // hops 17 and 8.6, 2,704 of 10 hops 10.2 and 8.2, 3,542 of 37 hops 16 and 21).
+  // Other columns run best on 16-B segments (16 columns of 16 sectors: FP64 1470 and 1610, FP32 1062 and 1082; 48
   // columns, FP64 4470 and 6456), as do the smallest bases, which want the warps of
   // more chunks: see narrow_variant.  Where the caller does not know, a large basis
   // launches both forms and the kernel that does not fit the columns leaves at once:
@@ -666,9 +669,10 @@ int rsed_proj_apply(const rsed_model_t& md, const rsed_sectors_t& sc, const void
   const bool gains = precision == 32 ? sc.n_cols >= 8 : sc.n_cols > 16 || (sc.n_cols >= 4 && elems >= (1 << 21));
   int wide = precision == 64 ? 4 : 8;
   while (wide < sc.n_cols && wide < 64) wide *= 2;
+  if (sc.n_cols > 64 && (sc.n_cols - 1) % 64 < 32) wide = 32;  // half of the last chunk empty
   wide += 600;
   const int narrow = narrow_variant(md, sc.n_cols, precision);
-  if (!fits || !gains || pairs == 0 || md.n_orbits < 2048 ||
+  if (!fits || !gains || pairs == 0 || md.n_orbits * mean_hops(md) < (1 << 16) ||
       (pairs < 0 && (small || (precision == 64 && elems * mean_hops(md) < (1 << 25)))))
     return launch_variant(md, sc, x, y, precision, narrow, 0, stream);
   const int rc = launch_variant(md, sc, x, y, precision, wide, pairs < 0 ? 1 : 0, stream);
