@@ -615,3 +615,36 @@ def test_projection_products_of_single_columns(n_site, reach, n):
         # the same products in another order: a few ulps of sums of up to 50 hops
         assert (Y[:, :n] - want[:, :n]).abs().max().item() < tol * top
         assert not Y[:, n:].any()
+
+
+# the tiled reduction in three groups (the blocks of a wave do not divide by it)
+# and the restart in three: as above
+@pytest.mark.parametrize("n_site,n_inst,block", [(20, 18, 4), (22, 24, 4), (22, 17, 4)])
+def test_three_groups(n_site, n_inst, block):
+    import torch
+
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200 import models
+    from realspace_exatdiagonalization_py_b200.lanczos import LanczosBatch
+
+    m = models.build_heisenberg_second_quantized_model(n_site, 1.0)
+    data = ed.build_ed_data(m, filling_fraction=Fraction(1, 2), symmetry_group=ed.build_translation_group(m.lattice))
+    dm, sset = data._device()
+    dm.build_projection(sset.sqrt_stab, precisions=(64,))
+    p = ed.LanczosParams(block=block)
+    b = LanczosBatch(dm, sset, [i % n_site for i in range(n_inst)], 1, p)
+    b.load_start(None)
+    b.start()
+    b.iterate_span(p.n_slots, True)  # up to the restart
+    n, K = b.keep, b.keep * block
+    HV = torch.empty_like(b.V[:n])
+    for s in range(n):
+        dm.apply_block(sset, b.col_sector, b.V[s], HV[s], 64)
+    for i in range(n_inst):
+        c = slice(i * block, (i + 1) * block)
+        Q = torch.cat([b.V[s][:, c] for s in range(n)], 1)
+        Z = torch.cat([HV[s][:, c] for s in range(n)], 1)
+        # a few ulps per Gram-Schmidt step and the restart; the restart basis holds Ritz vectors
+        assert ((Q.conj().T @ Q).cpu() - torch.eye(K, dtype=Q.dtype)).abs().max() < 1e-12
+        T = (Q.conj().T @ Z).cpu()
+        assert (T - torch.diag(b.ritz_val[i, :K].cpu())).abs().max() < 2e-12 * n_site
