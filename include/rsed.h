@@ -314,8 +314,8 @@ int rsed_position_overlaps(const rsed_group_t* grp, int64_t n_orbits, const uint
  * `stream`; the sums run in a fixed order for a given device. */
 size_t rsed_obdm_scratch_bytes(int32_t n_site);
 /* With rsed_obdm_states_bytes(n_states) more bytes of scratch (32 B a state,
- * 32-byte aligned) every state's amplitudes are written once and read back,
- * which is 4 times faster than evaluating them at every lookup. */
+ * 32-byte aligned) every state's amplitudes are written once and read back
+ * (10.5 million states: 2.9 ms, 6.5 ms evaluating them at every lookup). */
 size_t rsed_obdm_states_bytes(int64_t n_states);
 int rsed_one_body_density(const rsed_group_t* grp, const rsed_entry_t* table, int64_t n_orbits,
                           const uint64_t* repr_masks, const uint64_t* stab_mask, const uint64_t* member,

@@ -171,16 +171,13 @@ class BatchedSectorSolver:
         return int(sum(t.numel() * t.element_size() for t in tensors if t is not None))
 
 
-def projection_precisions(model: DeviceModel, precision: int, fraction: float = 0.25,
-                          free: int | None = None) -> tuple[int, ...]:
+def projection_precisions(model: DeviceModel, precision: int, fraction: float = 0.25) -> tuple[int, ...]:
     """Weights to build: an FP32 solve also streams FP64 weights in its
-    refinement when both fit in ``fraction`` of the free device memory
-    (``free``, asked for if not given); otherwise the refinement's few FP64
-    products run on the fly."""
+    refinement when both fit in ``fraction`` of the free device memory;
+    otherwise the refinement's few FP64 products run on the fly."""
     if precision == 64:
         return (64,)
-    if free is None:
-        free, _ = torch.cuda.mem_get_info(model.hdiag.device)
+    free, _ = torch.cuda.mem_get_info(model.hdiag.device)
     return (64, 32) if model.missing_projection_bytes((64, 32)) <= fraction * free else (32,)
 
 
@@ -188,19 +185,21 @@ def ensure_projection(model: DeviceModel, sset: SectorSet, precision: int, free:
     """Build the model's projection table with weights of ``precision``, or
     what of it is missing, unless that takes more than half the ``free`` device
     memory or there is no room for it; without them the products run on the
-    fly.  Without ``free`` (the query can stall for 100 ms) the memory is only
-    asked for above 1 GiB and for the second precision of an FP32 solve."""
+    fly.  An FP32 solve also gets the FP64 weights of its refinement where both
+    take a quarter at most.  Without ``free`` (the query can stall for 100 ms)
+    the memory is only asked for above 1 GiB."""
     if model.has_weights(precision):
         return
-    try:
-        nbytes = model.missing_projection_bytes((precision,))
-        if free is None and nbytes > 1 << 30:
-            free = torch.cuda.mem_get_info(model.hdiag.device)[0]
-        if free is not None and nbytes > 0.5 * free:
-            return
-        model.build_projection(sset.sqrt_stab, precisions=projection_precisions(model, precision, free=free))
-    except torch.cuda.OutOfMemoryError:
-        pass  # the model is as it was
+    for want, fraction in [((64, 32), 0.25), ((32,), 0.5)] if precision == 32 else [((64,), 0.5)]:
+        try:
+            nbytes = model.missing_projection_bytes(want)
+            if free is None and nbytes > 1 << 30:
+                free = torch.cuda.mem_get_info(model.hdiag.device)[0]
+            if free is None or nbytes <= fraction * free:
+                model.build_projection(sset.sqrt_stab, precisions=want)
+                return
+        except torch.cuda.OutOfMemoryError:
+            pass  # the model is as it was
 
 
 def streaming_view(model: DeviceModel, sset: SectorSet, precision: int) -> DeviceModel:

@@ -7,9 +7,9 @@ and ``static_structure_factor`` / ``compute_structure_factor_map``
 arguments, ED bootstrap, return values and layouts.  The reductions over the
 sector's orbits run on the GPU:
 
-* ``rsed_one_body_density`` -- <a_i^dagger a_j> for all (i, j) in one pass
-  over the (orbit, group element) kets, every hop projected back into the
-  sector through the catalog table;
+* ``rsed_one_body_density`` -- <a_i^dagger a_j> for all (i, j) as a contraction
+  over the states with one particle less, whose N - k + 1 neighbours' bra and
+  ket amplitudes come from the catalog table;
 * ``rsed_density_pairs`` -- sum over the representatives of |c|^2 n_a n_b;
   the group sum that turns it into <n_i n_j> and the densities is a |G| x N^2
   scatter on the host, followed by the flavour filters and the Fourier sums.

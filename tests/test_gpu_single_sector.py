@@ -154,3 +154,23 @@ def test_solves_from_two_threads():
     for s in range(4):
         for v in got[s]:
             np.testing.assert_allclose(v, want[s], atol=1e-10, rtol=0)
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_solve_asks_for_no_memory_figure(monkeypatch, precision):
+    """The free-memory query can stall for 100 ms: a solve with a small table
+    does without it, and an FP32 one streams its refinement all the same."""
+    import torch
+
+    import realspace_exatdiagonalization_py_b200 as ed
+    from realspace_exatdiagonalization_py_b200.batched import streaming_view
+
+    def query(*a):
+        raise AssertionError("free memory asked for")
+
+    data = _heisenberg(16)
+    dm, sset = data._device()
+    monkeypatch.setattr(torch.cuda, "mem_get_info", query)
+    ed.ed_scan_at_irrep_matrixfree(data.irrep_list[0].label, data, nev=2,
+                                   params=ed.LanczosParams(precision=precision))
+    assert streaming_view(dm, sset, precision).proj["precisions"] == ((64,) if precision == 64 else (32, 64))
